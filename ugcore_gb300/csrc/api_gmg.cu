@@ -361,6 +361,7 @@ struct GmgT : GmgBase {
             for (const DevBuf<int> &q : L.crow) mix(q.p);
             mix(L.ilu.val.p); mix(L.ilu.col.p); mix(L.ilu.rowptr.p); mix(L.ilu.nlow.p); mix(L.ilu.uinv.p);
             h ^= (uint64_t)L.n;
+            for (int k = 0; k < L.At.dia.S; ++k) mix((const void *)(intptr_t)L.At.dia.off.o[k]);
         }
         mix(Ainv.p);
         mix(z64.p);
@@ -380,7 +381,7 @@ struct GmgT : GmgBase {
         L.dA.alloc(n);
         L.dB.alloc(n);
         if (is_base) return;
-        if (!reuse) L.At_lay.known = false;
+        if (!reuse) L.At_lay = OpLayout();
         L.w.alloc(n);
         L.dinv64.alloc(n);
         L.dfac64.alloc(n);
@@ -918,6 +919,17 @@ static GmgBase *build_gmg(ug4gb_gmg *m, const ug4gb_matrix *A_top, GmgT<V> *reus
                 L.sweep2 = sweep2_prepare<V>(c, L.At, L.gp);
         }
     }
+    // a refilled level met a nonzero entry at an offset its layout leaves out:
+    // these levels keep all their offsets from now on
+    if (dia_left_out(c))
+        for (int l = m->base; l < nl; ++l) {
+            GLevel<V> &L = G->lev[l];
+            if (!L.At_lay.left_out) continue;
+            L.At_lay = OpLayout();
+            L.At_lay.keep_all = true;
+            op_from_csr_cached<V>(c, L.A, L.At, m->smoother == UG4GB_SMOOTHER_JACOBI ? L.dinv64.p : nullptr,
+                                  c.allow_dia, L.At_lay);
+        }
     G->setup_base(c);
     G->setup_coarse(c);
     if (sizeof(V) != sizeof(double)) G->z64.alloc(g->lev[nl - 1].nv);

@@ -46,6 +46,8 @@ static uint64_t op_signature(const OpMat<double> &M)
     mix((uint64_t)M.nrows);
     mix((uint64_t)(uintptr_t)M.dia.val.p);
     mix((uint64_t)M.dia.S);
+    if (M.kind == 1)
+        for (int k = 0; k < M.dia.S; ++k) mix((uint64_t)(int64_t)M.dia.off.o[k]);
     mix((uint64_t)(uintptr_t)M.sell.val.p);
     mix((uint64_t)(uintptr_t)M.sell.col.p);
     mix((uint64_t)(uintptr_t)M.sell.sptr.p);

@@ -129,6 +129,8 @@ struct Ctx {
     int sweep_fusion = 0;
     int sweep_fusion_min_rows = 1 << 18;
     int sweep_fusion_tz = 8;    // z planes per block
+    DevBuf<int> dia_flag;       // see dia_left_out
+    bool dia_flag_pending = false;
     int sweep_wait_test = 0;    // failure test only: bytes no copy delivers (fused sweeps' bounded waits run out)
     // levels above the base cycled by the one-block coarse kernel (-1: as
     // many as its cost model finds faster than separate launches, 0: none)
@@ -490,26 +492,35 @@ template <class T>
 void sell_from_csr(Ctx &c, const Csr &A, Sell<T> &S, const double *col_scale /* nullable */);
 // distinct column offsets (col - row) of A, sorted; false if more than max_s
 bool csr_offsets(Ctx &c, const Csr &A, int max_s, std::vector<int> &offs);
-template <class T>
-void dia_from_csr(Ctx &c, const Csr &A, Dia<T> &D, const std::vector<int> &offs, const double *col_scale,
-                  bool refill = false);
-// solve format: diagonal when A is square with <= 27 offsets and allow_dia, else SELL-32
-template <class T>
-void op_from_csr(Ctx &c, const Csr &A, OpMat<T> &M, const double *col_scale, bool allow_dia);
 // The layout an operator's solve format was built with (diagonal offsets or
 // SELL-32 slices).  While the caller knows the CRS pattern is unchanged (the
 // same level, re-assembled), op_from_csr_cached refills the values of the
-// existing buffers in place: no host round trip, no allocation, the same
-// device pointers (captured CUDA graphs stay valid).
+// existing buffers in place: no allocation, the same device pointers
+// (captured CUDA graphs stay valid).
+//
+// A diagonal layout leaves out the offsets whose entries were all exactly 0
+// when it was built.  A refill tests their entries again and reports a
+// nonzero one through a device flag: the caller asks dia_left_out() before
+// the operator is used and, if it is set, builds the layout with keep_all.
 struct OpLayout {
     bool known = false;
     int kind = 0;                 // 0 SELL-32, 1 diagonal
     int nrows = 0;
     int64_t nnz = 0;
     std::vector<int> offs;        // diagonal offsets (padded)
+    std::vector<int> all;         // offsets of the CRS entries, increasing
+    bool sorted = false;          // every CRS row holds its columns in strictly increasing order
+    bool left_out = false;        // offs misses some of `all`
+    bool keep_all = false;        // leave no offset out
 };
+// solve format: diagonal when A is square with <= 27 offsets and allow_dia, else SELL-32
+template <class T>
+void op_from_csr(Ctx &c, const Csr &A, OpMat<T> &M, const double *col_scale, bool allow_dia);
 template <class T>
 void op_from_csr_cached(Ctx &c, const Csr &A, OpMat<T> &M, const double *col_scale, bool allow_dia, OpLayout &lay);
+// whether a refill since the last call met a nonzero entry at an offset its
+// layout leaves out (waits for the stream only if such a layout was refilled)
+bool dia_left_out(Ctx &c);
 // T = A^T (structural zeros kept) and perm[k] = position in A of the entry
 // that lands at position k of T; transpose_values refills T's values from
 // A's through perm (the same pattern)

@@ -65,8 +65,13 @@ struct ug4gb_matrix {
     {
         if (!op_valid) {
             const uint64_t key = pattern_key();
-            if (!key || key != op_key) op_layout.known = false;
+            if (!key || key != op_key) op_layout = ug4gb::OpLayout();
             ug4gb::op_from_csr_cached<double>(ctx->c, A, op, nullptr, ctx->c.allow_dia, op_layout);
+            if (ug4gb::dia_left_out(ctx->c)) {
+                op_layout = ug4gb::OpLayout();
+                op_layout.keep_all = true;
+                ug4gb::op_from_csr_cached<double>(ctx->c, A, op, nullptr, ctx->c.allow_dia, op_layout);
+            }
             op_key = key;
             op_valid = true;
         }

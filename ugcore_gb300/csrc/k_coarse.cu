@@ -212,6 +212,7 @@ template <class V>
 void coarse_cycle(Ctx &c, const CoarsePlan<V> *plan_dev, int S, size_t smem_bytes, const int *skip)
 {
     switch (S) {
+    case 7: UG_LAUNCH_PDL(c, (k_coarse_cycle<V, 7>), 1, kCoarseThreads, smem_bytes, plan_dev, skip); break;
     case 9: UG_LAUNCH_PDL(c, (k_coarse_cycle<V, 9>), 1, kCoarseThreads, smem_bytes, plan_dev, skip); break;
     case 15: UG_LAUNCH_PDL(c, (k_coarse_cycle<V, 15>), 1, kCoarseThreads, smem_bytes, plan_dev, skip); break;
     case 27: UG_LAUNCH_PDL(c, (k_coarse_cycle<V, 27>), 1, kCoarseThreads, smem_bytes, plan_dev, skip); break;
@@ -219,11 +220,12 @@ void coarse_cycle(Ctx &c, const CoarsePlan<V> *plan_dev, int S, size_t smem_byte
     }
 }
 
-bool coarse_width_ok(int S) { return S == 9 || S == 15 || S == 27; }
+bool coarse_width_ok(int S) { return S == 7 || S == 9 || S == 15 || S == 27; }
 
 template <class V>
 void coarse_prepare(size_t smem_bytes)
 {
+    UG_CUDA(cudaFuncSetAttribute(k_coarse_cycle<V, 7>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes));
     UG_CUDA(cudaFuncSetAttribute(k_coarse_cycle<V, 9>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes));
     UG_CUDA(cudaFuncSetAttribute(k_coarse_cycle<V, 15>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes));
     UG_CUDA(cudaFuncSetAttribute(k_coarse_cycle<V, 27>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes));

@@ -31,6 +31,8 @@
 // which computes every element's geometry from its own corner coordinates)
 // to rounding: the cells of a structured level are congruent up to the
 // rounding of their corner coordinates i / (n - 1).
+#include <algorithm>
+#include <cmath>
 #include <cstring>
 #include <type_traits>
 
@@ -609,6 +611,16 @@ bool launch_assemble_rows(Ctx &c, const Level &L, const AsmArgs &a_in, RowAsmCac
             copy_out(c, cache.vol.data(), vol.p, sizeof(double) * cache.vol.size());
             int okh = 0;
             copy_out(c, &okh, ok.p, sizeof(int));
+            // entries that vanish in exact arithmetic (on a Kuhn tetrahedron
+            // the couplings of its non-path edges) come out of the box-method
+            // sums as rounding noise of some 1e-16 of the largest entry: exact
+            // zeros here, so the solve format can leave their diagonals out
+            for (int p = 0; p < CT::NC; ++p) {
+                double *Ap = cache.A.data() + (size_t)p * E::K * E::K, big = 0.0;
+                for (int q = 0; q < E::K * E::K; ++q) big = std::max(big, std::fabs(Ap[q]));
+                for (int q = 0; q < E::K * E::K; ++q)
+                    if (std::fabs(Ap[q]) < 1e-14 * big) Ap[q] = 0.0;
+            }
             cache.normal = std::move(nrm);
             cache.ipoff = std::move(ipo);
             cache.usable = (okh == 1);

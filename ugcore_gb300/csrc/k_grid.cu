@@ -482,32 +482,119 @@ bool csr_offsets(Ctx &c, const Csr &A, int max_s, std::vector<int> &offs)
     return true;
 }
 
+// For every offset of the CRS entries: its diagonal in the layout, -1 if the
+// layout leaves it out.
+struct DiaMap {
+    int n;
+    int off[kMaxDiag];
+    int slot[kMaxDiag];
+};
+
+static DiaMap dia_map(const OpLayout &lay)
+{
+    DiaMap m{};
+    m.n = (int)lay.all.size();
+    for (int k = 0; k < m.n; ++k) {
+        m.off[k] = lay.all[k];
+        const auto it = std::lower_bound(lay.offs.begin(), lay.offs.end(), lay.all[k]);
+        m.slot[k] = (it != lay.offs.end() && *it == lay.all[k]) ? (int)(it - lay.offs.begin()) : -1;
+    }
+    return m;
+}
+
+// which offsets hold a nonzero entry (bit k of used: offset m.off[k]), and
+// whether any row's columns are not strictly increasing
+__global__ void k_dia_used(const int *__restrict__ rowptr, const int *__restrict__ col,
+                           const double *__restrict__ val, int nrows, DiaMap m, unsigned *used, int *unsorted)
+{
+    __shared__ unsigned block_bits;
+    if (threadIdx.x == 0) block_bits = 0u;
+    __syncthreads();
+    unsigned bits = 0u;
+    bool bad = false;
+    const int stride = gridDim.x * blockDim.x;
+    for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < nrows; r += stride) {
+        int last = -1, k = 0;
+        for (int a = rowptr[r]; a < rowptr[r + 1]; ++a) {
+            const int cc = col[a];
+            bad = bad || cc <= last;
+            if (cc <= last) k = 0;
+            last = cc;
+            while (k < m.n && m.off[k] != cc - r) ++k;
+            if (k < m.n && val[a] != 0.0) bits |= 1u << k;
+        }
+    }
+    if (bits) atomicOr(&block_bits, bits);
+    if (bad) atomicExch(unsorted, 1);
+    __syncthreads();
+    if (threadIdx.x == 0 && block_bits) atomicOr(used, block_bits);
+}
+
+// CRS -> diagonals.  Bound by memory: 8 bytes read and sizeof(T) written per
+// entry.  A block takes kFillRows rows; their values, one contiguous range of
+// the CRS, are staged in shared memory by consecutive threads, then each
+// thread writes its row's entries, consecutive threads on consecutive values
+// of a diagonal.  A row that holds as many (increasing) columns as there are
+// offsets holds exactly those, in order, so its columns are not read; other
+// rows look theirs up.  129^3 hexes, FP64: one row per thread straight from
+// the CRS took 930 us, every entry's sector fetched by strided threads.
+constexpr int kFillRows = 128, kFillMax = 27;
+
 template <class T>
-__global__ void k_dia_fill(const int *rowptr, const int *col, const double *val, int nrows, int ld, Offs off, int S,
-                           const double *col_scale, T *dval)
+__global__ void __launch_bounds__(kFillRows) k_dia_fill(const int *__restrict__ rowptr, const int *__restrict__ col,
+                                                        const double *__restrict__ val, int nrows, int ld, DiaMap m,
+                                                        bool sorted, const double *__restrict__ col_scale,
+                                                        T *__restrict__ dval, int *__restrict__ left_out)
 {
     PDL_ENTRY();
-    int r = blockIdx.x * blockDim.x + threadIdx.x;
+    __shared__ double sv[kFillRows * kFillMax];
+    const int r0 = blockIdx.x * kFillRows, r1 = min(r0 + kFillRows, nrows);
+    const int q0 = rowptr[r0], q1 = rowptr[r1];
+    const bool staged = q1 - q0 <= kFillRows * kFillMax;
+    if (staged)
+        for (int q = q0 + threadIdx.x; q < q1; q += kFillRows) sv[q - q0] = ld_stream(val + q);
+    __syncthreads();
+    const int r = r0 + threadIdx.x;
     if (r >= nrows) return;
-    for (int a = rowptr[r]; a < rowptr[r + 1]; ++a) {
-        int o = col[a] - r;
-        int k = 0;
-        while (k < S && off.o[k] != o) ++k;
-        if (k == S) continue;   // cannot happen: offs holds every offset of A
-        double v = val[a];
-        if (col_scale) v *= col_scale[col[a]];
-        dval[(size_t)k * ld + r] = (T)v;
+    const int a0 = rowptr[r], len = rowptr[r + 1] - a0;
+    bool bad = false;
+    auto put = [&](int k, int c, double v) {
+        const int s = m.slot[k];
+        if (s < 0) {
+            bad = bad || v != 0.0;
+            return;
+        }
+        if (col_scale) v *= __ldg(col_scale + c);
+        T t;
+        if constexpr (sizeof(T) == 4) t = f64_to_f32(v);
+        else t = (T)v;
+        dval[(size_t)s * ld + r] = t;
+    };
+    if (sorted && len == m.n) {
+#pragma unroll 3
+        for (int k = 0; k < len; ++k) put(k, r + m.off[k], staged ? sv[a0 - q0 + k] : val[a0 + k]);
+    } else {
+        for (int a = a0; a < a0 + len; ++a) {
+            const int c = col[a];
+            int k = 0;
+            while (k < m.n && m.off[k] != c - r) ++k;
+            if (k < m.n) put(k, c, staged ? sv[a - q0] : val[a]);   // m holds every offset of A
+        }
     }
+    if (bad) *left_out = 1;
 }
 
 // refill: D already holds this pattern's layout (the same offsets, the same
 // CSR pattern): only the pattern's positions are rewritten, the zeros of the
-// absent entries, the padding rows and the guards are kept
+// absent entries, the padding rows and the guards are kept.  values_changed:
+// not the values the layout's offsets were chosen by (dia_left_out)
 template <class T>
-void dia_from_csr(Ctx &c, const Csr &A, Dia<T> &D, const std::vector<int> &offs, const double *col_scale,
-                  bool refill)
+static void dia_from_csr(Ctx &c, const Csr &A, Dia<T> &D, const OpLayout &lay, const double *col_scale, bool refill,
+                         bool values_changed)
 {
-    UG_REQUIRE((int)offs.size() <= kMaxDiag, UG4GB_ERR_INVALID, "dia_from_csr: too many offsets");
+    const std::vector<int> &offs = lay.offs;
+    UG_REQUIRE((int)offs.size() <= kMaxDiag && (int)lay.all.size() <= kMaxDiag, UG4GB_ERR_INVALID,
+               "dia_from_csr: too many offsets");
     const size_t want = (size_t)offs.size() * ((A.nrows + 31) / 32 * 32) + 2 * Dia<T>::kGuard;
     refill = refill && D.val.p && D.val.n == want && D.S == (int)offs.size() && D.nrows == A.nrows;
     D.nrows = A.nrows;
@@ -518,65 +605,120 @@ void dia_from_csr(Ctx &c, const Csr &A, Dia<T> &D, const std::vector<int> &offs,
     D.val.alloc((size_t)D.S * D.ld + 2 * Dia<T>::kGuard);
     // absent entries, the padding rows and the guards stay 0
     if (!refill) UG_CUDA(cudaMemsetAsync(D.val.p, 0, D.val.bytes(), c.stream));
-    UG_LAUNCH_PDL(c, k_dia_fill<T>, div_up(A.nrows, 256), 256, 0, A.rowptr.p, A.col.p, A.val.p, A.nrows, D.ld, D.off,
-              D.S, col_scale, D.vals());
+    if (lay.left_out) {
+        if (!c.dia_flag.p) {
+            c.dia_flag.alloc(1);
+            UG_CUDA(cudaMemsetAsync(c.dia_flag.p, 0, sizeof(int), c.stream));
+        }
+        if (values_changed) c.dia_flag_pending = true;
+    }
+    UG_LAUNCH_PDL(c, k_dia_fill<T>, div_up(A.nrows, kFillRows), kFillRows, 0, A.rowptr.p, A.col.p, A.val.p, A.nrows,
+                  D.ld, dia_map(lay), lay.sorted, col_scale, D.vals(), c.dia_flag.p);
 }
 
-// the diagonal kernels are instantiated for S = 9, 15, 27 (2D quads, Kuhn
-// tets, hexahedra); a smaller offset set is padded with offset 0 (value 0)
+bool dia_left_out(Ctx &c)
+{
+    if (!c.dia_flag_pending) return false;
+    c.dia_flag_pending = false;
+    int *h = (int *)c.host_pinned;
+    UG_CUDA(cudaMemcpyAsync(h, c.dia_flag.p, sizeof(int), cudaMemcpyDeviceToHost, c.stream));
+    UG_CUDA(cudaStreamSynchronize(c.stream));
+    if (!*h) return false;
+    UG_CUDA(cudaMemsetAsync(c.dia_flag.p, 0, sizeof(int), c.stream));
+    return true;
+}
+
+// the diagonal kernels are instantiated for S = 7 (Kuhn tets without their
+// zero diagonals), 9 (2D quads), 15 (Kuhn tets) and 27 (hexahedra); a smaller
+// offset set is padded with offsets that do not occur (value 0)
 static int dia_width(int s)
 {
+    if (s <= 7) return 7;
     if (s <= 9) return 9;
     if (s <= 15) return 15;
     if (s <= 27) return 27;
     return 0;
 }
 
+// the offsets of lay.all a layout of A stores: those with a nonzero entry
+// (all of them if none has one, or with keep_all), padded
 template <class T>
-void op_from_csr(Ctx &c, const Csr &A, OpMat<T> &M, const double *col_scale, bool allow_dia)
+static void choose_offsets(Ctx &c, const Csr &A, OpLayout &lay)
+{
+    OpLayout every;
+    every.offs = every.all = lay.all;
+    DevBuf<int> st;
+    st.alloc(2);
+    UG_CUDA(cudaMemsetAsync(st.p, 0, 2 * sizeof(int), c.stream));
+    UG_LAUNCH(c, k_dia_used, std::min<int>((int)div_up(A.nrows, 256), c.num_sms * 8), 256, 0, A.rowptr.p, A.col.p,
+              A.val.p, A.nrows, dia_map(every), (unsigned *)st.p, st.p + 1);
+    int h[2];
+    UG_CUDA(cudaMemcpyAsync(h, st.p, sizeof(h), cudaMemcpyDeviceToHost, c.stream));
+    UG_CUDA(cudaStreamSynchronize(c.stream));
+    const unsigned used = (unsigned)h[0];
+    lay.sorted = h[1] == 0;
+    // the fused sweeps (k_sweep2.cu) take the element types' whole stencils
+    const bool whole = lay.keep_all || used == 0 || (sizeof(T) == 4 && (c.sweep_fusion & 1));
+    lay.offs.clear();
+    for (size_t k = 0; k < lay.all.size(); ++k)
+        if (whole || ((used >> k) & 1u)) lay.offs.push_back(lay.all[k]);
+    // fewer offsets that still fill the same kernel's width save nothing
+    if (dia_width((int)lay.offs.size()) == dia_width((int)lay.all.size())) lay.offs = lay.all;
+    lay.left_out = lay.offs.size() < lay.all.size();
+    const int w = dia_width((int)lay.offs.size());
+    // pad with offsets that do not occur, keeping the set sorted
+    for (int cand = 1; (int)lay.offs.size() < w; cand = (cand > 0) ? -cand : -cand + 1)
+        if (!std::binary_search(lay.all.begin(), lay.all.end(), cand)) lay.offs.push_back(cand);
+    std::sort(lay.offs.begin(), lay.offs.end());
+}
+
+template <class T>
+static void op_build(Ctx &c, const Csr &A, OpMat<T> &M, const double *col_scale, bool allow_dia, OpLayout &lay)
 {
     M.nrows = A.nrows;
     M.ncols = A.ncols;
-    std::vector<int> offs;
-    if (allow_dia && A.nrows == A.ncols && csr_offsets(c, A, 27, offs)) {
-        int w = dia_width((int)offs.size());
-        // pad with offsets that do not occur (value 0), keeping the set sorted
-        int cand = 1;
-        while ((int)offs.size() < w) {
-            bool have = false;
-            for (int o : offs) have = have || (o == cand);
-            if (!have) offs.push_back(cand);
-            cand = (cand > 0) ? -cand : -cand + 1;
-        }
-        std::sort(offs.begin(), offs.end());
+    lay.all.clear();
+    lay.offs.clear();
+    lay.left_out = false;
+    if (allow_dia && A.nrows == A.ncols && csr_offsets(c, A, 27, lay.all)) {
+        choose_offsets<T>(c, A, lay);
         M.kind = 1;
-        dia_from_csr<T>(c, A, M.dia, offs, col_scale);
+        // the offsets were just chosen by these values: no entry to report
+        dia_from_csr<T>(c, A, M.dia, lay, col_scale, false, false);
         M.sell = Sell<T>();
     } else {
         M.kind = 0;
         sell_from_csr<T>(c, A, M.sell, col_scale);
         M.dia = Dia<T>();
     }
+    lay.known = true;
+    lay.kind = M.kind;
+    lay.nrows = A.nrows;
+    lay.nnz = A.nnz;
+}
+
+template <class T>
+void op_from_csr(Ctx &c, const Csr &A, OpMat<T> &M, const double *col_scale, bool allow_dia)
+{
+    OpLayout lay;
+    op_build<T>(c, A, M, col_scale, allow_dia, lay);
 }
 
 template <class T>
 void op_from_csr_cached(Ctx &c, const Csr &A, OpMat<T> &M, const double *col_scale, bool allow_dia, OpLayout &lay)
 {
-    if (lay.known && lay.nrows == A.nrows && lay.nnz == A.nnz && (lay.kind == 0 || allow_dia)) {
+    // the fused sweeps, switched on since, take the whole stencil (choose_offsets)
+    const bool widen = lay.left_out && sizeof(T) == 4 && (c.sweep_fusion & 1);
+    if (lay.known && lay.nrows == A.nrows && lay.nnz == A.nnz && (lay.kind == 0 || allow_dia) && !widen) {
         if (lay.kind == 1) {
-            dia_from_csr<T>(c, A, M.dia, lay.offs, col_scale, M.kind == 1);
+            dia_from_csr<T>(c, A, M.dia, lay, col_scale, M.kind == 1, true);
         } else {
             UG_LAUNCH(c, k_sell_fill<T>, div_up((size_t)M.sell.nslices * kSliceH, 256), 256, 0, A.rowptr.p, A.col.p,
                       A.val.p, A.nrows, M.sell.sptr.p, M.sell.swidth.p, col_scale, M.sell.col.p, M.sell.val.p);
         }
         return;
     }
-    op_from_csr<T>(c, A, M, col_scale, allow_dia);
-    lay.known = true;
-    lay.kind = M.kind;
-    lay.nrows = A.nrows;
-    lay.nnz = A.nnz;
-    lay.offs.assign(M.dia.off.o, M.dia.off.o + (M.kind == 1 ? M.dia.S : 0));
+    op_build<T>(c, A, M, col_scale, allow_dia, lay);
 }
 
 template void op_from_csr_cached<double>(Ctx &, const Csr &, OpMat<double> &, const double *, bool, OpLayout &);
@@ -720,10 +862,6 @@ void transpose_values(Ctx &c, const Csr &A, Csr &T, const DevBuf<int> &perm)
     if (T.nnz) UG_LAUNCH_PDL(c, k_gather_perm, div_up(T.nnz, (int64_t)256), 256, 0, T.nnz, perm.p, A.val.p, T.val.p);
 }
 
-template void dia_from_csr<double>(Ctx &, const Csr &, Dia<double> &, const std::vector<int> &, const double *,
-                                   bool);
-template void dia_from_csr<float>(Ctx &, const Csr &, Dia<float> &, const std::vector<int> &, const double *,
-                                  bool);
 template void op_from_csr<double>(Ctx &, const Csr &, OpMat<double> &, const double *, bool);
 template void op_from_csr<float>(Ctx &, const Csr &, OpMat<float> &, const double *, bool);
 

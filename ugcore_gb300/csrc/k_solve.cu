@@ -4,7 +4,7 @@
 // evict-first loads (coalesced 32-wide), the gathered vector kept in L1/L2.
 // Two operator layouts share the kernels through a "matrix view":
 //   SELL-32   general sparsity: 32-row slices, column-major in the slice;
-//   diagonal  <= 27 constant offsets (structured levels): values only, the
+//   diagonal  <= 27 constant offsets (structured levels; 7, 9, 15, 27): values only, the
 //             column of entry k is row + off[k]; no column stream and no
 //             load that depends on another load.
 // Row-local vector work is fused into the SpMV epilogue so each sweep reads
@@ -139,10 +139,10 @@ struct DiaMV {
     {
 #pragma unroll
         for (int e = 0; e < W; ++e) acc[e] = (V)0;
-        // diagonals in three batches: S/3 packs in flight per thread keeps
-        // the register count low enough for a full SM
-        constexpr int B = S / 3;
-        static_assert(B * 3 == S, "S must be a multiple of 3");
+        // diagonals in three batches (all 7 at once): the packs in flight per
+        // thread keep the register count low enough for a full SM
+        constexpr int B = (S == 7) ? 7 : S / 3;
+        static_assert(S % B == 0, "S must be a multiple of the batch");
 #pragma unroll 1
         for (int kb = 0; kb < S; kb += B) {
             Pack<V, W> a[B];
@@ -172,6 +172,7 @@ void with_mv(const OpMat<V> &m, F &&f)
     }
     const Dia<V> &d = m.dia;
     switch (d.S) {
+    case 7: f(DiaMV<V, 7>{d.nrows, d.ncols, d.ld, d.vals(), d.off}); break;
     case 9: f(DiaMV<V, 9>{d.nrows, d.ncols, d.ld, d.vals(), d.off}); break;
     case 15: f(DiaMV<V, 15>{d.nrows, d.ncols, d.ld, d.vals(), d.off}); break;
     case 27: f(DiaMV<V, 27>{d.nrows, d.ncols, d.ld, d.vals(), d.off}); break;
