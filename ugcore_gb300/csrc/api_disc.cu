@@ -49,6 +49,13 @@ const double *disc_coefficients(ug4gb_disc *d, int level)
     return D.Klev[level].p;
 }
 
+// class geometry of a structured level
+static RowAsmCache &class_cache(ug4gb_disc *d, int level)
+{
+    if (d->d.rows.size() < d->g->lev.size()) d->d.rows.resize(d->g->lev.size());
+    return d->d.rows[level];
+}
+
 // assemble the FV1 operator of `level` into A (and the rhs into b if given)
 void disc_assemble(ug4gb_disc *d, int level, ug4gb_matrix *A, double *b, const TimeScale *ts)
 {
@@ -94,11 +101,8 @@ void disc_assemble(ug4gb_disc *d, int level, ug4gb_matrix *A, double *b, const T
         a.sa1 = ts->sa1;
         a.u_old = ts->u_old;
     }
-    // structured levels, stationary: row by row, every value written once
-    if (c.row_assembly) {
-        if (D.rows.size() < d->g->lev.size()) D.rows.resize(d->g->lev.size());
-        if (launch_assemble_rows(c, L, a, D.rows[level])) return;
-    }
+    // structured levels: row by row, every value written once
+    if (c.row_assembly && launch_assemble_rows(c, L, a, class_cache(d, level))) return;
     if (!fresh) UG_CUDA(cudaMemsetAsync(A->A.val.p, 0, sizeof(double) * (size_t)A->A.nnz, c.stream));
     if (b) UG_CUDA(cudaMemsetAsync(b, 0, sizeof(double) * (size_t)L.nv, c.stream));
     launch_assemble(c, L, a);
@@ -113,7 +117,6 @@ void disc_defect(ug4gb_disc *d, int level, const double *u, double *dvec, const 
     const Level &L = d->g->lev[level];
     const DiscImpl &D = d->d;
     const bool top = (level == (int)d->g->lev.size() - 1);
-    UG_CUDA(cudaMemsetAsync(dvec, 0, sizeof(double) * (size_t)L.nv, c.stream));
     AsmArgs a;
     a.coords = L.coords.p;
     a.elems = L.elems.p;
@@ -143,7 +146,25 @@ void disc_defect(ug4gb_disc *d, int level, const double *u, double *dvec, const 
         a.sa1 = ts->sa1;
         a.u_old = ts->u_old;
     }
+    if (c.row_assembly && launch_defect_rows(c, L, a, class_cache(d, level))) return;
+    UG_CUDA(cudaMemsetAsync(dvec, 0, sizeof(double) * (size_t)L.nv, c.stream));
     launch_defect(c, L, a);
+}
+
+static void disc_grad_logk(ug4gb_disc *d, const double *K, const double *u, const double *lam, double *g)
+{
+    Ctx &c = d->ctx->c;
+    const int top = (int)d->g->lev.size() - 1;
+    if (c.row_assembly && launch_grad_logk_rows(c, d->g->lev[top], K, u, lam, g, class_cache(d, top))) return;
+    launch_grad_logk(c, d->g->lev[top], K, u, lam, g);
+}
+
+static void disc_grad_source(ug4gb_disc *d, const double *lam, double *g)
+{
+    Ctx &c = d->ctx->c;
+    const int top = (int)d->g->lev.size() - 1;
+    if (c.row_assembly && launch_grad_source_rows(c, d->g->lev[top], lam, g, class_cache(d, top))) return;
+    launch_grad_source(c, d->g->lev[top], lam, g);
 }
 
 }  // namespace ug4gb
@@ -502,11 +523,11 @@ int ug4gb_disc_grad_logk(ug4gb_disc *d, const ug4gb_vector *u, const ug4gb_vecto
         const double *K = disc_coefficients(d, (int)d->g->lev.size() - 1);
         if (is_device_ptr(grad)) {
             // in stream order on the context's stream
-            launch_grad_logk(c, L, K, u->d, lam->d, grad);
+            disc_grad_logk(d, K, u->d, lam->d, grad);
         } else {
             DevBuf<double> g;
             g.alloc(L.ne);
-            launch_grad_logk(c, L, K, u->d, lam->d, g.p);
+            disc_grad_logk(d, K, u->d, lam->d, g.p);
             copy_out(c, grad, g.p, g.bytes());
         }
     });
@@ -521,11 +542,11 @@ int ug4gb_disc_grad_source(ug4gb_disc *d, const ug4gb_vector *lam, double *grad)
     return guarded(d->ctx, [&] {
         Ctx &c = d->ctx->c;
         if (is_device_ptr(grad)) {
-            launch_grad_source(c, L, lam->d, grad);
+            disc_grad_source(d, lam->d, grad);
         } else {
             DevBuf<double> g;
             g.alloc(L.nv);
-            launch_grad_source(c, L, lam->d, g.p);
+            disc_grad_source(d, lam->d, g.p);
             copy_out(c, grad, g.p, g.bytes());
         }
     });

@@ -57,11 +57,18 @@ struct RowAsmCache {
     double volsum = 0.0;                // sum of an interior vertex's SCV volumes (gather order)
     DevBuf<int> brows;                  // the rows on the box boundary
     int nbrows = 0;
+    bool all_dirichlet = false;         // every row of brows is a Dirichlet vertex
+    int row_check = 0;                  // interior rows hold the stencil's entries: 1 yes, -1 no, 0 unknown
 };
-// stationary assembly of a structured level row by row (k_fv1_rows.cu):
-// every value of A and b written once, Dirichlet rows included; returns
-// false, launching nothing, where it does not apply
+// Structured levels from the class geometry (k_fv1_rows.cu): the assembly
+// (every value of A and b written once, Dirichlet rows included), the defect
+// (every entry of a.d written), the gradients.  Each returns false, launching
+// nothing, where it does not apply.
 bool launch_assemble_rows(Ctx &c, const Level &L, const AsmArgs &a, RowAsmCache &cache);
+bool launch_defect_rows(Ctx &c, const Level &L, const AsmArgs &a, RowAsmCache &cache);
+bool launch_grad_logk_rows(Ctx &c, const Level &L, const double *K, const double *u, const double *lam, double *g,
+                           RowAsmCache &cache);
+bool launch_grad_source_rows(Ctx &c, const Level &L, const double *lam, double *g, RowAsmCache &cache);
 void launch_dirichlet(Ctx &c, const Level &L, Csr &A, double *b);
 // d = defect of a.u on level L (a.d must be zero on entry; Dirichlet rows 0);
 // stationary, or instationary with a.inst and the scalings of AsmArgs

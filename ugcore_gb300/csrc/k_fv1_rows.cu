@@ -26,8 +26,16 @@
 // right-hand side (SetDirichletRow, sparsematrix_util.h:850-862); a boundary
 // row without the Dirichlet flag is assembled by the general path.
 //
-// The element kernel of k_fv1.cu stays the path of unstructured levels and of
-// the time-discrete assembly.  Values agree with it (and with the oracle,
+// The time-discrete operator sm0 M + sa0 A and its right-hand side (lumped
+// mass: a diagonal of control volumes), the defect and the adjoint gradients
+// use the same gathered row or class matrices.  Element by element, 8 colour
+// launches that each read and write the rows they touch, the time-discrete
+// assembly of 97^3 hexahedra took 7.3 ms and the defect of 49^3 Kuhn cells
+// 2.7 ms.
+//
+// The element kernels of k_fv1.cu stay the path of unstructured levels and of
+// boundary vertices without the Dirichlet flag outside the stationary
+// assembly.  Values agree with it (and with the oracle,
 // which computes every element's geometry from its own corner coordinates)
 // to rounding: the cells of a structured level are congruent up to the
 // rounding of their corner coordinates i / (n - 1).
@@ -335,8 +343,58 @@ __global__ void k_row_volsum(AsmArgs a, ClassData<T> cd, double *out)
     out[0] = s;
 }
 
-// interior rows: one thread per row, every value written once
+// Calls f(slot, offset in vertices) for the stencil of an interior row.
+template <int T, class F>
+__device__ __forceinline__ void for_stencil(int nx, int ny, F &&f)
+{
+    using S = Stencil<T>;
+#pragma unroll
+    for (int z = -1; z <= 1; ++z)
+#pragma unroll
+        for (int y = -1; y <= 1; ++y)
+#pragma unroll
+            for (int x = -1; x <= 1; ++x)
+                if (S::member(x, y, z)) f(S::slot(x, y, z), x + nx * (y + ny * z));
+}
+
+// (A v)_r from the gathered row of A
 template <int T>
+__device__ __forceinline__ double row_product(const double (&acc)[Stencil<T>::N], const double *__restrict__ v, int r,
+                                              int nx, int ny)
+{
+    double s = 0.0;
+    for_stencil<T>(nx, ny, [&](int k, int off) { s += acc[k] * __ldg(v + r + off); });
+    return s;
+}
+
+// Right-hand side of an interior row; acc: the row of A.  Time-discrete
+// (INST): sa0 f V - sm1 V u_old - sa1 (A u_old) + sa1 f V.
+template <int T, bool INST>
+__device__ __forceinline__ double row_rhs(const AsmArgs &a, const double (&acc)[Stencil<T>::N], int r, double volsum)
+{
+    const double fv = source_at(a, r) * volsum;
+    if constexpr (!INST) return fv;
+    double v = a.sa0 != 0.0 ? a.sa0 * fv : 0.0;
+    v -= a.sm1 * (volsum * a.u_old[r]);
+    if (a.sa1 != 0.0) {
+        v -= a.sa1 * row_product<T>(acc, a.u_old, r, a.cx + 1, a.cy + 1);
+        v += a.sa1 * fv;
+    }
+    return v;
+}
+
+// the row of A to the row of the time-discrete operator
+template <int T>
+__device__ __forceinline__ void row_in_time(const AsmArgs &a, double (&acc)[Stencil<T>::N], double volsum)
+{
+    using S = Stencil<T>;
+#pragma unroll
+    for (int s = 0; s < S::N; ++s) acc[s] *= a.sa0;
+    acc[S::slot(0, 0, 0)] += a.sm0 * volsum;
+}
+
+// interior rows: one thread per row, every value written once
+template <int T, bool INST>
 __global__ void __launch_bounds__(128) k_assemble_rows(AsmArgs a, ClassData<T> cd, const double *__restrict__ flux,
                                                        double volsum)
 {
@@ -352,10 +410,11 @@ __global__ void __launch_bounds__(128) k_assemble_rows(AsmArgs a, ClassData<T> c
 #pragma unroll
     for (int s = 0; s < S::N; ++s) acc[s] = 0.0;
     gather_row<T>(cd, a, i, j, k, flux, [&](int s, double v) { acc[s] += v; }, [](double) {});
+    if (a.b) a.b[r] = row_rhs<T, INST>(a, acc, r, volsum);
+    if constexpr (INST) row_in_time<T>(a, acc, volsum);
     double *row = a.val + __ldg(a.rowptr + r);
 #pragma unroll
     for (int s = 0; s < S::N; ++s) row[s] = acc[s];
-    if (a.b) a.b[r] = source_at(a, r) * volsum;
 }
 
 
@@ -440,7 +499,7 @@ __device__ __forceinline__ void boundary_row(const AsmArgs &a, const ClassData<T
 // small levels (launch-bound): every row of the level in one launch, one
 // thread per row, interior rows as k_assemble_rows, boundary rows as
 // k_assemble_boundary_rows
-template <int T>
+template <int T, bool INST>
 __global__ void __launch_bounds__(128) k_assemble_rows_all(AsmArgs a, ClassData<T> cd, const double *__restrict__ flux,
                                                            double volsum, const unsigned char *__restrict__ bnd)
 {
@@ -458,10 +517,11 @@ __global__ void __launch_bounds__(128) k_assemble_rows_all(AsmArgs a, ClassData<
 #pragma unroll
     for (int s = 0; s < S::N; ++s) acc[s] = 0.0;
     gather_row<T>(cd, a, i, j, k, flux, [&](int s, double v) { acc[s] += v; }, [](double) {});
+    if (a.b) a.b[r] = row_rhs<T, INST>(a, acc, r, volsum);
+    if constexpr (INST) row_in_time<T>(a, acc, volsum);
     double *row = a.val + __ldg(a.rowptr + r);
 #pragma unroll
     for (int s = 0; s < S::N; ++s) row[s] = acc[s];
-    if (a.b) a.b[r] = source_at(a, r) * volsum;
 }
 
 // the rows of a list (the box surface), one warp per row
@@ -494,13 +554,14 @@ __global__ void __launch_bounds__(256) k_assemble_boundary_rows(AsmArgs a, Class
 // memory: nx + 1 row pointers.
 constexpr int kLinesPerBlock = 1;
 
-template <int T>
+template <int T, bool INST>
 __global__ void __launch_bounds__(128) k_assemble_lines_uniform(AsmArgs a, ClassData<T> cd, double volsum, double kval,
                                                                 const unsigned char *__restrict__ bnd, int nlines)
 {
     PDL_ENTRY();
     using S = Stencil<T>;
-    __shared__ double st[S::N];
+    // the stencil of A (and of the time-discrete operator behind it)
+    __shared__ double st[S::N * (INST ? 2 : 1)];
     extern __shared__ int srp[];
     const int nx = a.cx + 1, ny = a.cy + 1, nz = (S::DIM == 3) ? a.cz + 1 : 1;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
@@ -513,6 +574,11 @@ __global__ void __launch_bounds__(128) k_assemble_lines_uniform(AsmArgs a, Class
                       [](double) {}, kval);
 #pragma unroll
         for (int s = 0; s < S::N; ++s) st[s] = acc[s];
+        if constexpr (INST) {
+            row_in_time<T>(a, acc, volsum);
+#pragma unroll
+            for (int s = 0; s < S::N; ++s) st[S::N + s] = acc[s];
+        }
     }
     __syncthreads();
     // the lines on the box surface come first (they take longer: started
@@ -568,11 +634,114 @@ __global__ void __launch_bounds__(128) k_assemble_lines_uniform(AsmArgs a, Class
         if (warp == 1) boundary_row<T>(a, cd, nullptr, bnd, rl, lane);
         else if (warp == 2) boundary_row<T>(a, cd, nullptr, bnd, rl + nx - 1, lane);
         double *line = a.val + __ldg(a.rowptr + r0);
-        if (a.b)
-            for (int i = threadIdx.x; i < nix; i += blockDim.x) a.b[r0 + i] = source_at(a, r0 + i) * volsum;
+        if (a.b) {
+            if constexpr (INST) {
+                double acc[S::N];
+#pragma unroll
+                for (int s = 0; s < S::N; ++s) acc[s] = st[s];
+                for (int i = threadIdx.x; i < nix; i += blockDim.x)
+                    a.b[r0 + i] = row_rhs<T, true>(a, acc, r0 + i, volsum);
+            } else {
+                for (int i = threadIdx.x; i < nix; i += blockDim.x) a.b[r0 + i] = source_at(a, r0 + i) * volsum;
+            }
+        }
         const int len = S::N * nix;
-        for (int q = threadIdx.x; q < len; q += blockDim.x) line[q] = st[q % S::N];
+        const double *val = st + (INST ? S::N : 0);
+        for (int q = threadIdx.x; q < len; q += blockDim.x) line[q] = val[q % S::N];
     }
+}
+
+// The defect of u (launch_defect) at every vertex, one thread each: the row
+// gathered as above times u (and u_old), Dirichlet vertices 0.  With the mass
+// and source terms of k_defect:
+//   stationary:     (A u)_i - f_i V_i
+//   time-discrete:  sm0 V u + sa0 ((A u) - f V) + sm1 V u_old + sa1 ((A u_old) - f V)
+template <int T>
+__global__ void __launch_bounds__(128) k_defect_rows(AsmArgs a, ClassData<T> cd, const double *__restrict__ flux,
+                                                     double volsum)
+{
+    using S = Stencil<T>;
+    const int nx = a.cx + 1, ny = a.cy + 1, nz = (S::DIM == 3) ? a.cz + 1 : 1;
+    const int r = blockIdx.x * blockDim.x + threadIdx.x;
+    if (r >= nx * ny * nz) return;
+    const int i = r % nx, j = (r / nx) % ny, k = r / (nx * ny);
+    if (i == 0 || i == nx - 1 || j == 0 || j == ny - 1 || (S::DIM == 3 && (k == 0 || k == nz - 1))) {
+        a.d[r] = 0.0;
+        return;
+    }
+    double acc[S::N];
+#pragma unroll
+    for (int s = 0; s < S::N; ++s) acc[s] = 0.0;
+    gather_row<T>(cd, a, i, j, k, flux, [&](int s, double v) { acc[s] += v; }, [](double) {});
+    const double fv = source_at(a, r) * volsum;
+    double v;
+    if (!a.inst) {
+        v = row_product<T>(acc, a.u, r, nx, ny) - fv;
+    } else {
+        v = a.sm0 * (volsum * a.u[r]);
+        if (a.sa0 != 0.0) {
+            v += a.sa0 * row_product<T>(acc, a.u, r, nx, ny);
+            v -= a.sa0 * fv;
+        }
+        v += a.sm1 * (volsum * a.u_old[r]);
+        if (a.sa1 != 0.0) {
+            v += a.sa1 * row_product<T>(acc, a.u_old, r, nx, ny);
+            v -= a.sa1 * fv;
+        }
+    }
+    a.d[r] = v;
+}
+
+// dJ/dm_e = -K_e sum_{i not Dirichlet} lambda_i (A1_c u_e)_i of the elements of
+// a cell, one thread per cell (k_grad_logk with the class matrices)
+template <int T>
+__global__ void __launch_bounds__(128) k_grad_logk_cells(ClassData<T> cd, int cx, int cy, int ncell,
+                                                         const unsigned char *__restrict__ bnd,
+                                                         const double *__restrict__ K, const double *__restrict__ u,
+                                                         const double *__restrict__ lam, double *__restrict__ g)
+{
+    using CT = ClassTraits<T>;
+    using E = Elem<T>;
+    constexpr int NV = (CT::DIM == 3) ? 8 : 4;
+    const int cell = blockIdx.x * blockDim.x + threadIdx.x;
+    if (cell >= ncell) return;
+    const int i = cell % cx, j = (cell / cx) % cy, k = cell / (cx * cy);
+    const int nx = cx + 1, ny = cy + 1, v0 = i + nx * (j + ny * k);
+    double uc[NV], lc[NV];
+#pragma unroll
+    for (int b = 0; b < NV; ++b) {
+        const int v = v0 + (b & 1) + nx * (((b >> 1) & 1) + ny * (b >> 2));
+        uc[b] = u[v];
+        lc[b] = bnd[v] ? 0.0 : lam[v];
+    }
+#pragma unroll
+    for (int p = 0; p < CT::NC; ++p) {
+        double s = 0.0;
+#pragma unroll
+        for (int q = 0; q < E::K; ++q) {
+            double r = 0.0;
+#pragma unroll
+            for (int t = 0; t < E::K; ++t) r += cd.A[p][q][t] * uc[class_corner_bits<T>(p, t)];
+            s += lc[class_corner_bits<T>(p, q)] * r;
+        }
+        const size_t e = (size_t)cell * CT::NC + p;
+        g[e] = -K[e] * s;
+    }
+}
+
+// dJ/df_i = lambda_i |SCV_i|, all vertices without the Dirichlet flag inside
+__global__ void k_grad_source_rows(double volsum, const unsigned char *__restrict__ bnd,
+                                   const double *__restrict__ lam, int nv, double *__restrict__ g)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < nv) g[i] = bnd[i] ? 0.0 : volsum * lam[i];
+}
+
+// every row of the list is a Dirichlet vertex
+__global__ void k_check_dirichlet(const unsigned char *bnd, const int *rows, int n, int *ok)
+{
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t < n && !bnd[rows[t]]) atomicExch(ok, 0);
 }
 
 }  // namespace
@@ -581,128 +750,226 @@ __global__ void __launch_bounds__(128) k_assemble_lines_uniform(AsmArgs a, Class
 // their assembly is bound by the launches, not by the rows
 constexpr int kSmallLevelRows = 1 << 16;
 
-// Assembles level L row by row when it is a structured level and the
-// assembly is stationary; returns false (nothing launched) otherwise.
+namespace {
+
+// Class geometry of level L (once per level, kept in cache), the SCV volume
+// sum of its interior rows, the list of its boundary rows; false where the
+// cells are not the classes' boxes.
+template <int T>
+bool class_data(Ctx &c, const Level &L, RowAsmCache &cache, ClassData<T> &cd)
+{
+    using CT = ClassTraits<T>;
+    using E = Elem<T>;
+    if (!L.structured || L.nx < 3 || L.ny < 3 || (L.dim == 3 && L.nz < 3)) return false;
+    if (!cache.ready) {
+        DevBuf<double> A, vol, nrm, ipo;
+        DevBuf<int> ok;
+        A.alloc(CT::NC * E::K * E::K);
+        vol.alloc(CT::NC * E::K);
+        nrm.alloc(CT::NC * E::NSCVF * 3);
+        ipo.alloc(CT::NC * E::NSCVF * 3);
+        ok.alloc(1);
+        const int one = 1;
+        copy_in(c, ok.p, &one, sizeof(int));
+        UG_LAUNCH(c, k_class_data<T>, 1, 32, 0, L.coords.p, L.elems.p, A.p, vol.p, nrm.p, ipo.p, ok.p);
+        cache.A.resize(CT::NC * E::K * E::K);
+        cache.vol.resize(CT::NC * E::K);
+        copy_out(c, cache.A.data(), A.p, sizeof(double) * cache.A.size());
+        copy_out(c, cache.vol.data(), vol.p, sizeof(double) * cache.vol.size());
+        int okh = 0;
+        copy_out(c, &okh, ok.p, sizeof(int));
+        // entries that vanish in exact arithmetic (on a Kuhn tetrahedron
+        // the couplings of its non-path edges) come out of the box-method
+        // sums as rounding noise of some 1e-16 of the largest entry: exact
+        // zeros here, so the solve format can leave their diagonals out
+        for (int p = 0; p < CT::NC; ++p) {
+            double *Ap = cache.A.data() + (size_t)p * E::K * E::K, big = 0.0;
+            for (int q = 0; q < E::K * E::K; ++q) big = std::max(big, std::fabs(Ap[q]));
+            for (int q = 0; q < E::K * E::K; ++q)
+                if (std::fabs(Ap[q]) < 1e-14 * big) Ap[q] = 0.0;
+        }
+        cache.normal = std::move(nrm);
+        cache.ipoff = std::move(ipo);
+        cache.usable = (okh == 1);
+        cache.ready = true;
+    }
+    if (!cache.usable) return false;
+    std::memcpy(&cd.A[0][0][0], cache.A.data(), sizeof(cd.A));
+    std::memcpy(&cd.vol[0][0], cache.vol.data(), sizeof(cd.vol));
+    if (cache.nbrows == 0) {
+        // once per level: the interior rows' SCV volume sum and the list of
+        // the rows on the box boundary
+        AsmArgs a{};
+        a.cx = L.nx - 1;
+        a.cy = L.ny - 1;
+        a.cz = (L.dim == 3) ? L.nz - 1 : 1;
+        DevBuf<double> vs;
+        vs.alloc(1);
+        UG_LAUNCH(c, k_row_volsum<T>, 1, 32, 0, a, cd, vs.p);
+        copy_out(c, &cache.volsum, vs.p, sizeof(double));
+        const int nx = L.nx, ny = L.ny, nz = (L.dim == 3) ? L.nz : 1;
+        std::vector<int> rows;
+        for (int k = 0; k < nz; ++k)
+            for (int j = 0; j < ny; ++j)
+                for (int i = 0; i < nx; ++i)
+                    if (i == 0 || i == nx - 1 || j == 0 || j == ny - 1 || (L.dim == 3 && (k == 0 || k == nz - 1)))
+                        rows.push_back(i + nx * (j + ny * k));
+        cache.brows.alloc(rows.size());
+        copy_in(c, cache.brows.p, rows.data(), sizeof(int) * rows.size());
+        DevBuf<int> ok;
+        ok.alloc(1);
+        int okh = 1;
+        copy_in(c, ok.p, &okh, sizeof(int));
+        UG_LAUNCH(c, k_check_dirichlet, div_up(rows.size(), 256), 256, 0, L.bnd.p, cache.brows.p, (int)rows.size(),
+                  ok.p);
+        copy_out(c, &okh, ok.p, sizeof(int));
+        cache.all_dirichlet = (okh == 1);
+        UG_CUDA(cudaStreamSynchronize(c.stream));
+        cache.nbrows = (int)rows.size();
+    }
+    return true;
+}
+
+// SCVF fluxes of the velocity field (null without one); they depend on the
+// field and the geometry only: computed again when the field changed.  False
+// in 2D, where there is no velocity field.
+template <int T>
+bool class_fluxes(Ctx &c, const AsmArgs &a, RowAsmCache &cache, const double *&flux)
+{
+    using CT = ClassTraits<T>;
+    using E = Elem<T>;
+    flux = nullptr;
+    if (a.vmodes <= 0) return true;
+    if constexpr (E::DIM == 3) {
+        const int ncell = a.cx * a.cy * a.cz;
+        const size_t nf = (size_t)ncell * CT::NC * E::NSCVF;
+        if (cache.flux.n < nf || cache.flux_version != a.vel_version) {
+            if (cache.flux.n < nf) cache.flux.alloc(nf);
+            const int ntab = CT::NC * CT::NF * a.vmodes;
+            DevBuf<double> tab;
+            tab.alloc(3 * (size_t)ntab);
+            UG_LAUNCH(c, k_flux_table<T>, div_up(ntab, 128), 128, 0, a.vmodes, a.vk, a.vc, cache.normal.p,
+                      cache.ipoff.p, tab.p);
+            UG_LAUNCH(c, k_scvf_flux<T>, div_up(ncell * CT::NC, 128), 128, 0, a.cx, a.cy, ncell, 1.0 / (double)a.cx,
+                      1.0 / (double)a.cy, 1.0 / (double)a.cz, a.vmodes, a.vk, a.vphase, a.vscale, tab.p, cache.flux.p);
+            // the table is freed on return: its kernel must have read it
+            UG_CUDA(cudaStreamSynchronize(c.stream));
+            cache.flux_version = a.vel_version;
+        }
+        flux = cache.flux.p;
+        return true;
+    } else {
+        return false;
+    }
+}
+
+template <class F>
+bool dispatch_rows(int elem_type, F &&f)
+{
+    switch (elem_type) {
+        case UG4GB_QUAD: return f(std::integral_constant<int, UG4GB_QUAD>());
+        case UG4GB_HEX: return f(std::integral_constant<int, UG4GB_HEX>());
+        case UG4GB_TET: return f(std::integral_constant<int, UG4GB_TET>());
+        default: return false;
+    }
+}
+
+AsmArgs with_cells(const Level &L, AsmArgs a)
+{
+    a.cx = L.nx - 1;
+    a.cy = L.ny - 1;
+    a.cz = (L.dim == 3) ? L.nz - 1 : 1;
+    return a;
+}
+
+template <int T, bool INST>
+void run_assemble_rows(Ctx &c, const Level &L, const AsmArgs &a, const ClassData<T> &cd, const double *flux,
+                       const RowAsmCache &cache)
+{
+    const int nint = (a.cx - 1) * (a.cy - 1) * ((L.dim == 3) ? a.cz - 1 : 1);
+    const size_t line_smem = sizeof(int) * (size_t)(L.nx + 1);
+    if (a.k_uniform && !flux && line_smem <= 32 * 1024) {
+        // every grid line, the boundary rows with it
+        const int nlines = L.ny * ((L.dim == 3) ? L.nz : 1);
+        UG_LAUNCH_PDL(c, (k_assemble_lines_uniform<T, INST>), div_up(nlines, kLinesPerBlock), 128, line_smem, a, cd,
+                      cache.volsum, a.k_value, L.bnd.p, nlines);
+    } else if (L.nv <= kSmallLevelRows) {
+        UG_LAUNCH_PDL(c, (k_assemble_rows_all<T, INST>), div_up(L.nv, 128), 128, 0, a, cd, flux, cache.volsum, L.bnd.p);
+    } else {
+        UG_LAUNCH_PDL(c, (k_assemble_rows<T, INST>), div_up(nint, 128), 128, 0, a, cd, flux, cache.volsum);
+        UG_LAUNCH_PDL(c, k_assemble_boundary_rows<T>, div_up(cache.nbrows, 8), 256, 0, a, cd, flux, L.bnd.p,
+                      cache.brows.p, cache.nbrows);
+    }
+}
+
+}  // namespace
+
+// Assembles level L row by row when it is a structured level (time-discrete:
+// with a Dirichlet boundary all around, whose rows are identity rows in both);
+// returns false (nothing launched) otherwise.
 bool launch_assemble_rows(Ctx &c, const Level &L, const AsmArgs &a_in, RowAsmCache &cache)
 {
-    if (!L.structured || a_in.inst || L.nx < 3 || L.ny < 3 || (L.dim == 3 && L.nz < 3)) return false;
-    bool done = false;
-    auto run = [&](auto tag) {
+    return dispatch_rows(L.elem_type, [&](auto tag) {
         constexpr int T = decltype(tag)::value;
-        using CT = ClassTraits<T>;
-        using E = Elem<T>;
-        const int cx = L.nx - 1, cy = L.ny - 1, cz = (L.dim == 3) ? L.nz - 1 : 1;
-        const int nint = (cx - 1) * (cy - 1) * ((L.dim == 3) ? cz - 1 : 1);
-        if (!cache.ready) {
-            DevBuf<double> A, vol, nrm, ipo;
-            DevBuf<int> ok;
-            A.alloc(CT::NC * E::K * E::K);
-            vol.alloc(CT::NC * E::K);
-            nrm.alloc(CT::NC * E::NSCVF * 3);
-            ipo.alloc(CT::NC * E::NSCVF * 3);
-            ok.alloc(1);
-            const int one = 1;
-            copy_in(c, ok.p, &one, sizeof(int));
-            UG_LAUNCH(c, k_class_data<T>, 1, 32, 0, L.coords.p, L.elems.p, A.p, vol.p, nrm.p, ipo.p, ok.p);
-            UG_LAUNCH(c, k_check_row_lengths<T>, div_up(nint, 256), 256, 0, cx, cy, cz, a_in.rowptr, ok.p);
-            cache.A.resize(CT::NC * E::K * E::K);
-            cache.vol.resize(CT::NC * E::K);
-            copy_out(c, cache.A.data(), A.p, sizeof(double) * cache.A.size());
-            copy_out(c, cache.vol.data(), vol.p, sizeof(double) * cache.vol.size());
-            int okh = 0;
-            copy_out(c, &okh, ok.p, sizeof(int));
-            // entries that vanish in exact arithmetic (on a Kuhn tetrahedron
-            // the couplings of its non-path edges) come out of the box-method
-            // sums as rounding noise of some 1e-16 of the largest entry: exact
-            // zeros here, so the solve format can leave their diagonals out
-            for (int p = 0; p < CT::NC; ++p) {
-                double *Ap = cache.A.data() + (size_t)p * E::K * E::K, big = 0.0;
-                for (int q = 0; q < E::K * E::K; ++q) big = std::max(big, std::fabs(Ap[q]));
-                for (int q = 0; q < E::K * E::K; ++q)
-                    if (std::fabs(Ap[q]) < 1e-14 * big) Ap[q] = 0.0;
-            }
-            cache.normal = std::move(nrm);
-            cache.ipoff = std::move(ipo);
-            cache.usable = (okh == 1);
-            cache.ready = true;
-        }
-        if (!cache.usable) return;
         ClassData<T> cd;
-        std::memcpy(&cd.A[0][0][0], cache.A.data(), sizeof(cd.A));
-        std::memcpy(&cd.vol[0][0], cache.vol.data(), sizeof(cd.vol));
-        AsmArgs a = a_in;
-        a.cx = cx;
-        a.cy = cy;
-        a.cz = cz;
-        if (cache.nbrows == 0) {
-            // once per level: the interior rows' SCV volume sum and the list of
-            // the rows on the box boundary
-            DevBuf<double> vs;
-            vs.alloc(1);
-            UG_LAUNCH(c, k_row_volsum<T>, 1, 32, 0, a, cd, vs.p);
-            copy_out(c, &cache.volsum, vs.p, sizeof(double));
-            const int nx = L.nx, ny = L.ny, nz = (L.dim == 3) ? L.nz : 1;
-            std::vector<int> rows;
-            for (int k = 0; k < nz; ++k)
-                for (int j = 0; j < ny; ++j)
-                    for (int i = 0; i < nx; ++i)
-                        if (i == 0 || i == nx - 1 || j == 0 || j == ny - 1 || (L.dim == 3 && (k == 0 || k == nz - 1)))
-                            rows.push_back(i + nx * (j + ny * k));
-            cache.brows.alloc(rows.size());
-            copy_in(c, cache.brows.p, rows.data(), sizeof(int) * rows.size());
-            UG_CUDA(cudaStreamSynchronize(c.stream));
-            cache.nbrows = (int)rows.size();
+        if (!class_data<T>(c, L, cache, cd)) return false;
+        const AsmArgs a = with_cells(L, a_in);
+        if (cache.row_check == 0) {
+            const int nint = (a.cx - 1) * (a.cy - 1) * ((L.dim == 3) ? a.cz - 1 : 1);
+            DevBuf<int> ok;
+            ok.alloc(1);
+            int okh = 1;
+            copy_in(c, ok.p, &okh, sizeof(int));
+            UG_LAUNCH(c, k_check_row_lengths<T>, div_up(nint, 256), 256, 0, a.cx, a.cy, a.cz, a.rowptr, ok.p);
+            copy_out(c, &okh, ok.p, sizeof(int));
+            cache.row_check = (okh == 1) ? 1 : -1;
         }
-        const double *flux = nullptr;
-        if (a.vmodes > 0) {
-            if constexpr (E::DIM == 3) {
-                const int ncell = a.cx * a.cy * a.cz;
-                const size_t nf = (size_t)ncell * CT::NC * E::NSCVF;
-                // the fluxes depend on the velocity field and the geometry
-                // only: computed again when the field changed
-                if (cache.flux.n < nf || cache.flux_version != a.vel_version) {
-                    if (cache.flux.n < nf) cache.flux.alloc(nf);
-                    const int ntab = CT::NC * CT::NF * a.vmodes;
-                    DevBuf<double> tab;
-                    tab.alloc(3 * (size_t)ntab);
-                    UG_LAUNCH(c, k_flux_table<T>, div_up(ntab, 128), 128, 0, a.vmodes, a.vk, a.vc, cache.normal.p,
-                              cache.ipoff.p, tab.p);
-                    UG_LAUNCH(c, k_scvf_flux<T>, div_up(ncell * CT::NC, 128), 128, 0, a.cx, a.cy, ncell,
-                              1.0 / (double)a.cx, 1.0 / (double)a.cy, 1.0 / (double)a.cz, a.vmodes, a.vk, a.vphase,
-                              a.vscale, tab.p, cache.flux.p);
-                    // the table is freed on return: its kernel must have read it
-                    UG_CUDA(cudaStreamSynchronize(c.stream));
-                    cache.flux_version = a.vel_version;
-                }
-                flux = cache.flux.p;
-            } else {
-                return;   // no 2D velocity field
-            }
-        }
-        const size_t line_smem = sizeof(int) * (size_t)(L.nx + 1);
-        if (a.k_uniform && !flux && line_smem <= 32 * 1024) {
-            // every grid line, the boundary rows with it
-            const int nlines = L.ny * ((L.dim == 3) ? L.nz : 1);
-            UG_LAUNCH_PDL(c, k_assemble_lines_uniform<T>, div_up(nlines, kLinesPerBlock), 128, line_smem, a, cd,
-                      cache.volsum, a.k_value, L.bnd.p, nlines);
-        } else {
-            if (L.nv <= kSmallLevelRows) {
-                UG_LAUNCH_PDL(c, k_assemble_rows_all<T>, div_up(L.nv, 128), 128, 0, a, cd, flux, cache.volsum, L.bnd.p);
-            } else {
-                UG_LAUNCH_PDL(c, k_assemble_rows<T>, div_up(nint, 128), 128, 0, a, cd, flux, cache.volsum);
-                UG_LAUNCH_PDL(c, k_assemble_boundary_rows<T>, div_up(cache.nbrows, 8), 256, 0, a, cd, flux, L.bnd.p,
-                          cache.brows.p, cache.nbrows);
-            }
-        }
-        done = true;
-    };
-    switch (L.elem_type) {
-        case UG4GB_QUAD: run(std::integral_constant<int, UG4GB_QUAD>()); break;
-        case UG4GB_HEX: run(std::integral_constant<int, UG4GB_HEX>()); break;
-        case UG4GB_TET: run(std::integral_constant<int, UG4GB_TET>()); break;
-        default: break;
-    }
-    return done;
+        if (cache.row_check < 0 || (a.inst && !cache.all_dirichlet)) return false;
+        const double *flux;
+        if (!class_fluxes<T>(c, a, cache, flux)) return false;
+        if (a.inst) run_assemble_rows<T, true>(c, L, a, cd, flux, cache);
+        else run_assemble_rows<T, false>(c, L, a, cd, flux, cache);
+        return true;
+    });
+}
+
+bool launch_defect_rows(Ctx &c, const Level &L, const AsmArgs &a_in, RowAsmCache &cache)
+{
+    return dispatch_rows(L.elem_type, [&](auto tag) {
+        constexpr int T = decltype(tag)::value;
+        ClassData<T> cd;
+        if (!class_data<T>(c, L, cache, cd) || !cache.all_dirichlet) return false;
+        const AsmArgs a = with_cells(L, a_in);
+        const double *flux;
+        if (!class_fluxes<T>(c, a, cache, flux)) return false;
+        UG_LAUNCH(c, k_defect_rows<T>, div_up(L.nv, 128), 128, 0, a, cd, flux, cache.volsum);
+        return true;
+    });
+}
+
+bool launch_grad_logk_rows(Ctx &c, const Level &L, const double *K, const double *u, const double *lam, double *g,
+                           RowAsmCache &cache)
+{
+    return dispatch_rows(L.elem_type, [&](auto tag) {
+        constexpr int T = decltype(tag)::value;
+        ClassData<T> cd;
+        if (!class_data<T>(c, L, cache, cd)) return false;
+        const AsmArgs a = with_cells(L, AsmArgs{});
+        const int ncell = a.cx * a.cy * a.cz;
+        UG_LAUNCH(c, k_grad_logk_cells<T>, div_up(ncell, 128), 128, 0, cd, a.cx, a.cy, ncell, L.bnd.p, K, u, lam, g);
+        return true;
+    });
+}
+
+bool launch_grad_source_rows(Ctx &c, const Level &L, const double *lam, double *g, RowAsmCache &cache)
+{
+    return dispatch_rows(L.elem_type, [&](auto tag) {
+        constexpr int T = decltype(tag)::value;
+        ClassData<T> cd;
+        if (!class_data<T>(c, L, cache, cd) || !cache.all_dirichlet) return false;
+        UG_LAUNCH(c, k_grad_source_rows, div_up(L.nv, 256), 256, 0, cache.volsum, L.bnd.p, lam, L.nv, g);
+        return true;
+    });
 }
 
 }  // namespace ug4gb
