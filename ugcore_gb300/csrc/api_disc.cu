@@ -103,6 +103,9 @@ void disc_assemble(ug4gb_disc *d, int level, ug4gb_matrix *A, double *b, const T
     }
     // structured levels: row by row, every value written once
     if (c.row_assembly && launch_assemble_rows(c, L, a, class_cache(d, level))) return;
+    // unstructured simplices: row by row from the elements around a vertex
+    if (D.gather.size() < d->g->lev.size()) D.gather.resize(d->g->lev.size());
+    if (c.row_assembly && launch_assemble_gather(c, L, a, D.gather[level])) return;
     if (!fresh) UG_CUDA(cudaMemsetAsync(A->A.val.p, 0, sizeof(double) * (size_t)A->A.nnz, c.stream));
     if (b) UG_CUDA(cudaMemsetAsync(b, 0, sizeof(double) * (size_t)L.nv, c.stream));
     launch_assemble(c, L, a);

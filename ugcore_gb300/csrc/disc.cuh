@@ -69,6 +69,17 @@ bool launch_defect_rows(Ctx &c, const Level &L, const AsmArgs &a, RowAsmCache &c
 bool launch_grad_logk_rows(Ctx &c, const Level &L, const double *K, const double *u, const double *lam, double *g,
                            RowAsmCache &cache);
 bool launch_grad_source_rows(Ctx &c, const Level &L, const double *lam, double *g, RowAsmCache &cache);
+// Unstructured simplex levels without convection (k_fv1_gather.cu): every
+// value of A and b written once, Dirichlet rows included; false, launching
+// nothing, where it does not apply.  The lists depend on the mesh only.
+struct GatherCache {
+    bool ready = false;
+    DevBuf<int> vptr;                   // per vertex: its range in adj
+    DevBuf<unsigned> adj, slots;        // per vertex and element: 4 * element + corner; corner positions in the row
+    size_t smem = 0;                    // shared memory of a block's rows
+    DevBuf<double> ws;                  // per element: off-diagonal entries, SCV volume
+};
+bool launch_assemble_gather(Ctx &c, const Level &L, const AsmArgs &a, GatherCache &g);
 void launch_dirichlet(Ctx &c, const Level &L, Csr &A, double *b);
 // d = defect of a.u on level L (a.d must be zero on entry; Dirichlet rows 0);
 // stationary, or instationary with a.inst and the scalings of AsmArgs

@@ -100,6 +100,7 @@ struct DiscImpl {
     int f_kind = 0;                        // 0 none, 1 array, 2 seeded uniform
     uint64_t f_seed = 0;
     std::vector<RowAsmCache> rows;         // per level: class geometry of the row-wise assembly
+    std::vector<GatherCache> gather;       // per level: lists of the unstructured row-wise assembly
 };
 
 template <class V>
@@ -255,7 +256,7 @@ struct ug4gb_solver {
     // captured solve graph: the prologue, then the iteration loop
     cudaGraphExec_t iter_graph = nullptr;
     int64_t iter_kernels = 0;       // kernels of one loop body
-    int64_t prologue_kernels = 0;   // kernels before the loop (entry test included)
+    int64_t prologue_kernels = 0;   // kernels outside the loop (entry test and epilogue included)
     void *pinned = nullptr;         // page-locked read-back of the scalars and the history
     size_t pinned_bytes = 0;
     const double *graph_x = nullptr;
