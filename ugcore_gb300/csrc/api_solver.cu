@@ -93,8 +93,9 @@ const double *precond(ug4gb_solver *s, const double *d, const double *r_rho, int
         return d;
     }
     bool fused = false;
-    // CG: d is r, whose FP32 copy krylov_start / cg_update already wrote
-    const bool ready = s->kind == UG4GB_SOLVER_CG && s->pre->impl->top_defect_buffer() != nullptr;
+    // the kernels that wrote d (krylov_start / cg_update, bicg_p / bicg_x_s)
+    // already wrote its FP32 copy
+    const bool ready = s->pre->impl->top_defect_buffer() != nullptr;
     const double *z = s->pre->impl->apply(c, d, skip, r_rho, &red, rho_kind, fused, ready);
     if (r_rho && !fused) rho_dot<double>(c, s->n, z, r_rho, rho_kind, red);
     return z;
@@ -116,18 +117,16 @@ void bicg_iteration(ug4gb_solver *s, double *x, double *r)
     RedArgs red = red_of(s);
     const int n = s->n;
     c.prof_tag = "K";
-    bicg_restart(c, n, r, s->r0.p, s->p.p, s->v.p, red);
-    bicg_rho(c, n, s->r0.p, r, red);
-    bicg_p(c, n, r, s->p.p, s->v.p, red);
+    float *d32 = s->pre ? s->pre->impl->top_defect_buffer() : nullptr;
+    bicg_p(c, n, r, s->p.p, s->v.p, s->r0.p, d32, red);
     const double *q = precond(s, s->p.p, nullptr, 0);
     c.prof_tag = "K";
     bicg_spmv_dot_t<double>(c, s->A->op, q, s->v.p, s->r0.p, red);
-    bicg_x_s<double>(c, n, x, q, r, s->v.p, s->s.p, red);
-    bicg_s_to_r(c, n, s->s.p, r, red);
+    bicg_x_s<double>(c, n, x, q, r, s->v.p, s->s.p, d32, red);
     q = precond(s, s->s.p, nullptr, 0);
     c.prof_tag = "K";
     bicg_spmv_2dot_t<double>(c, s->A->op, q, s->t.p, s->s.p, red);
-    bicg_x_r<double>(c, n, x, q, s->s.p, s->t.p, r, red);
+    bicg_x_r<double>(c, n, x, q, s->s.p, s->t.p, r, s->r0.p, red);
 }
 
 // the entry test after the prologue and the last node of the loop body:
@@ -151,13 +150,21 @@ void prologue(ug4gb_solver *s, double *x, double *r)
     RedArgs red = red_of(s);
     c.prof_tag = "K";
     krylov_start(c, s->A->op, x, r, red,
-                 s->kind == UG4GB_SOLVER_CG && s->pre ? s->pre->impl->top_defect_buffer() : nullptr);
+                 s->kind == UG4GB_SOLVER_CG && s->pre ? s->pre->impl->top_defect_buffer() : nullptr,
+                 s->kind == UG4GB_SOLVER_BICGSTAB);
     if (s->kind == UG4GB_SOLVER_CG) cg_iteration(s, x, r, true);
+}
+
+// after the loop: BiCGStab's defect where it ended at a half step
+void epilogue(ug4gb_solver *s, double *r)
+{
+    if (s->kind == UG4GB_SOLVER_BICGSTAB) bicg_s_to_r(s->ctx->c, s->n, s->s.p, r, red_of(s));
 }
 
 // The whole solve as one graph: the prologue and k_loop_cond (captured), then
 // a conditional WHILE node whose body is one Krylov iteration (multigrid
-// cycle included) followed by k_loop_cond.  The loop ends when the
+// cycle included) followed by k_loop_cond, then the epilogue (captured).  The
+// loop ends when the
 // device-side StdConvCheck (or a breakdown) sets done, at the latest after
 // max_steps iterations; a solve that ends in the prologue skips it.
 void build_loop_graph(ug4gb_solver *s, double *x, double *r)
@@ -221,6 +228,18 @@ void build_loop_graph(ug4gb_solver *s, double *x, double *r)
         cudaGraph_t tmp;
         UG_CUDA(cudaStreamEndCapture(c.stream, &tmp));
         s->iter_kernels = c.launches - body_start;
+        if (s->kind == UG4GB_SOLVER_BICGSTAB) {
+            const int64_t end_start = c.launches;
+            UG_CUDA(cudaStreamBeginCaptureToGraph(c.stream, g, &node, nullptr, 1, cudaStreamCaptureModeThreadLocal));
+            try {
+                epilogue(s, r);
+            } catch (...) {
+                cudaStreamEndCapture(c.stream, &tmp);
+                throw;
+            }
+            UG_CUDA(cudaStreamEndCapture(c.stream, &tmp));
+            s->prologue_kernels += c.launches - end_start;
+        }
         UG_CUDA(cudaGraphInstantiate(&exec, g, 0));
     } catch (...) {
         c.launches = before;
@@ -266,6 +285,7 @@ void run(ug4gb_solver *s, double *x, double *r)
             iteration(s, x, r);
             read_flags(s, &done);
         }
+        epilogue(s, r);
     } else {
         int pre_gen = s->pre ? s->pre->gen : -1;
         if (!s->iter_graph || s->graph_x != x || s->graph_r != r || s->graph_pre_gen != pre_gen) {

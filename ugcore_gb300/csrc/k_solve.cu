@@ -480,42 +480,124 @@ void prolong_apply(Ctx &c, const OpMat<V> &P, const V *scc, V *sc, const V *dfac
 
 // ------------------------------------------- grid-index transfers ---------
 
-// The transfer kernels run in one of two thread layouts.  TILED: a 2D grid
-// of 32 x 8 vertex tiles of the (x, y) plane, each thread walking z with the
-// grid's z stride, so that a thread knows its grid indices without integer
-// divisions by runtime extents (FP32 levels: +15% on the 129^3 prolongation).
-// Else one vertex per thread of a 1D grid-stride loop, every lane busy:
-// FP64 levels are bound by the FP64 issue rate, where a partly filled warp
-// costs as much as a full one.
-// t = P scc for fine vertex (i, j, k); sc += t; w = t * dfac (k_prolong on the assembled P)
-template <class V>
-__device__ __forceinline__ void prolong_row(const GridPair &g, const V *__restrict__ scc, V *__restrict__ sc,
-                                            const V *__restrict__ dfac, V *__restrict__ w, int i, int j, int k)
-{
-    const int f = i + g.nx * (j + g.ny * k);
-    V t = prolong_value<V>(g, scc, i, j, k);
-    if (g.dprol != 1.0) t = mul_rn(t, (V)g.dprol);
-    sc[f] = add_rn(sc[f], t);
-    if (w) w[f] = mul_rn(t, dfac[f]);
-}
+// Division by a run-time constant d >= 1 of 0 <= n < 2^31 as a multiplication
+// and a shift (Granlund and Montgomery, "Division by invariant integers using
+// multiplication", 1994): m = ceil(2^(31+s) / d) with s = ceil(log2 d).
+struct FastDiv {
+    unsigned d, m, s;
+    explicit FastDiv(int n) : d((unsigned)n), m(0), s(0)
+    {
+        while ((1u << s) < d) ++s;
+        m = (unsigned)((((unsigned long long)1 << (31 + s)) + d - 1) / d);
+    }
+    __device__ __forceinline__ int div(int n) const
+    {
+        return (int)(((unsigned long long)(unsigned)n * m) >> (31 + s));
+    }
+};
 
-template <class V, bool TILED>
-__global__ void __launch_bounds__(NT) k_prolong_grid(GridPair g, const V *__restrict__ scc, V *__restrict__ sc,
+// t = P scc ; sc += t ; w = t * dfac (k_prolong on the assembled P), the
+// parents and weights of prolong_value in its order.  A thread takes the two
+// fine vertices 2I and 2I + 1 of a grid line: they share the coarse values
+// of the lines around them, and the parities that choose the parents are those
+// of the line, so a warp does not diverge; all loads of a pair are issued before
+// its sums, the Jacobi factors of a thread's first pair (no solve kernel writes
+// them) before the launch wait.  One vertex per thread, with loops over its 1
+// to 8 parents, took 46 us on the 129^3 FP64 level and 54 us on the 193^3 FP32
+// one.
+template <class V>
+__global__ void __launch_bounds__(NT) k_prolong_grid(GridPair g, FastDiv pairs, FastDiv lines, int npairs,
+                                                     const V *__restrict__ scc, V *__restrict__ sc,
                                                      const V *__restrict__ dfac, V *__restrict__ w, const int *skip)
 {
-    PDL_ENTRY();
+    const int stride = gridDim.x * NT;
+    int q = blockIdx.x * NT + threadIdx.x;
+    // fine vertices f and, if two, f + 1 of pair q; its line
+    auto locate = [&](int qq, int &line, int &I, int &f, bool &two) {
+        line = pairs.div(qq);
+        I = qq - line * (int)pairs.d;
+        f = 2 * I + g.nx * line;
+        two = 2 * I + 1 < g.nx;
+    };
+    int line = 0, I = 0, f = 0;
+    bool two = false;
+    V df0 = (V)0, df1 = (V)0;
+    pdl_trigger();
+    if (q < npairs) {
+        locate(q, line, I, f, two);
+        if (w) {
+            df0 = dfac[f];
+            if (two) df1 = dfac[f + 1];
+        }
+    }
+    pdl_wait();
     if (skip && *skip) return;
-    if constexpr (TILED) {
-        const int i = blockIdx.x * 32 + threadIdx.x, j = blockIdx.y * 8 + threadIdx.y;
-        if (i >= g.nx || j >= g.ny) return;
-        for (int k = blockIdx.z; k < g.nz; k += gridDim.z) prolong_row<V>(g, scc, sc, dfac, w, i, j, k);
-    } else {
-        const int n = g.nx * g.ny * g.nz, stride = gridDim.x * NT;
-        for (int f = blockIdx.x * NT + threadIdx.x; f < n; f += stride)
-            prolong_row<V>(g, scc, sc, dfac, w, f % g.nx, (f / g.nx) % g.ny, f / (g.nx * g.ny));
+    for (bool first = true; q < npairs; q += stride, first = false) {
+        if (!first) {
+            locate(q, line, I, f, two);
+            if (w) {
+                df0 = dfac[f];
+                if (two) df1 = dfac[f + 1];
+            }
+        }
+        const int k = lines.div(line), j = line - k * (int)lines.d, i = 2 * I;
+        const int p1 = j & 1, p2 = k & 1, J = j >> 1, K = k >> 1, I1 = two ? 1 : 0;
+        V s0 = sc[f], s1 = two ? sc[f + 1] : (V)0;
+        const bool edge = j == 0 || j == g.ny - 1 || (g.dim == 3 && (k == 0 || k == g.nz - 1));
+        // on the boundary: only a coinciding coarse vertex, weight 1
+        const bool b0 = edge || i == 0 || i == g.nx - 1, b1 = edge;
+        const V *c = scc + I + g.cnx * (J + g.cny * K);
+        V t0 = (V)0, t1 = (V)0;
+        if (g.tet) {
+            const V *e = c + g.cnx * (p1 + g.cny * p2);
+            const bool odd = (p1 | p2) != 0;
+            const V w0 = odd ? (b0 ? (V)0 : (V)0.5) : (V)1, w1 = b1 ? (V)0 : (V)0.5;
+            const V c0 = c[0], e0 = e[0], e1 = e[I1];
+            t0 = fma_rn(w0, c0, t0);
+            if (odd) t0 = fma_rn(w0, e0, t0);
+            t1 = fma_rn(w1, c0, t1);
+            t1 = fma_rn(w1, e1, t1);
+        } else {
+            const V w0 = b0 ? ((p1 | p2) ? (V)0 : (V)1) : grid_weight<V>(p1 + p2);
+            const V w1 = b1 ? (V)0 : grid_weight<V>(1 + p1 + p2);
+            // the 1, 2 or 4 lines of coarse vertices around this line, in
+            // increasing y, then z
+            V a[4] = {}, b[4] = {};
+#pragma unroll
+            for (int m = 0; m < 4; ++m)
+                if ((m & 1) <= p1 && (m >> 1) <= p2) {
+                    const V *e = c + g.cnx * ((m & 1) + g.cny * (m >> 1));
+                    a[m] = e[0];
+                    b[m] = e[I1];
+                }
+#pragma unroll
+            for (int m = 0; m < 4; ++m)
+                if ((m & 1) <= p1 && (m >> 1) <= p2) {
+                    t0 = fma_rn(w0, a[m], t0);
+                    t1 = fma_rn(w1, a[m], t1);
+                    t1 = fma_rn(w1, b[m], t1);
+                }
+        }
+        if (g.dprol != 1.0) {
+            t0 = mul_rn(t0, (V)g.dprol);
+            t1 = mul_rn(t1, (V)g.dprol);
+        }
+        sc[f] = add_rn(s0, t0);
+        if (w) w[f] = mul_rn(t0, df0);
+        if (two) {
+            sc[f + 1] = add_rn(s1, t1);
+            if (w) w[f + 1] = mul_rn(t1, df1);
+        }
     }
 }
 
+// The restriction runs in one of two thread layouts.  TILED: a 2D grid
+// of 32 x 8 vertex tiles of the (x, y) plane, each thread walking z with the
+// grid's z stride, so that a thread knows its grid indices without integer
+// divisions by runtime extents (FP32 levels).
+// Else one vertex per thread of a 1D grid-stride loop, every lane busy:
+// FP64 levels are bound by the FP64 issue rate, where a partly filled warp
+// costs as much as a full one.
 template <class V, bool TILED>
 __global__ void __launch_bounds__(NT) k_restrict_grid(GridPair g, const V *__restrict__ d, V *__restrict__ dc,
                                                       const int *skip)
@@ -546,12 +628,9 @@ static dim3 transfer_grid(const Ctx &c, int nx, int ny, int nz)
 template <class V>
 void prolong_grid(Ctx &c, const GridPair &g, const V *scc, V *sc, const V *dfac, V *w, const int *skip)
 {
-    if constexpr (sizeof(V) == 4)
-        UG_LAUNCH_PDL(c, (k_prolong_grid<V, true>), transfer_grid(c, g.nx, g.ny, g.nz), dim3(32, 8), 0, g, scc, sc,
-                      dfac, w, skip);
-    else
-        UG_LAUNCH_PDL(c, (k_prolong_grid<V, false>), row_grid(c, g.nx * g.ny * g.nz), NT, 0, g, scc, sc, dfac, w,
-                      skip);
+    const int per = (g.nx + 1) / 2, npairs = per * g.ny * g.nz;
+    UG_LAUNCH_PDL(c, k_prolong_grid<V>, row_grid(c, npairs), NT, 0, g, FastDiv(per), FastDiv(g.ny), npairs, scc, sc,
+                  dfac, w, skip);
 }
 
 template <class V>
@@ -691,10 +770,50 @@ template void residual_update<float, double>(Ctx &, const OpMat<float> &, const 
                                              float *, int, const int *);
 
 // ------------------------------------------------------------ Krylov -----
-// r = b - A x (r holds b on entry); start the convergence check with |r|
+// (BiCGStab::apply_return_defect, bicgstab.h:158-390).  A restart at the top
+// of an iteration comes from the previous iteration's orthogonality test
+// (ks->restart) or from the fixed restart period (step % num_restarts == 0,
+// bicgstab.h:161-170; the check counts half steps).
+__device__ __forceinline__ bool bicg_restarting(const KScal *ks)
+{
+    return ks->restart || (ks->num_restarts > 0 && ks->step % ks->num_restarts == 0);
+}
+
+// The scalars at the top of an iteration from r0r = (r0, r) and rr = (r, r),
+// called by the kernel that wrote r (there is no pass of its own over r0 and
+// r for them): rho, beta, whether this iteration restarts (k_bicg_p then
+// sets r0 = p = r, so (r0, r) is (r, r)).
+__device__ __forceinline__ void bicg_top(KScal *ks, double r0r, double rr)
+{
+    if (ks->done) return;
+    const bool again = bicg_restarting(ks);
+    ks->restarted = again ? 1 : 0;
+    if (again) {
+        ks->alpha = 0.0;
+        ks->omega = 1.0;
+        ks->rho = 1.0;
+        ks->norm_r0 = ks->dcur;
+        ks->restart = 0;
+    }
+    const double tot = again ? rr : r0r;
+    const double rho_old = ks->rho;
+    ks->rho_old = rho_old;
+    ks->rho = tot;
+    // restart in the next iteration when (r, r0) <= minOrtho |r| |r0|
+    // (bicgstab.h:206-215)
+    if (fabs(tot) / (ks->dcur * ks->norm_r0) <= ks->min_ortho) ks->restart = 1;
+    if (rho_old == 0.0) {
+        ks->fail = 1;
+        ks->done = 1;
+    }
+    ks->beta = (tot / rho_old) * (ks->alpha / ks->omega);
+}
+
+// r = b - A x (r holds b on entry); start the convergence check with |r|;
+// bicg: and BiCGStab's first iteration, which restarts
 template <class MV>
 __global__ void __launch_bounds__(NT) k_krylov_start(MV A, const double *__restrict__ x, double *__restrict__ r,
-                                                     float *__restrict__ r32, RedArgs red)
+                                                     float *__restrict__ r32, bool bicg, RedArgs red)
 {
     PDL_ENTRY();
     double sum = 0.0;
@@ -718,13 +837,14 @@ __global__ void __launch_bounds__(NT) k_krylov_start(MV A, const double *__restr
         ks->restart = 1;
         if (ks->hist && ks->hist_cap > 0) ks->hist[0] = d;
         if (conv_ended(ks)) ks->done = 1;
+        if (bicg) bicg_top(ks, tot[0], tot[0]);
     });
 }
 
-void krylov_start(Ctx &c, const OpMat<double> &A, const double *x, double *r, RedArgs red, float *r32)
+void krylov_start(Ctx &c, const OpMat<double> &A, const double *x, double *r, RedArgs red, float *r32, bool bicg)
 {
     with_mv(A, [&](auto mv) {
-        UG_LAUNCH_PDL(c, k_krylov_start<decltype(mv)>, row_grid(c, A.nrows), NT, 0, mv, x, r, r32, red);
+        UG_LAUNCH_PDL(c, k_krylov_start<decltype(mv)>, row_grid(c, A.nrows), NT, 0, mv, x, r, r32, bicg, red);
     });
 }
 
@@ -892,83 +1012,28 @@ template void copy_z<double>(Ctx &, int, const double *, double *, const int *);
 template void copy_z<float>(Ctx &, int, const float *, double *, const int *);
 
 // ------------------------------------------------------------ BiCGStab ---
-// (BiCGStab::apply_return_defect, bicgstab.h:158-390).  A restart at the top
-// of an iteration comes from the previous iteration's orthogonality test
-// (ks->restart) or from the fixed restart period (step % num_restarts == 0,
-// bicgstab.h:161-170; the check counts half steps).
-__device__ __forceinline__ bool bicg_restarting(const KScal *ks)
-{
-    return ks->restart || (ks->num_restarts > 0 && ks->step % ks->num_restarts == 0);
-}
-
-__global__ void k_bicg_restart(int n, const double *__restrict__ r, double *__restrict__ r0, double *__restrict__ p,
-                               double *__restrict__ v, KScal *ks)
-{
-    PDL_ENTRY();
-    if (ks->done || !bicg_restarting(ks)) return;
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) {
-        r0[i] = r[i];
-        p[i] = 0.0;
-        v[i] = 0.0;
-    }
-}
-
-void bicg_restart(Ctx &c, int n, const double *r, double *r0, double *p, double *v, RedArgs red)
-{
-    UG_LAUNCH_PDL(c, k_bicg_restart, div_up(n, NT), NT, 0, n, r, r0, p, v, red.ks);
-}
-
-__global__ void __launch_bounds__(NT) k_bicg_rho(int n, const double *__restrict__ r0, const double *__restrict__ r,
-                                                 RedArgs red)
-{
-    PDL_ENTRY();
-    KScal *ks = red.ks;
-    if (ks->done) return;
-    double sum = 0.0;
-    const int stride = gridDim.x * NT;
-    for (int i = blockIdx.x * NT + threadIdx.x; i < n; i += stride) sum += r0[i] * r[i];
-    double v[1] = {sum};
-    grid_reduce<NT, 1>(v, red.partials, red.counter, [&](const double(&tot)[1]) {
-        if (bicg_restarting(ks)) {
-            ks->alpha = 0.0;
-            ks->omega = 1.0;
-            ks->rho = 1.0;
-            ks->norm_r0 = ks->dcur;
-            ks->restart = 0;
-        }
-        const double rho_old = ks->rho;
-        ks->rho_old = rho_old;
-        ks->rho = tot[0];
-        // restart in the next iteration when (r, r0) <= minOrtho |r| |r0|
-        // (bicgstab.h:206-215)
-        if (fabs(tot[0]) / (ks->dcur * ks->norm_r0) <= ks->min_ortho) ks->restart = 1;
-        if (rho_old == 0.0) {
-            ks->fail = 1;
-            ks->done = 1;
-        }
-        ks->beta = (tot[0] / rho_old) * (ks->alpha / ks->omega);
-    });
-}
-
-void bicg_rho(Ctx &c, int n, const double *r0, const double *r, RedArgs red)
-{
-    UG_LAUNCH_PDL(c, k_bicg_rho, row_grid(c, n), NT, 0, n, r0, r, red);
-}
-
-__global__ void k_bicg_p(int n, const double *__restrict__ r, double *__restrict__ p, const double *__restrict__ v,
-                         const KScal *ks)
+// p = r + beta p - beta omega v; a restart: r0 = p = r.  Optionally p32 =
+// (float) p, the FP32 defect the mixed-precision multigrid starts from.
+__global__ void __launch_bounds__(NT) k_bicg_p(int n, const double *__restrict__ r, double *__restrict__ p,
+                                               const double *__restrict__ v, double *__restrict__ r0,
+                                               float *__restrict__ p32, const KScal *ks)
 {
     PDL_ENTRY();
     if (ks->done) return;
+    const bool again = ks->restarted != 0;
     const double beta = ks->beta, bo = -ks->beta * ks->omega;
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) p[i] = 1.0 * r[i] + beta * p[i] + bo * v[i];
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const double rv = r[i];
+    const double pv = again ? rv : 1.0 * rv + beta * p[i] + bo * v[i];
+    p[i] = pv;
+    if (again) r0[i] = rv;
+    if (p32) p32[i] = f64_to_f32(pv);
 }
 
-void bicg_p(Ctx &c, int n, const double *r, double *p, const double *v, RedArgs red)
+void bicg_p(Ctx &c, int n, const double *r, double *p, const double *v, double *r0, float *p32, RedArgs red)
 {
-    UG_LAUNCH_PDL(c, k_bicg_p, div_up(n, NT), NT, 0, n, r, p, v, red.ks);
+    UG_LAUNCH_PDL(c, k_bicg_p, div_up(n, NT), NT, 0, n, r, p, v, r0, p32, red.ks);
 }
 
 template <class MV, class ZT>
@@ -1005,10 +1070,11 @@ void bicg_spmv_dot_t(Ctx &c, const OpMat<double> &A, const ZT *q, double *v, con
 template void bicg_spmv_dot_t<double>(Ctx &, const OpMat<double> &, const double *, double *, const double *, RedArgs);
 template void bicg_spmv_dot_t<float>(Ctx &, const OpMat<double> &, const float *, double *, const double *, RedArgs);
 
+// x += alpha q ; s = r - alpha v ; |s| -> check; optionally s32 = (float) s
 template <class ZT>
 __global__ void __launch_bounds__(NT) k_bicg_x_s(int n, double *__restrict__ x, const ZT *__restrict__ q,
                                                  const double *__restrict__ r, const double *__restrict__ v,
-                                                 double *__restrict__ s, RedArgs red)
+                                                 double *__restrict__ s, float *__restrict__ s32, RedArgs red)
 {
     PDL_ENTRY();
     KScal *ks = red.ks;
@@ -1020,6 +1086,7 @@ __global__ void __launch_bounds__(NT) k_bicg_x_s(int n, double *__restrict__ x, 
         x[i] = 1.0 * x[i] + alpha * (double)q[i];
         double sv = 1.0 * r[i] + (-alpha) * v[i];
         s[i] = sv;
+        if (s32) s32[i] = f64_to_f32(sv);
         sum += sv * sv;
     }
     double vv[1] = {sum};
@@ -1027,13 +1094,17 @@ __global__ void __launch_bounds__(NT) k_bicg_x_s(int n, double *__restrict__ x, 
 }
 
 template <class ZT>
-void bicg_x_s(Ctx &c, int n, double *x, const ZT *q, const double *r, const double *v, double *s, RedArgs red)
+void bicg_x_s(Ctx &c, int n, double *x, const ZT *q, const double *r, const double *v, double *s, float *s32,
+              RedArgs red)
 {
-    UG_LAUNCH_PDL(c, k_bicg_x_s<ZT>, row_grid(c, n), NT, 0, n, x, q, r, v, s, red);
+    UG_LAUNCH_PDL(c, k_bicg_x_s<ZT>, row_grid(c, n), NT, 0, n, x, q, r, v, s, s32, red);
 }
-template void bicg_x_s<double>(Ctx &, int, double *, const double *, const double *, const double *, double *, RedArgs);
-template void bicg_x_s<float>(Ctx &, int, double *, const float *, const double *, const double *, double *, RedArgs);
+template void bicg_x_s<double>(Ctx &, int, double *, const double *, const double *, const double *, double *, float *,
+                               RedArgs);
+template void bicg_x_s<float>(Ctx &, int, double *, const float *, const double *, const double *, double *, float *,
+                              RedArgs);
 
+// after the loop: a solve that ended at a half step returns s as the defect
 __global__ void k_bicg_s_to_r(int n, const double *__restrict__ s, double *__restrict__ r, const KScal *ks)
 {
     PDL_ENTRY();
@@ -1044,7 +1115,7 @@ __global__ void k_bicg_s_to_r(int n, const double *__restrict__ s, double *__res
 
 void bicg_s_to_r(Ctx &c, int n, const double *s, double *r, RedArgs red)
 {
-    UG_LAUNCH_PDL(c, k_bicg_s_to_r, div_up(n, NT), NT, 0, n, s, r, red.ks);
+    UG_LAUNCH(c, k_bicg_s_to_r, div_up(n, NT), NT, 0, n, s, r, red.ks);
 }
 
 template <class MV, class ZT>
@@ -1083,40 +1154,47 @@ template void bicg_spmv_2dot_t<double>(Ctx &, const OpMat<double> &, const doubl
                                        RedArgs);
 template void bicg_spmv_2dot_t<float>(Ctx &, const OpMat<double> &, const float *, double *, const double *, RedArgs);
 
+// x += omega q ; r = s - omega t ; |r| -> check, and (r0, r) for the next
+// iteration (bicg_top)
 template <class ZT>
 __global__ void __launch_bounds__(NT) k_bicg_x_r(int n, double *__restrict__ x, const ZT *__restrict__ q,
                                                  const double *__restrict__ s, const double *__restrict__ t,
-                                                 double *__restrict__ r, RedArgs red)
+                                                 double *__restrict__ r, const double *__restrict__ r0, RedArgs red)
 {
     PDL_ENTRY();
     KScal *ks = red.ks;
     if (ks->done) return;
     const double omega = ks->omega;
-    double sum = 0.0;
+    double sum = 0.0, r0r = 0.0;
     const int stride = gridDim.x * NT;
     for (int i = blockIdx.x * NT + threadIdx.x; i < n; i += stride) {
         x[i] = 1.0 * x[i] + omega * (double)q[i];
         double rv = 1.0 * s[i] + (-omega) * t[i];
         r[i] = rv;
         sum += rv * rv;
+        r0r += r0[i] * rv;
     }
-    double vv[1] = {sum};
-    grid_reduce<NT, 1>(vv, red.partials, red.counter, [&](const double(&tot)[1]) {
+    double vv[2] = {sum, r0r};
+    grid_reduce<NT, 2>(vv, red.partials, red.counter, [&](const double(&tot)[2]) {
         conv_update(ks, sqrt(tot[0]), 1);
         if (ks->omega == 0.0) {
             ks->fail = 1;
             ks->done = 1;
         }
+        bicg_top(ks, tot[1], tot[0]);
     });
 }
 
 template <class ZT>
-void bicg_x_r(Ctx &c, int n, double *x, const ZT *q, const double *s, const double *t, double *r, RedArgs red)
+void bicg_x_r(Ctx &c, int n, double *x, const ZT *q, const double *s, const double *t, double *r, const double *r0,
+              RedArgs red)
 {
-    UG_LAUNCH_PDL(c, k_bicg_x_r<ZT>, row_grid(c, n), NT, 0, n, x, q, s, t, r, red);
+    UG_LAUNCH_PDL(c, k_bicg_x_r<ZT>, row_grid(c, n), NT, 0, n, x, q, s, t, r, r0, red);
 }
-template void bicg_x_r<double>(Ctx &, int, double *, const double *, const double *, const double *, double *, RedArgs);
-template void bicg_x_r<float>(Ctx &, int, double *, const float *, const double *, const double *, double *, RedArgs);
+template void bicg_x_r<double>(Ctx &, int, double *, const double *, const double *, const double *, double *,
+                               const double *, RedArgs);
+template void bicg_x_r<float>(Ctx &, int, double *, const float *, const double *, const double *, double *,
+                              const double *, RedArgs);
 
 // ------------------------------------------------------ vector/matrix API --
 __global__ void __launch_bounds__(NT) k_vec_dot(int n, const double *__restrict__ a, const double *__restrict__ b,

@@ -16,6 +16,7 @@ namespace ug4gb {
 // (lib_algebra/operator/convergence_check_impl.h:85-172).
 struct KScal {
     int step, done, fail, restart;
+    int restarted;                              // BiCGStab: this iteration set r0 = r
     int maxit, hist_cap;
     double min_def, rel_red;
     double d0, dcur;
@@ -256,8 +257,9 @@ void ilu_apply(Ctx &c, const IluFactors<V> &F, const std::vector<DevBuf<int>> &c
                const V *d, V *y, V *t, double damp, const int *skip);
 
 // ---- Krylov kernels (FP64 outer vectors; z may be FP32 in mixed mode) ----
-// r -= A x, |r| starts the check; optionally r32 = (float) r
-void krylov_start(Ctx &c, const OpMat<double> &A, const double *x, double *r, RedArgs red, float *r32 = nullptr);
+// r -= A x, |r| starts the check; optionally r32 = (float) r; bicg: the scalars
+// of BiCGStab's first iteration too
+void krylov_start(Ctx &c, const OpMat<double> &A, const double *x, double *r, RedArgs red, float *r32, bool bicg);
 // first: p = z, q = A z; else p = z + beta p, q = A z + beta q; lambda = (q,p), alpha = rho_old/lambda
 template <class ZT>
 void cg_spmv_dot_t(Ctx &c, const OpMat<double> &A, const ZT *z, double *p, double *q, int first, RedArgs red);
@@ -270,18 +272,19 @@ void rho_dot(Ctx &c, int n, const ZT *z, const double *r, int kind, RedArgs red)
 template <class ZT>
 void copy_z(Ctx &c, int n, const ZT *z, double *out, const int *skip);
 
-void bicg_restart(Ctx &c, int n, const double *r, double *r0, double *p, double *v, RedArgs red);
-void bicg_rho(Ctx &c, int n, const double *r0, const double *r, RedArgs red);
-void bicg_p(Ctx &c, int n, const double *r, double *p, const double *v, RedArgs red);
+// p32, s32: FP32 copies for the mixed-precision multigrid, or null
+void bicg_p(Ctx &c, int n, const double *r, double *p, const double *v, double *r0, float *p32, RedArgs red);
 template <class ZT>
 void bicg_spmv_dot_t(Ctx &c, const OpMat<double> &A, const ZT *q, double *v, const double *r0, RedArgs red);
 template <class ZT>
-void bicg_x_s(Ctx &c, int n, double *x, const ZT *q, const double *r, const double *v, double *s, RedArgs red);
+void bicg_x_s(Ctx &c, int n, double *x, const ZT *q, const double *r, const double *v, double *s, float *s32,
+              RedArgs red);
 void bicg_s_to_r(Ctx &c, int n, const double *s, double *r, RedArgs red);
 template <class ZT>
 void bicg_spmv_2dot_t(Ctx &c, const OpMat<double> &A, const ZT *q, double *t, const double *s, RedArgs red);
 template <class ZT>
-void bicg_x_r(Ctx &c, int n, double *x, const ZT *q, const double *s, const double *t, double *r, RedArgs red);
+void bicg_x_r(Ctx &c, int n, double *x, const ZT *q, const double *s, const double *t, double *r, const double *r0,
+              RedArgs red);
 
 // ---- BLAS-1 / SpMV for the public vector and matrix API ----
 void vec_dot(Ctx &c, int n, const double *a, const double *b, RedArgs red);
