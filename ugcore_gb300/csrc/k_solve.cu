@@ -162,6 +162,39 @@ struct DiaMV {
     }
 };
 
+template <class MV>
+struct is_dia : std::false_type {};
+template <class V, int S>
+struct is_dia<DiaMV<V, S>> : std::true_type {};
+
+// Grid of a kernel with one row product per thread and iteration.  FP64
+// products of 15 or 27 diagonals are bound by the FP64 issue rate, and the warps
+// of an SM do not get equal shares of it: with one resident wave of blocks that
+// stride over the rows, some finish early and the rest leave the pipe idle
+// (129^3 hexes: 86% busy, 74% of the warps present).  More blocks than
+// resident ones keep it fed: one row per thread (a smoothing step 126 -> 112
+// us); with a reduction at each block's end one to four, about three waves
+// of blocks (last step 140 -> 134 us, q = A z 130 -> 126 us at two rows, 125
+// at four).  Products bound by memory (SELL, 7 or 9 diagonals, FP32) and
+// levels of less than a wave keep the one wave.
+template <class MV, class V>
+static int spmv_grid(const Ctx &c, int nrows, bool reduces)
+{
+    constexpr bool fp64_bound = [] {
+        if constexpr (is_dia<MV>::value) return sizeof(V) == 8 && MV::kS >= 15;
+        else return false;
+    }();
+    const int wave = c.num_sms * 8 * NT;
+    if (!fp64_bound || nrows <= wave) return row_grid(c, nrows);
+    int per = 1;
+    if (reduces) {
+        per = nrows / (3 * wave);
+        per = per < 1 ? 1 : (per > 4 ? 4 : per);
+        while (div_up(nrows, (size_t)NT * per) > (unsigned)kRedMaxBlocks) ++per;
+    }
+    return (int)div_up(nrows, (size_t)NT * per);
+}
+
 // calls f(view) with the view type matching the operator's layout
 template <class V, class F>
 void with_mv(const OpMat<V> &m, F &&f)
@@ -346,10 +379,6 @@ __global__ void __launch_bounds__(NT, 8) k_smooth_dia(DiaMV<V, S> A, const V *__
     }
 }
 
-template <class MV>
-struct is_dia : std::false_type {};
-template <class V, int S>
-struct is_dia<DiaMV<V, S>> : std::true_type {};
 
 inline bool aligned16(const void *p) { return ((uintptr_t)p & 15u) == 0; }
 
@@ -357,9 +386,9 @@ template <class V, class XT, class DT>
 void smooth_step(Ctx &c, const OpMat<V> &At, const XT *x, const DT *dbase, const V *dinv, V *sc, V *dout, int sc_mode,
                  const int *skip, const double *r_rho, RedArgs *red, int rho_kind, double *z64)
 {
-    const int g = row_grid(c, At.nrows);
     with_mv(At, [&](auto mv) {
         using MV = decltype(mv);
+        const int g = spmv_grid<MV, V>(c, At.nrows, r_rho != nullptr);
         if constexpr (is_dia<MV>::value && std::is_same<XT, V>::value && std::is_same<DT, V>::value) {
             // FP32 levels of at least three full waves of one-row threads:
             // there the wider loads pay (8-9% per sweep on GB300).  FP64 sweeps
@@ -844,7 +873,7 @@ __global__ void __launch_bounds__(NT) k_krylov_start(MV A, const double *__restr
 void krylov_start(Ctx &c, const OpMat<double> &A, const double *x, double *r, RedArgs red, float *r32, bool bicg)
 {
     with_mv(A, [&](auto mv) {
-        UG_LAUNCH_PDL(c, k_krylov_start<decltype(mv)>, row_grid(c, A.nrows), NT, 0, mv, x, r, r32, bicg, red);
+        UG_LAUNCH_PDL(c, k_krylov_start<decltype(mv)>, (spmv_grid<decltype(mv), double>(c, A.nrows, true)), NT, 0, mv, x, r, r32, bicg, red);
     });
 }
 
@@ -882,7 +911,7 @@ template <class ZT>
 void cg_spmv_dot_t(Ctx &c, const OpMat<double> &A, const ZT *z, double *p, double *q, int first, RedArgs red)
 {
     with_mv(A, [&](auto mv) {
-        UG_LAUNCH_PDL(c, (k_cg_spmv_dot<decltype(mv), ZT>), row_grid(c, A.nrows), NT, 0, mv, z, p, q, first, red);
+        UG_LAUNCH_PDL(c, (k_cg_spmv_dot<decltype(mv), ZT>), (spmv_grid<decltype(mv), double>(c, A.nrows, true)), NT, 0, mv, z, p, q, first, red);
     });
 }
 template void cg_spmv_dot_t<double>(Ctx &, const OpMat<double> &, const double *, double *, double *, int, RedArgs);
@@ -1064,7 +1093,7 @@ template <class ZT>
 void bicg_spmv_dot_t(Ctx &c, const OpMat<double> &A, const ZT *q, double *v, const double *r0, RedArgs red)
 {
     with_mv(A, [&](auto mv) {
-        UG_LAUNCH_PDL(c, (k_bicg_spmv_dot<decltype(mv), ZT>), row_grid(c, A.nrows), NT, 0, mv, q, v, r0, red);
+        UG_LAUNCH_PDL(c, (k_bicg_spmv_dot<decltype(mv), ZT>), (spmv_grid<decltype(mv), double>(c, A.nrows, true)), NT, 0, mv, q, v, r0, red);
     });
 }
 template void bicg_spmv_dot_t<double>(Ctx &, const OpMat<double> &, const double *, double *, const double *, RedArgs);
@@ -1147,7 +1176,7 @@ template <class ZT>
 void bicg_spmv_2dot_t(Ctx &c, const OpMat<double> &A, const ZT *q, double *t, const double *s, RedArgs red)
 {
     with_mv(A, [&](auto mv) {
-        UG_LAUNCH_PDL(c, (k_bicg_spmv_2dot<decltype(mv), ZT>), row_grid(c, A.nrows), NT, 0, mv, q, t, s, red);
+        UG_LAUNCH_PDL(c, (k_bicg_spmv_2dot<decltype(mv), ZT>), (spmv_grid<decltype(mv), double>(c, A.nrows, true)), NT, 0, mv, q, t, s, red);
     });
 }
 template void bicg_spmv_2dot_t<double>(Ctx &, const OpMat<double> &, const double *, double *, const double *,
@@ -1243,7 +1272,7 @@ void op_axpy(Ctx &c, const OpMat<double> &A, double *dest, double alpha, const d
              const double *w1)
 {
     with_mv(A, [&](auto mv) {
-        UG_LAUNCH_PDL(c, k_op_axpy<decltype(mv)>, row_grid(c, A.nrows), NT, 0, mv, dest, alpha, v1, beta, w1);
+        UG_LAUNCH_PDL(c, k_op_axpy<decltype(mv)>, (spmv_grid<decltype(mv), double>(c, A.nrows, false)), NT, 0, mv, dest, alpha, v1, beta, w1);
     });
 }
 
