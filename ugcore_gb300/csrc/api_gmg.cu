@@ -366,7 +366,7 @@ struct GmgT : GmgBase {
         mix(Ainv.p);
         mix(z64.p);
         mix(coarse_plan.p);
-        h ^= (uint64_t)(coarse_top + 2);
+        h ^= (uint64_t)(coarse_top + 2) ^ ((uint64_t)coarse_host.ctas << 8) ^ ((uint64_t)coarse_smem << 16);
         h *= 1099511628211ULL;
         return h;
     }
@@ -538,17 +538,16 @@ struct GmgT : GmgBase {
         nbase = n;
     }
 
-    // Which coarse levels the one-block kernel cycles (Ctx::coarse_levels),
-    // and its shared-memory layout (CoarsePlan).  Inside the one block every
-    // phase is a chain of dependent FMAs on one SM; on GB300 an FP64 chain
-    // issues at a small fraction of the FP32 rate, so the block only pays
-    // where a phase is shorter than a separate launch (about 1.5 us).
-    // Measured on GB300 (c0/c3 quads, c1 hexes, c2 Kuhn tets, c4 upwind
-    // hexes): levels whose Jacobi sweep is at most about 4000 FP64 row-
-    // operations, rows x (S + 3), an FP32 one counting a quarter, gain
-    // (9-point 2D levels up to 17^2 in FP64 and 33^2 in FP32: 8-15% of a
-    // solve); a base level of more than 32 rows loses (its dense solve, one
-    // warp per row with a five-step warp sum, is FP64 bound on one SM).
+    // Which coarse levels the cluster kernel cycles (Ctx::coarse_levels), which
+    // of them its first block alone, and its shared-memory layout (CoarsePlan).
+    // Measured on GB300 (129^2 and 257^2 quads, 129^3 hexes and Kuhn tets, 49^3
+    // tets, 97^3 upwind hexes; FP64 and FP32): a phase of the cluster takes 0.8
+    // us and more, at about 110000 row-operations (rows x (S + 3)) of a Jacobi
+    // sweep as much as a launch; a barrier of one block beats the cluster's up to
+    // about 1000.  Against separate launches above one block's levels: 129^2
+    // solve 690 -> 651 us, 257^2 gradient 4.13 -> 3.98 ms, Newton on 49^3 tets
+    // 4.45 -> 4.07 ms.  A base of more than 32 rows is shared too: one warp per
+    // row is FP64 bound on one SM.
     void setup_coarse(Ctx &c)
     {
         coarse_top = -1;
@@ -556,70 +555,87 @@ struct GmgT : GmgBase {
         if (c.coarse_levels == 0 || cycle != 1 || smoother != UG4GB_SMOOTHER_JACOBI ||
             smoother2 != UG4GB_SMOOTHER_JACOBI || base_kind != UG4GB_BASE_LU)
             return;
-        constexpr double kSweepWork = 4000.0;
+        constexpr size_t kSmemMax = 208 * 1024;
+        int &coarse_ctas = c.coarse_ctas[sizeof(V) == 8 ? 0 : 1];
+        if (coarse_ctas == 0) coarse_ctas = coarse_prepare<V>(c, kSmemMax);   // the most any multigrid asks for
+        constexpr double kSharedWork = 110e3, kSoloWork = 1000.0;
         constexpr int kBaseRows = 32;
-        constexpr size_t kSmemMax = 216 * 1024;
         constexpr int kAlign = 16 / (int)sizeof(V);   // elements per 16 bytes
         auto up = [](size_t v, size_t a) { return (v + a - 1) / a * a; };
-        if (c.coarse_levels < 0 && nbase > kBaseRows) return;
-        CoarsePlan<V> &P = coarse_host;
-        P = CoarsePlan<V>{};
-        P.vbase = (int)up((size_t)(nbase + 1) * nbase * sizeof(double), 16);
-        size_t e = up(2 * (size_t)lev[base].n, kAlign);   // level-precision elements so far
-        P.lev[0].n = lev[base].n;
-        P.lev[0].vofs = 0;
-        int best = -1;
+        auto work = [&](int l) { return (double)lev[l].n * (lev[l].At.dia.S + 3); };
+        const bool solo_base = nbase <= kBaseRows;
+        CoarsePlan<V> best{};
         size_t best_bytes = 0;
-        const int last = std::min(top() - 1, base + kCoarseMaxLevels - 1);
-        for (int l = base + 1; l <= last; ++l) {
-            const GLevel<V> &L = lev[l];
-            const GridPair &gp = L.gp;
-            if (!L.grid_transfer || L.At.kind != 1 || L.At.nrows != L.n || L.At.ncols != L.n ||
-                gp.nx * gp.ny * gp.nz != L.n || gp.cnx * gp.cny * gp.cnz != lev[l - 1].n ||
-                !coarse_width_ok(L.At.dia.S) || L.At.dia.S != lev[base + 1].At.dia.S)
+        int best_top = -1;
+        // the plan for every candidate entry level, the coarsest first: the
+        // last that fits and pays is taken
+        for (int t = base + 1; t <= std::min(top() - 1, base + kCoarseMaxLevels - 1); ++t) {
+            const GLevel<V> &T = lev[t];
+            if (!T.grid_transfer || T.At.kind != 1 || T.At.nrows != T.n || T.At.ncols != T.n ||
+                T.gp.nx * T.gp.ny * T.gp.nz != T.n || T.gp.cnx * T.gp.cny * T.gp.cnz != lev[t - 1].n ||
+                !coarse_width_ok(T.At.dia.S) || T.At.dia.S != lev[base + 1].At.dia.S)
                 break;
-            const Dia<V> &D = L.At.dia;
-            CoarseLevel<V> &Q = P.lev[l - base];
-            Q.n = L.n;
-            Q.val = D.vals();
-            Q.dinv = L.dinv.p;
-            Q.dfac = L.dfac.p;
-            Q.ncols = D.ncols;
-            Q.ld = D.ld;
-            Q.S = D.S;
-            for (int k = 0; k < D.S; ++k) Q.off[k] = D.off.o[k];
-            Q.gp = gp;
-            Q.aofs = (int)e;
-            e = up(e + (size_t)D.S * D.ld, kAlign);
-            Q.iofs = (int)e;
-            e = up(e + (size_t)L.n, kAlign);
-            Q.fofs = (int)e;
-            e = up(e + (size_t)L.n, kAlign);
-            Q.vofs = (int)e;
-            e = up(e + 4 * (size_t)L.n, kAlign);
+            if (c.coarse_levels > 0 ? t - base > c.coarse_levels : work(t) > kSharedWork) break;
+            CoarsePlan<V> P{};
+            P.m = t - base + 1;
+            bool any_shared = !solo_base;
+            for (int l = base + 1; l <= t; ++l) any_shared |= work(l) > kSoloWork;
+            P.ctas = any_shared ? coarse_ctas : 1;
+            size_t e = 0;   // level-precision elements so far
+            bool solo = any_shared ? solo_base : true, ok = true;
+            for (int l = base; l <= t; ++l) {
+                const GLevel<V> &L = lev[l];
+                CoarseLevel<V> &Q = P.lev[l - base];
+                if (any_shared && l > base && work(l) > kSoloWork) solo = false;
+                Q.n = L.n;
+                Q.solo = solo ? 1 : 0;
+                Q.per = (int)up(solo ? (size_t)L.n : (size_t)div_up(L.n, P.ctas), 4);
+                Q.mul = (unsigned)((((uint64_t)1 << 32) + Q.per - 1) / Q.per);
+                ok = ok && (uint64_t)L.n * Q.per < ((uint64_t)1 << 32);
+                if (l == base) {
+                    P.vbase = (int)up((size_t)(Q.per + 1) * nbase * sizeof(double), 16);
+                    Q.vofs = 0;
+                    e = up(2 * (size_t)Q.per, kAlign);
+                    continue;
+                }
+                const Dia<V> &D = L.At.dia;
+                Q.val = D.vals();
+                Q.dinv = L.dinv.p;
+                Q.dfac = L.dfac.p;
+                Q.ncols = D.ncols;
+                Q.ld = D.ld;
+                Q.S = D.S;
+                for (int k = 0; k < D.S; ++k) Q.off[k] = D.off.o[k];
+                Q.gp = L.gp;
+                Q.aofs = (int)e;
+                e += (size_t)D.S * Q.per;
+                Q.iofs = (int)e;
+                e += (size_t)Q.per;
+                Q.fofs = (int)e;
+                e += (size_t)Q.per;
+                Q.vofs = (int)e;
+                e += 4 * (size_t)Q.per;
+            }
             const size_t bytes = (size_t)P.vbase + e * sizeof(V);
             if (bytes > kSmemMax) break;
-            if (c.coarse_levels > 0) {
-                if (l - base > c.coarse_levels) break;
-            } else if ((double)L.n * (D.S + 3) * (sizeof(V) == 8 ? 1.0 : 0.25) > kSweepWork) {
-                break;
-            }
-            best = l;
+            if (!ok) break;
+            best = P;
             best_bytes = bytes;
+            best_top = t;
         }
-        if (best < 0) return;
-        P.m = best - base + 1;
+        if (best_top < 0) return;
+        CoarsePlan<V> &P = coarse_host;
+        P = best;
         P.nu1 = nu1;
         P.nu2 = nu2;
         P.nbase = nbase;
         P.Ainv = Ainv.p;
-        P.d_in = lev[best].dA.p;
-        P.sc_out = lev[best].sc.p;
+        P.d_in = lev[best_top].dA.p;
+        P.sc_out = lev[best_top].sc.p;
         coarse_smem = best_bytes;
         coarse_plan.alloc(1);
         copy_in(c, coarse_plan.p, &P, sizeof(P));   // from pageable memory: staged on return
-        coarse_prepare<V>(kSmemMax);   // the most any multigrid asks for
-        coarse_top = best;
+        coarse_top = best_top;
     }
 
     // ------------------------------------------------------------ cycle --
@@ -688,7 +704,7 @@ struct GmgT : GmgBase {
         } else if (l - 1 == coarse_top) {
             // V-cycle below: the coarse end in one launch (setup_coarse)
             c.prof_tag = "L" + std::to_string(base) + "-" + std::to_string(l - 1);
-            coarse_cycle<V>(c, coarse_plan.p, coarse_host.lev[1].S, coarse_smem, skip);
+            coarse_cycle<V>(c, coarse_plan.p, coarse_host.ctas, coarse_host.lev[1].S, coarse_smem, skip);
         } else {
             const int visits = (ctype == -1) ? 2 : ctype;
             for (int i = 0; i < visits; ++i) {

@@ -135,6 +135,7 @@ struct Ctx {
     // levels above the base cycled by the one-block coarse kernel (-1: as
     // many as its cost model finds faster than separate launches, 0: none)
     int coarse_levels = -1;
+    int coarse_ctas[2] = {0, 0};   // blocks per cluster it runs with, FP64 and FP32 levels (0: not asked yet)
     std::string prof_tag;       // set by the orchestration (level / phase)
     std::vector<ProfRec> prof;
     std::vector<cudaEvent_t> ev_pool;
@@ -391,6 +392,29 @@ __device__ __forceinline__ void st_pack(T *p, const Pack<T, W> &v)
     *reinterpret_cast<Pack<T, W> *>(p) = v;
 }
 
+// Sum over the block's NT threads of NV values each, in sh[q][0] of the first
+// thread of warp 2q on return (a fixed tree).  FP64 additions are scarce on
+// GB300 (a warp's takes 64 cycles of its pipe, some 130 to the next dependent
+// one): 64 threads add four values each, then two warps reduce, 17 additions
+// issued per value and 9 in a row, where a shuffle reduction of every warp
+// issues 45.
+template <int NT, int NV>
+__device__ __forceinline__ void block_sum(const double (&v)[NV], double (&sh)[NV][NT])
+{
+    static_assert(NT == 256 && 64 * NV <= NT, "two warps per value");
+#pragma unroll
+    for (int q = 0; q < NV; ++q) sh[q][threadIdx.x] = v[q];
+    __syncthreads();
+    const int q = threadIdx.x >> 6, t = threadIdx.x & 63;
+    if (q < NV) {
+        double s = (sh[q][t] + sh[q][t + 64]) + (sh[q][t + 128] + sh[q][t + 192]);
+        s = warp_sum(s);
+        if ((t & 31) == 0) sh[q][t] = s;   // read by its own thread only
+    }
+    __syncthreads();
+    if (q < NV && t == 0) sh[q][0] = sh[q][0] + sh[q][32];
+}
+
 // Deterministic grid-wide sum of NV values per thread.  Each block reduces
 // in a fixed tree, writes its partials, and the last block to finish sums
 // the partials in block order and calls fin(total) with thread 0.
@@ -398,27 +422,16 @@ template <int NT, int NV, class Fin>
 __device__ __forceinline__ void grid_reduce(const double (&v)[NV], double *partials, unsigned int *counter,
                                             Fin fin)
 {
-    __shared__ double sh[NV][NT / 32];
+    __shared__ double sh[NV][NT];
     __shared__ bool is_last;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    block_sum<NT, NV>(v, sh);
+    if (NV > 1) __syncthreads();
+    if (threadIdx.x == 0) {
 #pragma unroll
-    for (int q = 0; q < NV; ++q) {
-        double s = warp_sum(v[q]);
-        if (lane == 0) sh[q][warp] = s;
-    }
-    __syncthreads();
-    if (warp == 0) {
-#pragma unroll
-        for (int q = 0; q < NV; ++q) {
-            double s = (lane < NT / 32) ? sh[q][lane] : 0.0;
-            s = warp_sum(s);
-            if (lane == 0) partials[q * kRedMaxBlocks + blockIdx.x] = s;
-        }
-        if (lane == 0) {
-            __threadfence();
-            unsigned t = atomicAdd(counter, 1u);
-            is_last = (t == gridDim.x - 1);
-        }
+        for (int q = 0; q < NV; ++q) partials[q * kRedMaxBlocks + blockIdx.x] = sh[q][0];
+        __threadfence();
+        unsigned t = atomicAdd(counter, 1u);
+        is_last = (t == gridDim.x - 1);
     }
     __syncthreads();
     if (!is_last) return;
@@ -428,17 +441,13 @@ __device__ __forceinline__ void grid_reduce(const double (&v)[NV], double *parti
     for (int q = 0; q < NV; ++q) {
         double s = 0.0;
         for (int b = threadIdx.x; b < (int)gridDim.x; b += NT) s += __ldcg(partials + q * kRedMaxBlocks + b);
-        s = warp_sum(s);
-        if (lane == 0) sh[q][warp] = s;
+        tot[q] = s;
     }
-    __syncthreads();
+    block_sum<NT, NV>(tot, sh);
+    if (NV > 1) __syncthreads();
     if (threadIdx.x == 0) {
 #pragma unroll
-        for (int q = 0; q < NV; ++q) {
-            double s = 0.0;
-            for (int w = 0; w < NT / 32; ++w) s += sh[q][w];
-            tot[q] = s;
-        }
+        for (int q = 0; q < NV; ++q) tot[q] = sh[q][0];
         *counter = 0u;
         fin(tot);
     }

@@ -333,16 +333,6 @@ __global__ void k_check_row_lengths(int cx, int cy, int cz, const int *__restric
     if (rowptr[r + 1] - rowptr[r] != S::N) atomicExch(ok, 0);
 }
 
-// the sum of an interior vertex's SCV volumes in the order of gather_row
-template <int T>
-__global__ void k_row_volsum(AsmArgs a, ClassData<T> cd, double *out)
-{
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    double s = 0.0;
-    gather_row<T>(cd, a, 1, 1, (Stencil<T>::DIM == 3) ? 1 : 0, nullptr, [](int, double) {}, [&](double v) { s += v; });
-    out[0] = s;
-}
-
 // Calls f(slot, offset in vertices) for the stencil of an interior row.
 template <int T, class F>
 __device__ __forceinline__ void for_stencil(int nx, int ny, F &&f)
@@ -753,31 +743,47 @@ constexpr int kSmallLevelRows = 1 << 16;
 namespace {
 
 // Class geometry of level L (once per level, kept in cache), the SCV volume
-// sum of its interior rows, the list of its boundary rows; false where the
-// cells are not the classes' boxes.
+// sum of its interior rows, the list of its boundary rows and, with rowptr, the
+// check of its row lengths; false where the cells are not the classes' boxes.
 template <int T>
-bool class_data(Ctx &c, const Level &L, RowAsmCache &cache, ClassData<T> &cd)
+bool class_data(Ctx &c, const Level &L, RowAsmCache &cache, ClassData<T> &cd, const int *rowptr = nullptr)
 {
     using CT = ClassTraits<T>;
     using E = Elem<T>;
     if (!L.structured || L.nx < 3 || L.ny < 3 || (L.dim == 3 && L.nz < 3)) return false;
+    const int cx = L.nx - 1, cy = L.ny - 1, cz = (L.dim == 3) ? L.nz - 1 : 1;
+    auto check_rows = [&](int *ok) {
+        const int nint = (cx - 1) * (cy - 1) * ((L.dim == 3) ? cz - 1 : 1);
+        UG_LAUNCH(c, k_check_row_lengths<T>, div_up(nint, 256), 256, 0, cx, cy, cz, rowptr, ok);
+    };
     if (!cache.ready) {
-        DevBuf<double> A, vol, nrm, ipo;
+        std::vector<int> rows;   // on the box boundary
+        const int nx = L.nx, ny = L.ny, nz = (L.dim == 3) ? L.nz : 1;
+        for (int k = 0; k < nz; ++k)
+            for (int j = 0; j < ny; ++j) {
+                const bool face = j == 0 || j == ny - 1 || (L.dim == 3 && (k == 0 || k == nz - 1));
+                for (int i = 0; i < nx; i += face ? 1 : nx - 1) rows.push_back(i + nx * (j + ny * k));
+            }
+        cache.brows.alloc(rows.size());
+        copy_in(c, cache.brows.p, rows.data(), sizeof(int) * rows.size());
+        DevBuf<double> A, nrm, ipo;
         DevBuf<int> ok;
-        A.alloc(CT::NC * E::K * E::K);
-        vol.alloc(CT::NC * E::K);
+        constexpr int nA = CT::NC * E::K * E::K, nV = CT::NC * E::K;
+        A.alloc(nA + nV);   // element matrices, then SCV volumes
         nrm.alloc(CT::NC * E::NSCVF * 3);
         ipo.alloc(CT::NC * E::NSCVF * 3);
-        ok.alloc(1);
-        const int one = 1;
-        copy_in(c, ok.p, &one, sizeof(int));
-        UG_LAUNCH(c, k_class_data<T>, 1, 32, 0, L.coords.p, L.elems.p, A.p, vol.p, nrm.p, ipo.p, ok.p);
-        cache.A.resize(CT::NC * E::K * E::K);
-        cache.vol.resize(CT::NC * E::K);
-        copy_out(c, cache.A.data(), A.p, sizeof(double) * cache.A.size());
-        copy_out(c, cache.vol.data(), vol.p, sizeof(double) * cache.vol.size());
-        int okh = 0;
-        copy_out(c, &okh, ok.p, sizeof(int));
+        ok.alloc(3);        // corners as the classes number them, boundary all Dirichlet, row lengths
+        int okh[3] = {1, 1, 1};
+        copy_in(c, ok.p, okh, sizeof(okh));
+        UG_LAUNCH(c, k_class_data<T>, 1, 32, 0, L.coords.p, L.elems.p, A.p, A.p + nA, nrm.p, ipo.p, ok.p);
+        UG_LAUNCH(c, k_check_dirichlet, div_up(rows.size(), 256), 256, 0, L.bnd.p, cache.brows.p, (int)rows.size(),
+                  ok.p + 1);
+        if (rowptr) check_rows(ok.p + 2);
+        cache.A.resize(nA + nV);
+        copy_out(c, cache.A.data(), A.p, A.bytes());
+        copy_out(c, okh, ok.p, sizeof(okh));
+        cache.vol.assign(cache.A.begin() + nA, cache.A.end());
+        cache.A.resize(nA);
         // entries that vanish in exact arithmetic (on a Kuhn tetrahedron
         // the couplings of its non-path edges) come out of the box-method
         // sums as rounding noise of some 1e-16 of the largest entry: exact
@@ -788,45 +794,32 @@ bool class_data(Ctx &c, const Level &L, RowAsmCache &cache, ClassData<T> &cd)
             for (int q = 0; q < E::K * E::K; ++q)
                 if (std::fabs(Ap[q]) < 1e-14 * big) Ap[q] = 0.0;
         }
+        // the sum of an interior vertex's SCV volumes in the order of gather_row
+        cache.volsum = 0.0;
+        for (int b = CT::NCELL - 1; b >= 0; --b)
+            for (int p = 0; p < CT::NC; ++p)
+                for (int q = 0; q < E::K; ++q)
+                    if (class_corner_bits<T>(p, q) == b) cache.volsum += cache.vol[p * E::K + q];
         cache.normal = std::move(nrm);
         cache.ipoff = std::move(ipo);
-        cache.usable = (okh == 1);
+        cache.usable = (okh[0] == 1);
+        cache.all_dirichlet = (okh[1] == 1);
+        if (rowptr) cache.row_check = (okh[2] == 1) ? 1 : -1;
+        cache.nbrows = (int)rows.size();
         cache.ready = true;
     }
     if (!cache.usable) return false;
-    std::memcpy(&cd.A[0][0][0], cache.A.data(), sizeof(cd.A));
-    std::memcpy(&cd.vol[0][0], cache.vol.data(), sizeof(cd.vol));
-    if (cache.nbrows == 0) {
-        // once per level: the interior rows' SCV volume sum and the list of
-        // the rows on the box boundary
-        AsmArgs a{};
-        a.cx = L.nx - 1;
-        a.cy = L.ny - 1;
-        a.cz = (L.dim == 3) ? L.nz - 1 : 1;
-        DevBuf<double> vs;
-        vs.alloc(1);
-        UG_LAUNCH(c, k_row_volsum<T>, 1, 32, 0, a, cd, vs.p);
-        copy_out(c, &cache.volsum, vs.p, sizeof(double));
-        const int nx = L.nx, ny = L.ny, nz = (L.dim == 3) ? L.nz : 1;
-        std::vector<int> rows;
-        for (int k = 0; k < nz; ++k)
-            for (int j = 0; j < ny; ++j)
-                for (int i = 0; i < nx; ++i)
-                    if (i == 0 || i == nx - 1 || j == 0 || j == ny - 1 || (L.dim == 3 && (k == 0 || k == nz - 1)))
-                        rows.push_back(i + nx * (j + ny * k));
-        cache.brows.alloc(rows.size());
-        copy_in(c, cache.brows.p, rows.data(), sizeof(int) * rows.size());
+    if (rowptr && cache.row_check == 0) {
         DevBuf<int> ok;
         ok.alloc(1);
         int okh = 1;
         copy_in(c, ok.p, &okh, sizeof(int));
-        UG_LAUNCH(c, k_check_dirichlet, div_up(rows.size(), 256), 256, 0, L.bnd.p, cache.brows.p, (int)rows.size(),
-                  ok.p);
+        check_rows(ok.p);
         copy_out(c, &okh, ok.p, sizeof(int));
-        cache.all_dirichlet = (okh == 1);
-        UG_CUDA(cudaStreamSynchronize(c.stream));
-        cache.nbrows = (int)rows.size();
+        cache.row_check = (okh == 1) ? 1 : -1;
     }
+    std::memcpy(&cd.A[0][0][0], cache.A.data(), sizeof(cd.A));
+    std::memcpy(&cd.vol[0][0], cache.vol.data(), sizeof(cd.vol));
     return true;
 }
 
@@ -912,18 +905,8 @@ bool launch_assemble_rows(Ctx &c, const Level &L, const AsmArgs &a_in, RowAsmCac
     return dispatch_rows(L.elem_type, [&](auto tag) {
         constexpr int T = decltype(tag)::value;
         ClassData<T> cd;
-        if (!class_data<T>(c, L, cache, cd)) return false;
+        if (!class_data<T>(c, L, cache, cd, a_in.rowptr)) return false;
         const AsmArgs a = with_cells(L, a_in);
-        if (cache.row_check == 0) {
-            const int nint = (a.cx - 1) * (a.cy - 1) * ((L.dim == 3) ? a.cz - 1 : 1);
-            DevBuf<int> ok;
-            ok.alloc(1);
-            int okh = 1;
-            copy_in(c, ok.p, &okh, sizeof(int));
-            UG_LAUNCH(c, k_check_row_lengths<T>, div_up(nint, 256), 256, 0, a.cx, a.cy, a.cz, a.rowptr, ok.p);
-            copy_out(c, &okh, ok.p, sizeof(int));
-            cache.row_check = (okh == 1) ? 1 : -1;
-        }
         if (cache.row_check < 0 || (a.inst && !cache.all_dirichlet)) return false;
         const double *flux;
         if (!class_fluxes<T>(c, a, cache, flux)) return false;

@@ -67,13 +67,32 @@ struct SellMV {
     template <class ACC, class XT>
     __device__ __forceinline__ ACC dot_cached(const XT *__restrict__ x, int, const Cache &c) const
     {
+        ACC xv[kCache];
+#pragma unroll
+        for (int k = 0; k < kCache; ++k)
+            if (k < c.w) xv[k] = (ACC)x[c.col[k]];
         ACC acc = (ACC)0;
 #pragma unroll
         for (int k = 0; k < kCache; ++k)
-            if (k < c.w) acc += (ACC)c.val[k] * (ACC)x[c.col[k]];
-        for (int k = kCache; k < c.w; ++k) {
-            const int idx = c.base + k * kSliceH;
-            acc += (ACC)ld_stream(s.val + idx) * (ACC)x[ld_stream(s.col + idx)];
+            if (k < c.w) acc = fma_rn((ACC)c.val[k], xv[k], acc);
+        // the rest: the loads of kCache entries issued before their sum (one
+        // entry after the other cost a level of 15000 rows 2 us per product)
+#pragma unroll 1
+        for (int k = kCache; k < c.w; k += kCache) {
+            int col[kCache];
+            V val[kCache];
+#pragma unroll
+            for (int q = 0; q < kCache; ++q)
+                if (k + q < c.w) {
+                    col[q] = ld_stream(s.col + c.base + (k + q) * kSliceH);
+                    val[q] = ld_stream(s.val + c.base + (k + q) * kSliceH);
+                }
+#pragma unroll
+            for (int q = 0; q < kCache; ++q)
+                if (k + q < c.w) xv[q] = (ACC)x[col[q]];
+#pragma unroll
+            for (int q = 0; q < kCache; ++q)
+                if (k + q < c.w) acc = fma_rn((ACC)val[q], xv[q], acc);
         }
         return acc;
     }
@@ -108,17 +127,18 @@ struct DiaMV {
 #pragma unroll
         for (int k = 0; k < S; ++k) c.a[k] = ld_stream(val + (size_t)k * ld + i);
     }
+    // rows of a latency-bound level (row_sum)
     template <class ACC, class XT>
     __device__ __forceinline__ ACC dot_cached(const XT *__restrict__ x, int i, const Cache &c) const
     {
-        ACC acc = (ACC)0;
+        ACC xv[S];
 #pragma unroll
         for (int k = 0; k < S; ++k) {
             int j = i + off.o[k];
             j = j < 0 ? 0 : (j >= ncols ? ncols - 1 : j);
-            acc = fma_rn((ACC)c.a[k], (ACC)x[j], acc);
+            xv[k] = (ACC)x[j];
         }
-        return acc;
+        return row_sum<ACC, S>(c.a, xv);
     }
     template <class ACC, class XT>
     __device__ __forceinline__ ACC dot(const XT *__restrict__ x, int i) const

@@ -56,6 +56,30 @@ __device__ __forceinline__ V jacobi_row(V acc, V db, V dinv, int mode, V sc_in, 
     return dn;
 }
 
+// Sum of a row's S products on a level small enough that latency rules
+// (k_smooth with its row loaded ahead, the coarse cycle).  FP32: the one FMA
+// chain of the other kernels.  A dependent FP64 FMA takes some 130 cycles on
+// GB300, twice what its issue does: FP64 rows go in two chains, the lower
+// offsets and the rest (so that symmetric layouts of one matrix, with and
+// without its zero diagonals, sum the same terms), added at the end.
+template <class V, int S>
+__device__ __forceinline__ V row_sum(const V (&a)[S], const V (&x)[S])
+{
+    if constexpr (sizeof(V) == 4) {
+        V acc = (V)0;
+#pragma unroll
+        for (int k = 0; k < S; ++k) acc = fma_rn(a[k], x[k], acc);
+        return acc;
+    } else {
+        V lo = (V)0, hi = (V)0;
+#pragma unroll
+        for (int k = 0; k < S / 2; ++k) lo = fma_rn(a[k], x[k], lo);
+#pragma unroll
+        for (int k = S / 2; k < S; ++k) hi = fma_rn(a[k], x[k], hi);
+        return add_rn(lo, hi);
+    }
+}
+
 struct RedArgs {
     double *partials;
     unsigned int *counter;
@@ -128,58 +152,77 @@ __device__ __forceinline__ V grid_weight(int nodd)
 // assemble_prolongation_p1, std_transfer_impl.h:47-168, with
 // DirichletBoundary::adjust_prolongation: a Dirichlet fine vertex keeps only
 // a coinciding coarse parent, weight 1).
-template <class V>
-__device__ __forceinline__ V prolong_value(const GridPair &g, const V *__restrict__ scc, int i, int j, int k)
+// at(c): the coarse value of vertex c; the loads are issued before the sum.
+template <class V, class F>
+__device__ __forceinline__ V prolong_value(const GridPair &g, F &&at, int i, int j, int k)
 {
-    const int p0 = i & 1, p1 = j & 1, p2 = k & 1, b0 = i >> 1, b1 = j >> 1, b2 = k >> 1;
+    const int p0 = i & 1, p1 = j & 1, p2 = k & 1;
+    const int c = (i >> 1) + g.cnx * ((j >> 1) + g.cny * (k >> 1));
     const bool bnd = on_box_boundary(i, j, k, g.nx, g.ny, g.nz, g.dim);
     V t = (V)0;
     if (g.tet) {
         const bool odd = (p0 | p1 | p2) != 0;
         const V wt = odd ? (bnd ? (V)0 : (V)0.5) : (V)1;
-        t = fma_rn(wt, scc[b0 + g.cnx * (b1 + g.cny * b2)], t);
-        if (odd) t = fma_rn(wt, scc[(b0 + p0) + g.cnx * ((b1 + p1) + g.cny * (b2 + p2))], t);
+        const V v0 = at(c), v1 = at(c + p0 + g.cnx * (p1 + g.cny * p2));
+        t = fma_rn(wt, v0, t);
+        if (odd) t = fma_rn(wt, v1, t);
     } else {
         const int np = 1 << (p0 + p1 + p2);
         const V wt = bnd ? (np == 1 ? (V)1 : (V)0) : grid_weight<V>(p0 + p1 + p2);
-        for (int dk = 0; dk <= p2; ++dk)
-            for (int dj = 0; dj <= p1; ++dj)
-                for (int di = 0; di <= p0; ++di)
-                    t = fma_rn(wt, scc[(b0 + di) + g.cnx * ((b1 + dj) + g.cny * (b2 + dk))], t);
+        V v[8] = {};
+#pragma unroll
+        for (int q = 0; q < 8; ++q)
+            if ((q & 1) <= p0 && ((q >> 1) & 1) <= p1 && (q >> 2) <= p2)
+                v[q] = at(c + (q & 1) + g.cnx * (((q >> 1) & 1) + g.cny * (q >> 2)));
+#pragma unroll
+        for (int q = 0; q < 8; ++q)
+            if ((q & 1) <= p0 && ((q >> 1) & 1) <= p1 && (q >> 2) <= p2) t = fma_rn(wt, v[q], t);
     }
     return t;
 }
 
-// dc = R d for coarse vertex (I, J, K): R = P^T, Dirichlet coarse rows =
-// injection (k_restrict on the assembled R); children in increasing fine index
+// (R d) for coarse vertex (I, J, K): R = P^T, Dirichlet coarse rows =
+// injection (k_restrict on the assembled R); children in increasing fine
+// index.  at(f): the fine value of vertex f.  The loads of a plane of
+// children are issued before their sum.
+template <class V, class F>
+__device__ __forceinline__ V restrict_value(const GridPair &g, F &&at, int I, int J, int K)
+{
+    const int fv = 2 * I + g.nx * (2 * J + g.ny * 2 * K);
+    if (on_box_boundary(I, J, K, g.cnx, g.cny, g.cnz, g.dim)) {
+        const V v = (V)0 + (V)1 * at(fv);
+        return (g.dres != 1.0) ? mul_rn(v, (V)g.dres) : v;
+    }
+    const int kr = (g.dim == 3) ? 1 : 0;
+    V acc = (V)0;
+#pragma unroll 1
+    for (int dk = -kr; dk <= kr; ++dk) {
+        V v[9];
+#pragma unroll
+        for (int q = 0; q < 9; ++q) v[q] = at(fv + (q % 3 - 1) + g.nx * ((q / 3 - 1) + g.ny * dk));
+#pragma unroll
+        for (int q = 0; q < 9; ++q) {
+            const int di = q % 3 - 1, dj = q / 3 - 1;
+            const int nodd = (di != 0) + (dj != 0) + (dk != 0);
+            V wt;
+            if (g.tet) {
+                const bool pos = di > 0 || dj > 0 || dk > 0, neg = di < 0 || dj < 0 || dk < 0;
+                if (pos && neg) continue;   // not a Kuhn edge through this vertex
+                wt = nodd ? (V)0.5 : (V)1;
+            } else {
+                wt = grid_weight<V>(nodd);
+            }
+            acc = fma_rn(wt, v[q], acc);
+        }
+    }
+    return (g.dres != 1.0) ? mul_rn(acc, (V)g.dres) : acc;
+}
+
 template <class V>
 __device__ __forceinline__ void restrict_row(const GridPair &g, const V *__restrict__ d, V *__restrict__ dc, int I,
                                              int J, int K)
 {
-    const int c = I + g.cnx * (J + g.cny * K);
-    const int fv = 2 * I + g.nx * (2 * J + g.ny * 2 * K);
-    if (on_box_boundary(I, J, K, g.cnx, g.cny, g.cnz, g.dim)) {
-        const V v = (V)0 + (V)1 * d[fv];
-        dc[c] = (g.dres != 1.0) ? mul_rn(v, (V)g.dres) : v;
-        return;
-    }
-    const int kr = (g.dim == 3) ? 1 : 0;
-    V acc = (V)0;
-    for (int dk = -kr; dk <= kr; ++dk)
-        for (int dj = -1; dj <= 1; ++dj)
-            for (int di = -1; di <= 1; ++di) {
-                const int nodd = (di != 0) + (dj != 0) + (dk != 0);
-                V wt;
-                if (g.tet) {
-                    const bool pos = di > 0 || dj > 0 || dk > 0, neg = di < 0 || dj < 0 || dk < 0;
-                    if (pos && neg) continue;   // not a Kuhn edge through this vertex
-                    wt = nodd ? (V)0.5 : (V)1;
-                } else {
-                    wt = grid_weight<V>(nodd);
-                }
-                acc += wt * d[fv + di + g.nx * (dj + g.ny * dk)];
-            }
-    dc[c] = (g.dres != 1.0) ? mul_rn(acc, (V)g.dres) : acc;
+    dc[I + g.cnx * (J + g.cny * K)] = restrict_value<V>(g, [&](int f) { return d[f]; }, I, J, K);
 }
 
 template <class V>
@@ -194,27 +237,33 @@ void base_solve(Ctx &c, const double *Ainv, int n, const V *d, V *sc, const int 
 // structured hierarchy with damped-Jacobi smoothing on diagonal-layout
 // operators and grid transfers; the entry level's defect arrives in d_in
 // (its dA) and its correction leaves in sc_out (its sc), bit-identical to
-// the separate launches of lmgc.  The kernel keeps everything in shared
-// memory: Ainv (nbase^2 doubles) at byte 0 followed by the base defect in
-// FP64 (nbase doubles), then the level-precision region
-// at byte vbase holding, per level, the operator (S x ld), the Jacobi
-// factors and the vectors, at the element offsets below (the operator and
-// the factors 16-byte aligned).
+// the separate launches of lmgc.  A cluster of `ctas` blocks keeps everything
+// in shared memory: block q holds rows [q * per, (q + 1) * per) of a level, of
+// a solo level block 0 holds all.  The layout is the same in every block:
+// its rows of Ainv (per x nbase doubles) at byte 0, the base defect in FP64
+// (nbase doubles), then the level-precision region at byte vbase with, per
+// level, its part of the operator (S x per), the Jacobi factors and the
+// vectors, at the element offsets below (the operator and the factors 16-byte
+// aligned; per is a multiple of 4).
 constexpr int kCoarseMaxLevels = 8;
 template <class V>
 struct alignas(16) CoarseLevel {
     const V *val;           // column-scaled operator At, diagonal layout (Dia::vals(), S x ld)
     const V *dinv, *dfac;   // Jacobi factors (unused on the base level)
     int n, ncols, ld, S;
+    int solo;               // block 0 alone works on it
+    int per;                // rows per block
+    unsigned mul;           // j / per == (j * mul) >> 32 for j < n
     int off[kMaxDiag];
     GridPair gp;            // this level and the next coarser one (unused on the base level)
-    int aofs;               // operator values (S * ld elements)
-    int iofs, fofs;         // dinv, dfac (n elements each)
-    int vofs;               // vectors sc, dA[, dB, w] (n elements each)
+    int aofs;               // operator values (S * per elements)
+    int iofs, fofs;         // dinv, dfac (per elements each)
+    int vofs;               // vectors sc, dA[, dB, w] (per elements each)
 };
 template <class V>
 struct alignas(16) CoarsePlan {
     int m, nu1, nu2, nbase;
+    int ctas;
     const double *Ainv;     // nbase x nbase, row-major
     const V *d_in;
     V *sc_out;
@@ -225,11 +274,12 @@ struct alignas(16) CoarsePlan {
 // width of every level above the base (coarse_width_ok); smem_bytes: the
 // extent of the layout above
 template <class V>
-void coarse_cycle(Ctx &c, const CoarsePlan<V> *plan_dev, int S, size_t smem_bytes, const int *skip);
+void coarse_cycle(Ctx &c, const CoarsePlan<V> *plan_dev, int ctas, int S, size_t smem_bytes, const int *skip);
 bool coarse_width_ok(int S);
-// set-up: allows launches with up to smem_bytes of dynamic shared memory
+// set-up: allows launches with up to smem_bytes of dynamic shared memory;
+// returns the blocks per cluster the device runs with that much (16 or 8)
 template <class V>
-void coarse_prepare(size_t smem_bytes);
+int coarse_prepare(Ctx &c, size_t smem_bytes);
 template <class V>
 void mcgs_colour(Ctx &c, const OpMat<V> &A, const int *rows, int nrows_c, const V *dinv_relax, const V *d, V *t,
                  const int *skip);
