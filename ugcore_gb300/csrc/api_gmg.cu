@@ -362,6 +362,7 @@ struct GmgT : GmgBase {
             mix(L.ilu.val.p); mix(L.ilu.col.p); mix(L.ilu.rowptr.p); mix(L.ilu.nlow.p); mix(L.ilu.uinv.p);
             h ^= (uint64_t)L.n;
             for (int k = 0; k < L.At.dia.S; ++k) mix((const void *)(intptr_t)L.At.dia.off.o[k]);
+            mix((const void *)(intptr_t)(L.gs.usable ? 1 : 0));
         }
         mix(Ainv.p);
         mix(z64.p);
@@ -800,13 +801,19 @@ struct GmgT : GmgBase {
             ilu_apply<V>(c, L.ilu, L.crow, L.ncrow, dv, L.y.p, L.t.p, dmp, skip);
             return;
         }
-        UG_LAUNCH_PDL(c, k_zero<V>, div_up(L.n, 256), 256, 0, L.n, L.t.p, skip);
-        if (kind != UG4GB_SMOOTHER_MCBGS)
-            for (size_t q = 0; q < L.crow.size(); ++q)
-                if (L.ncrow[q] > 0) mcgs_colour<V>(c, L.At, L.crow[q].p, L.ncrow[q], dinv, dv, L.t.p, skip);
-        if (kind == UG4GB_SMOOTHER_MCSGS || kind == UG4GB_SMOOTHER_MCBGS)
-            for (size_t q = L.crow.size(); q-- > 0;)
-                if (L.ncrow[q] > 0) mcgs_colour<V>(c, L.At, L.crow[q].p, L.ncrow[q], dinv, dv, L.t.p, skip);
+        const bool fwd = kind != UG4GB_SMOOTHER_MCBGS, bwd = kind != UG4GB_SMOOTHER_MCGS;
+        if (L.gs.usable) {
+            if (fwd) mcgs_sweep_lines<V>(c, L.At, L.gs, L.gp, false, true, dinv, dv, L.t.p, skip);
+            if (bwd) mcgs_sweep_lines<V>(c, L.At, L.gs, L.gp, true, !fwd, dinv, dv, L.t.p, skip);
+        } else {
+            UG_LAUNCH_PDL(c, k_zero<V>, div_up(L.n, 256), 256, 0, L.n, L.t.p, skip);
+            if (fwd)
+                for (size_t q = 0; q < L.crow.size(); ++q)
+                    if (L.ncrow[q] > 0) mcgs_colour<V>(c, L.At, L.crow[q].p, L.ncrow[q], dinv, dv, L.t.p, skip);
+            if (bwd)
+                for (size_t q = L.crow.size(); q-- > 0;)
+                    if (L.ncrow[q] > 0) mcgs_colour<V>(c, L.At, L.crow[q].p, L.ncrow[q], dinv, dv, L.t.p, skip);
+        }
         // SymmetricGaussSeidel (sgs_step, core_smoothers.h:189-206) is
         // (D/w + U)^{-1} D (D/w + L)^{-1}; the backward sweep above, which
         // updates the forward result by w/a_ii times the defect, gives
@@ -945,6 +952,18 @@ static GmgBase *build_gmg(ug4gb_gmg *m, const ug4gb_matrix *A_top, GmgT<V> *reus
             L.At_lay.keep_all = true;
             op_from_csr_cached<V>(c, L.A, L.At, m->smoother == UG4GB_SMOOTHER_JACOBI ? L.dinv64.p : nullptr,
                                   c.allow_dia, L.At_lay);
+        }
+    // Gauss-Seidel sweeps by lines: structured levels whose operator has the
+    // level's element pattern (or R A P of it); a user's top operator may couple
+    // vertices across the ends of grid lines
+    if (m->smoother != UG4GB_SMOOTHER_JACOBI)
+        for (int l = m->base; l < nl; ++l) {
+            GLevel<V> &L = G->lev[l];
+            const uint64_t key = (g->uid << 6) + (uint64_t)(l + 1), have = A_top->pattern_key();
+            const bool own = l < nl - 1 || have == key || have == (key | (1ULL << 63));
+            L.gs = GsLines();
+            if (own && l > m->base && L.grid_transfer && L.At.kind == 1 && L.At_lay.known)
+                L.gs = gs_lines(L.At.dia.off, L.At.dia.S, L.At_lay.all, L.gp);
         }
     G->setup_base(c);
     G->setup_coarse(c);

@@ -119,6 +119,7 @@ struct GLevel {
     V *dcur = nullptr;
     std::vector<DevBuf<int>> crow;   // MCGS / ILU colour row lists
     std::vector<int> ncrow;
+    GsLines gs;                      // colour sweeps line by line (structured levels)
     DevBuf<int> vcolor;              // unstructured levels: colours of the operator's own graph
     IluFactors<V> ilu;               // ILU smoother factors
     DevBuf<V> y;                     // ILU forward-substitution scratch

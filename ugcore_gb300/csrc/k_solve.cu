@@ -22,6 +22,8 @@
 //                   pass (CG::apply_return_defect, cg.h:163-226)
 // Reductions are deterministic (grid_reduce: fixed-order tree per block,
 // block partials summed in block order by the last block).
+#include <algorithm>
+
 #include "k_solve.cuh"
 
 namespace ug4gb {
@@ -435,7 +437,10 @@ void smooth_step(Ctx &c, const OpMat<V> &At, const XT *x, const DT *dbase, const
                 return;
             }
         }
-        const bool pf = At.nrows <= c.num_sms * NT;
+        // rows loaded ahead of the launch wait: FP64 levels of one row per thread
+        // in a block per SM, FP32 ones of a whole wave (eight blocks per SM; 0.5 to
+        // 3% of a solve over the smaller limit, where FP64 lost up to 7%)
+        const bool pf = At.nrows <= c.num_sms * NT * (sizeof(V) == 4 ? 8 : 1);
         RedArgs none{nullptr, nullptr, nullptr};
         if (r_rho && pf) {
             UG_LAUNCH_PDL(c, (k_smooth<MV, V, XT, DT, true, true>), g, NT, 0, mv, x, dbase, dinv, sc, dout, sc_mode,
@@ -481,7 +486,7 @@ template <class V>
 void restrict_apply(Ctx &c, const OpMat<V> &R, const V *d, V *dc, const int *skip)
 {
     with_mv(R, [&](auto mv) {
-        if (R.nrows <= c.num_sms * NT)
+        if (R.nrows <= c.num_sms * NT * (sizeof(V) == 4 ? 8 : 1))
             UG_LAUNCH_PDL(c, (k_restrict<decltype(mv), V, true>), row_grid(c, R.nrows), NT, 0, mv, d, dc, skip);
         else
             UG_LAUNCH_PDL(c, (k_restrict<decltype(mv), V, false>), row_grid(c, R.nrows), NT, 0, mv, d, dc, skip);
@@ -518,7 +523,7 @@ template <class V>
 void prolong_apply(Ctx &c, const OpMat<V> &P, const V *scc, V *sc, const V *dfac, V *w, const int *skip)
 {
     with_mv(P, [&](auto mv) {
-        if (P.nrows <= c.num_sms * NT)
+        if (P.nrows <= c.num_sms * NT * (sizeof(V) == 4 ? 8 : 1))
             UG_LAUNCH_PDL(c, (k_prolong<decltype(mv), V, true>), row_grid(c, P.nrows), NT, 0, mv, scc, sc, dfac, w,
                           skip);
         else
@@ -773,6 +778,144 @@ void mcgs_colour(Ctx &c, const OpMat<V> &A, const int *rows, int nrows_c, const 
                   skip);
     });
 }
+
+// Two colours of a structured level in one launch: the lines (j, k) with the
+// parities (b1, b2), whose vertices couple within a line and to lines of other
+// parities only.  A block takes whole lines; a thread updates a vertex of
+// the first colour (x parity first), then, behind a barrier, its neighbour of
+// the second, so both halves of every sector of the operator are used while it
+// is in the cache, and a sweep takes 4 launches (2D: 2) instead of 8.
+// A sweep from t = 0 only reads the diagonals towards colours it has
+// updated (mask_even / mask_odd: those of the two x parities): the others
+// would multiply zeros, which leaves every sum as it is.
+// The operator entries of the first colour are loaded before the launch wait.
+// 97^3 hexes, FP32: eight launches of one colour each, with a pass that zeroed
+// t, 54 us a sweep.
+template <class V, int S>
+__global__ void __launch_bounds__(NT) k_mcgs_lines(DiaMV<V, S> A, int nx, int ny, int b1, int b2, int nly, int nlines,
+                                                   int nz, int per, int per_block, int first, unsigned mask_even,
+                                                   unsigned mask_odd, GsLines gs, bool from_zero,
+                                                   const V *__restrict__ dr,
+                                                   const V *__restrict__ d, V *t, const int *skip)
+{
+    const int step = per < NT ? per : NT;   // vertices of a line (one x parity) that are in work at a time
+    const int ln = threadIdx.x / step, q0 = threadIdx.x - ln * step;
+    const int line = blockIdx.x * per_block + ln;
+    const bool mine = ln < per_block && line < nlines;
+    const int j = b1 + 2 * (line % nly), k = b2 + 2 * (line / nly), base = nx * (j + ny * k);
+    unsigned off = 0u;   // the diagonals that leave the grid from this line
+    if (j == 0) off |= gs.edge[2];
+    if (j == ny - 1) off |= gs.edge[3];
+    if (k == 0) off |= gs.edge[4];
+    if (k == nz - 1) off |= gs.edge[5];
+    auto inside = [&](int i, unsigned mask) {
+        unsigned m = mask & ~off;
+        if (i == 0) m &= ~gs.edge[0];
+        if (i == nx - 1) m &= ~gs.edge[1];
+        return m;
+    };
+    auto load = [&](int i, unsigned mask, V(&a)[S]) {
+        mask = inside(i, mask);
+#pragma unroll
+        for (int e = 0; e < S; ++e)
+            if ((mask >> e) & 1u) a[e] = ld_stream(A.val + (size_t)e * A.ld + base + i);
+    };
+    auto update = [&](int i, unsigned mask, const V(&a)[S]) {
+        const int row = base + i;
+        mask = inside(i, mask);
+        V x[S];
+#pragma unroll
+        for (int e = 0; e < S; ++e)
+            if ((mask >> e) & 1u) x[e] = t[row + A.off.o[e]];
+        V acc = (V)0;
+#pragma unroll
+        for (int e = 0; e < S; ++e)
+            if ((mask >> e) & 1u) acc = fma_rn(a[e], x[e], acc);
+        const V old = from_zero ? (V)0 : t[row];
+        t[row] = fma_rn(dr[row], sub_rn(d[row], acc), old);
+    };
+    V a[S];
+    const unsigned m0 = first ? mask_odd : mask_even, m1 = first ? mask_even : mask_odd;
+    const int i0 = 2 * q0 + first;
+    pdl_trigger();
+    if (mine && i0 < nx) load(i0, m0, a);
+    pdl_wait();
+    if (skip && *skip) return;
+    if (mine)
+        for (int q = q0; q < per; q += step) {
+            const int i = 2 * q + first;
+            if (i >= nx) break;
+            if (q != q0) load(i, m0, a);
+            update(i, m0, a);
+        }
+    const int i1 = 2 * q0 + 1 - first;
+    if (mine && i1 < nx) load(i1, m1, a);
+    __syncthreads();
+    if (mine)
+        for (int q = q0; q < per; q += step) {
+            const int i = 2 * q + 1 - first;
+            if (i >= nx) break;
+            if (q != q0) load(i, m1, a);
+            update(i, m1, a);
+        }
+}
+
+GsLines gs_lines(const Offs &offs, int S, const std::vector<int> &entries, const GridPair &gp)
+{
+    GsLines g;
+    if (gp.nx < 3 || gp.ny < 3 || S > 32) return g;
+    for (int k = 0; k < S; ++k) {
+        const int o = offs.o[k];
+        if (!std::binary_search(entries.begin(), entries.end(), o)) continue;
+        int pm = -1;   // parity bits that differ along this offset
+        for (int z = gp.dim == 3 ? -1 : 0; z <= (gp.dim == 3 ? 1 : 0); ++z)
+            for (int y = -1; y <= 1; ++y)
+                for (int x = -1; x <= 1; ++x)
+                    if (x + gp.nx * (y + gp.ny * z) == o) {
+                        pm = (x & 1) | ((y & 1) << 1) | ((z & 1) << 2);
+                        if (x) g.edge[x > 0 ? 1 : 0] |= 1u << k;
+                        if (y) g.edge[y > 0 ? 3 : 2] |= 1u << k;
+                        if (z) g.edge[z > 0 ? 5 : 4] |= 1u << k;
+                    }
+        if (pm < 0) return g;
+        g.all |= 1u << k;
+        for (int c = 0; c < 8; ++c) {
+            if ((c ^ pm) < c) g.below[c] |= 1u << k;
+            if ((c ^ pm) > c) g.above[c] |= 1u << k;
+        }
+    }
+    g.usable = true;
+    return g;
+}
+
+template <class V>
+void mcgs_sweep_lines(Ctx &c, const OpMat<V> &A, const GsLines &gs, const GridPair &gp, bool backward, bool from_zero,
+                      const V *dinv_relax, const V *d, V *t, const int *skip)
+{
+    with_mv(A, [&](auto mv) {
+        using MV = decltype(mv);
+        if constexpr (is_dia<MV>::value) {
+            const int np = gp.dim == 3 ? 4 : 2, per = (gp.nx + 1) / 2, per_block = per < NT ? NT / per : 1;
+            for (int s = 0; s < np; ++s) {
+                const int p = backward ? np - 1 - s : s, b1 = p & 1, b2 = p >> 1;
+                const int nly = (gp.ny - b1 + 1) / 2, nlz = gp.dim == 3 ? (gp.nz - b2 + 1) / 2 : 1;
+                const int nlines = nly * nlz;
+                if (nlines <= 0) continue;
+                const unsigned *m = backward ? gs.above : gs.below;
+                const unsigned even = from_zero ? m[2 * p] : gs.all, odd = from_zero ? m[2 * p + 1] : gs.all;
+                UG_LAUNCH_PDL(c, (k_mcgs_lines<V, MV::kS>), div_up(nlines, per_block), NT, 0, mv, gp.nx, gp.ny, b1, b2,
+                              nly, nlines, gp.nz, per, per_block, backward ? 1 : 0, even, odd, gs, from_zero,
+                              dinv_relax, d, t, skip);
+            }
+        } else {
+            throw Error{UG4GB_ERR_INVALID, "Gauss-Seidel by lines: not a diagonal layout"};
+        }
+    });
+}
+template void mcgs_sweep_lines<double>(Ctx &, const OpMat<double> &, const GsLines &, const GridPair &, bool, bool,
+                                       const double *, const double *, double *, const int *);
+template void mcgs_sweep_lines<float>(Ctx &, const OpMat<float> &, const GsLines &, const GridPair &, bool, bool,
+                                      const float *, const float *, float *, const int *);
 
 template <class MV, class V, class DT>
 __global__ void __launch_bounds__(NT) k_resupd(MV A, const V *__restrict__ t, const DT *__restrict__ dbase,

@@ -280,6 +280,27 @@ bool coarse_width_ok(int S);
 // returns the blocks per cluster the device runs with that much (16 or 8)
 template <class V>
 int coarse_prepare(Ctx &c, size_t smem_bytes);
+// Multicolour Gauss-Seidel sweeps of a structured level line by line
+// (k_mcgs_lines): per colour (parity bits of the vertex), which diagonals lead
+// to vertices of lower colours, of higher ones, and which are entries at all.
+// (An entry beyond the grid's edge would multiply 0 with another line's value,
+// which a sweep from zero may not have written.)
+struct GsLines {
+    bool usable = false;
+    unsigned below[8] = {}, above[8] = {};
+    unsigned all = 0;
+    unsigned edge[6] = {};   // the diagonals that leave the grid at x = 0, x = max, y = 0, ...
+};
+// offs: the layout's offsets, entries: those of them that the CRS holds (the
+// rest is padding); unusable where an entry is no neighbour in the grid or
+// couples vertices of one colour
+GsLines gs_lines(const Offs &offs, int S, const std::vector<int> &entries, const GridPair &gp);
+// one sweep over all colours: t_i = t_i + dinv_relax_i (d_i - (A t)_i), colours
+// increasing or (backward) decreasing; from_zero: t is 0 before the sweep and
+// need not be written
+template <class V>
+void mcgs_sweep_lines(Ctx &c, const OpMat<V> &A, const GsLines &gs, const GridPair &gp, bool backward, bool from_zero,
+                      const V *dinv_relax, const V *d, V *t, const int *skip);
 template <class V>
 void mcgs_colour(Ctx &c, const OpMat<V> &A, const int *rows, int nrows_c, const V *dinv_relax, const V *d, V *t,
                  const int *skip);
