@@ -576,7 +576,8 @@ struct GmgT : GmgBase {
                 T.gp.nx * T.gp.ny * T.gp.nz != T.n || T.gp.cnx * T.gp.cny * T.gp.cnz != lev[t - 1].n ||
                 !coarse_width_ok(T.At.dia.S) || T.At.dia.S != lev[base + 1].At.dia.S)
                 break;
-            if (c.coarse_levels > 0 ? t - base > c.coarse_levels : work(t) > kSharedWork) break;
+            // (a level prepared for two steps per pass keeps its own launches)
+            if (c.coarse_levels > 0 ? t - base > c.coarse_levels : work(t) > kSharedWork || T.sweep2) break;
             CoarsePlan<V> P{};
             P.m = t - base + 1;
             bool any_shared = !solo_base;
