@@ -208,17 +208,22 @@ static void dense_lu_inverse(int n, std::vector<double> &M, std::vector<double> 
 
 // The same factorisation on the device for bases of at most kDeviceLuMax
 // unknowns (no host round trip in a re-initialisation): one block, M in
-// shared memory, the inverse X built in place in the output array.  Partial
-// pivoting as above (the first row of the largest magnitude), row swaps
-// applied to X = I as they happen, products and differences rounded
-// separately; the forward substitution runs over all columns at once,
-// right-looking (subtracting in increasing column order), the backward one
-// column by column in the order of SolveLU, so that each element of the
-// inverse takes the operations of the host statement above.  *status = 1 on a
-// pivot below 1e-10 (the output is then not an inverse).
-constexpr int kDeviceLuMax = 160;
-constexpr int kLuThreads = 256;
+// shared memory, up to kLuSharedX unknowns the inverse X too (beyond them it is
+// built in place in the output array).  Partial pivoting as above (the first
+// row of the largest magnitude), row swaps applied to M and X = I, products and
+// differences rounded separately; the forward substitution runs over all columns
+// as the factorisation goes (subtracting in increasing column order), the
+// backward one column by column in the order of SolveLU, so that each element of
+// the inverse takes the operations of the host statement above.  That order
+// leaves chains of dependent FP64 differences, and FP64 is slow on one SM; but
+// most rows of a base level are Dirichlet rows (56 of 64 for 3 x 3 x 3 cells):
+// products with a zero factor, which change nothing, are skipped, by rows, by
+// warps of columns, and in the backward sums by the row's nonzero bits.
+// *status = 1 on a pivot below 1e-10 (the output is then not an inverse).
+constexpr int kDeviceLuMax = 160, kLuSharedX = 104;
+constexpr int kLuThreads = 512, kLuWords = (kDeviceLuMax + 31) / 32;
 
+template <bool XS>
 __global__ void __launch_bounds__(kLuThreads) k_base_lu(const int *__restrict__ rowptr, const int *__restrict__ col,
                                                         const double *__restrict__ val, int n,
                                                         double *__restrict__ inv, int *__restrict__ status)
@@ -226,8 +231,10 @@ __global__ void __launch_bounds__(kLuThreads) k_base_lu(const int *__restrict__ 
     PDL_ENTRY();
     extern __shared__ double lu_sh[];
     __shared__ int big_sh;
-    double *M = lu_sh, *X = inv;
-    const int tid = threadIdx.x, nt = blockDim.x, nn = n * n;
+    __shared__ unsigned bits[kDeviceLuMax][kLuWords];
+    const int tid = threadIdx.x, nt = blockDim.x, nn = n * n, lane = tid & 31, warp = tid >> 5, nw = nt >> 5;
+    double *M = lu_sh;
+    double *X = XS ? lu_sh + nn : inv;
     for (int i = tid; i < nn; i += nt) {
         M[i] = 0.0;
         X[i] = 0.0;
@@ -263,7 +270,7 @@ __global__ void __launch_bounds__(kLuThreads) k_base_lu(const int *__restrict__ 
         }
         __syncthreads();
         const int big = big_sh;
-        if (big != k)
+        if (big != k) {
             for (int j = tid; j < n; j += nt) {
                 const double t = M[k * n + j];
                 M[k * n + j] = M[big * n + j];
@@ -272,37 +279,69 @@ __global__ void __launch_bounds__(kLuThreads) k_base_lu(const int *__restrict__ 
                 X[k * n + j] = X[big * n + j];
                 X[big * n + j] = u;
             }
-        __syncthreads();
+            __syncthreads();
+        }
         const double p = M[k * n + k];
         if (!(fabs(p) >= 1e-10)) {
             if (tid == 0) *status = 1;
             return;
         }
-        for (int i = k + 1 + tid; i < n; i += nt) M[i * n + k] = __ddiv_rn(M[i * n + k], p);
+        for (int i = k + 1 + tid; i < n; i += nt)
+            if (M[i * n + k] != 0.0) M[i * n + k] = __ddiv_rn(M[i * n + k], p);
         __syncthreads();
-        const int m = n - k - 1;
-        for (int t = tid; t < m * m; t += nt) {
-            const int i = k + 1 + t / m, j = k + 1 + t % m;
-            M[i * n + j] = __dsub_rn(M[i * n + j], __dmul_rn(M[i * n + k], M[k * n + j]));
+        for (int c0 = 0; c0 < n; c0 += 32) {
+            const int c = c0 + lane;
+            const double mk = (c > k && c < n) ? M[k * n + c] : 0.0, xk = c < n ? X[k * n + c] : 0.0;
+            const bool some_m = __any_sync(0xffffffffu, mk != 0.0), some_x = __any_sync(0xffffffffu, xk != 0.0);
+            if (!some_m && !some_x) continue;
+            for (int i = k + 1 + warp; i < n; i += nw) {
+                const double f = M[i * n + k];
+                if (f == 0.0) continue;
+                if (some_m && c > k && c < n) M[i * n + c] = __dsub_rn(M[i * n + c], __dmul_rn(f, mk));
+                if (some_x && c < n) X[i * n + c] = __dsub_rn(X[i * n + c], __dmul_rn(f, xk));
+            }
         }
         __syncthreads();
     }
-    for (int k = 0; k < n; ++k) {
-        const int m = n - k - 1;
-        for (int t = tid; t < m * n; t += nt) {
-            const int i = k + 1 + t / n, c = t % n;
-            X[i * n + c] = __dsub_rn(X[i * n + c], __dmul_rn(M[i * n + k], X[k * n + c]));
+    // the nonzero columns behind each row's diagonal
+    for (int t = tid; t < n * kLuWords; t += nt) {
+        const int i = t / kLuWords, w = t % kLuWords;
+        unsigned b = 0u;
+        for (int q = 0; q < 32; ++q) {
+            const int k = 32 * w + q;
+            if (k > i && k < n && M[i * n + k] != 0.0) b |= 1u << q;
         }
-        __syncthreads();
+        bits[i][w] = b;
     }
+    __syncthreads();
     // backward: one thread per column, each row's sum in increasing column
     // order as SolveLU (the columns are independent: no barrier)
     for (int c = tid; c < n; c += nt)
         for (int i = n - 1; i >= 0; --i) {
             double v = X[i * n + c];
-            for (int k = i + 1; k < n; ++k) v = __dsub_rn(v, __dmul_rn(M[i * n + k], X[k * n + c]));
-            X[i * n + c] = __ddiv_rn(v, M[i * n + i]);
+            const double *m = M + i * n;
+            for (int w = i / 32; w < (n + 31) / 32; ++w)
+                for (unsigned b = bits[i][w]; b;) {
+                    double pr[4];
+                    int cnt = 0;
+#pragma unroll
+                    for (int q = 0; q < 4; ++q)
+                        if (b) {
+                            const int k = 32 * w + __ffs(b) - 1;
+                            b &= b - 1u;
+                            pr[q] = __dmul_rn(m[k], X[k * n + c]);
+                            cnt = q + 1;
+                        }
+#pragma unroll
+                    for (int q = 0; q < 4; ++q)
+                        if (q < cnt) v = __dsub_rn(v, pr[q]);
+                }
+            X[i * n + c] = m[i] == 1.0 ? v : __ddiv_rn(v, m[i]);
         }
+    if (XS) {
+        __syncthreads();
+        for (int i = tid; i < nn; i += nt) inv[i] = X[i];
+    }
     if (tid == 0) *status = 0;
 }
 
@@ -511,12 +550,19 @@ struct GmgT : GmgBase {
         int n = A.nrows;
         UG_REQUIRE(n <= 4096, UG4GB_ERR_INVALID, "GMG base level larger than 4096 unknowns (dense LU limit)");
         if (n <= kDeviceLuMax) {
-            const size_t smem = (size_t)kDeviceLuMax * kDeviceLuMax * sizeof(double);
-            UG_CUDA(cudaFuncSetAttribute(k_base_lu, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+            const bool xs = n <= kLuSharedX;
+            const size_t smem = (size_t)n * n * sizeof(double) * (xs ? 2 : 1);
+            if (smem > 48 * 1024)
+                UG_CUDA(cudaFuncSetAttribute(xs ? k_base_lu<true> : k_base_lu<false>,
+                                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
             Ainv.alloc((size_t)n * n);
             lu_status.alloc(1);
-            UG_LAUNCH_PDL(c, k_base_lu, 1, kLuThreads, (size_t)n * n * sizeof(double), A.rowptr.p, A.col.p, A.val.p,
-                      n, Ainv.p, lu_status.p);
+            if (xs)
+                UG_LAUNCH_PDL(c, k_base_lu<true>, 1, kLuThreads, smem, A.rowptr.p, A.col.p, A.val.p, n, Ainv.p,
+                              lu_status.p);
+            else
+                UG_LAUNCH_PDL(c, k_base_lu<false>, 1, kLuThreads, smem, A.rowptr.p, A.col.p, A.val.p, n, Ainv.p,
+                              lu_status.p);
             // no wait: the status is read back behind the factorisation and
             // checked after the next apply's or solve's own wait (check_base)
             if (!lu_host) UG_CUDA(cudaMallocHost((void **)&lu_host, sizeof(int)));

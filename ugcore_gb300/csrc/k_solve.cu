@@ -320,8 +320,12 @@ __global__ void __launch_bounds__(NT) k_smooth(MV A, const XT *__restrict__ x, c
 // thread that owns the last, partial group.  Per row the arithmetic is that
 // of k_smooth.  32 registers (8 blocks of 256 threads per SM): the sweep is
 // bound by memory latency, and the extra resident warps gave 2-4% per sweep.
+// (The 7-diagonal step with the reduction spilled at 32: 40 registers, 6 blocks,
+// 25.7 -> 22.0 us on the 129^3 tet level.)
+constexpr int smooth_dia_blocks(int S, bool rho) { return S == 7 && rho ? 6 : 8; }   // resident per SM
+
 template <class V, int S, bool RHO>
-__global__ void __launch_bounds__(NT, 8) k_smooth_dia(DiaMV<V, S> A, const V *__restrict__ x, const V *__restrict__ dbase,
+__global__ void __launch_bounds__(NT, smooth_dia_blocks(S, RHO)) k_smooth_dia(DiaMV<V, S> A, const V *__restrict__ x, const V *__restrict__ dbase,
                                                    const V *__restrict__ dinv, V *__restrict__ sc, V *__restrict__ dout,
                                                    int sc_mode, const int *skip, const double *__restrict__ r_rho,
                                                    RedArgs red, int rho_kind, double *__restrict__ z64)
@@ -426,7 +430,7 @@ void smooth_step(Ctx &c, const OpMat<V> &At, const XT *x, const DT *dbase, const
                     // with the fused (z, r) reduction: one resident wave of blocks
                     // (8 per SM), so the blocks' reduction tails overlap and the
                     // last block sums fewer partials (-12% on the 129^3 tet level)
-                    const int gr = gv < c.num_sms * 8 ? gv : c.num_sms * 8;
+                    const int wave = c.num_sms * smooth_dia_blocks(MV::kS, true), gr = gv < wave ? gv : wave;
                     UG_LAUNCH_PDL(c, (k_smooth_dia<V, MV::kS, true>), gr, NT, 0, mv, x, dbase, dinv, sc, dout, sc_mode,
                                   skip, r_rho, *red, rho_kind, z64);
                 } else {
@@ -683,7 +687,8 @@ template <class V>
 void prolong_grid(Ctx &c, const GridPair &g, const V *scc, V *sc, const V *dfac, V *w, const int *skip)
 {
     const int per = (g.nx + 1) / 2, npairs = per * g.ny * g.nz;
-    UG_LAUNCH_PDL(c, k_prolong_grid<V>, row_grid(c, npairs), NT, 0, g, FastDiv(per), FastDiv(g.ny), npairs, scc, sc,
+    const int grid = sizeof(V) == 8 ? (int)div_up(npairs, NT) : row_grid(c, npairs);
+    UG_LAUNCH_PDL(c, k_prolong_grid<V>, grid, NT, 0, g, FastDiv(per), FastDiv(g.ny), npairs, scc, sc,
                   dfac, w, skip);
 }
 
@@ -818,7 +823,7 @@ __global__ void __launch_bounds__(NT) k_mcgs_lines(DiaMV<V, S> A, int nx, int ny
         mask = inside(i, mask);
 #pragma unroll
         for (int e = 0; e < S; ++e)
-            if ((mask >> e) & 1u) a[e] = ld_stream(A.val + (size_t)e * A.ld + base + i);
+            if ((mask >> e) & 1u) a[e] = __ldg(A.val + (size_t)e * A.ld + base + i);
     };
     auto update = [&](int i, unsigned mask, const V(&a)[S]) {
         const int row = base + i;
