@@ -383,31 +383,6 @@ __device__ __forceinline__ void row_in_time(const AsmArgs &a, double (&acc)[Sten
     acc[S::slot(0, 0, 0)] += a.sm0 * volsum;
 }
 
-// interior rows: one thread per row, every value written once
-template <int T, bool INST>
-__global__ void __launch_bounds__(128) k_assemble_rows(AsmArgs a, ClassData<T> cd, const double *__restrict__ flux,
-                                                       double volsum)
-{
-    PDL_ENTRY();
-    using S = Stencil<T>;
-    const int nix = a.cx - 1, niy = a.cy - 1, niz = (S::DIM == 3) ? a.cz - 1 : 1;
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= nix * niy * niz) return;
-    const int i = 1 + t % nix, j = 1 + (t / nix) % niy, k = (S::DIM == 3) ? 1 + t / (nix * niy) : 0;
-    const int nx = a.cx + 1, ny = a.cy + 1;
-    const int r = i + nx * (j + ny * k);
-    double acc[S::N];
-#pragma unroll
-    for (int s = 0; s < S::N; ++s) acc[s] = 0.0;
-    gather_row<T>(cd, a, i, j, k, flux, [&](int s, double v) { acc[s] += v; }, [](double) {});
-    if (a.b) a.b[r] = row_rhs<T, INST>(a, acc, r, volsum);
-    if constexpr (INST) row_in_time<T>(a, acc, volsum);
-    double *row = a.val + __ldg(a.rowptr + r);
-#pragma unroll
-    for (int s = 0; s < S::N; ++s) row[s] = acc[s];
-}
-
-
 // rows on the box boundary: the identity row and b = 0 at Dirichlet
 // vertices; otherwise the elements that exist, entries found by search
 // a boundary row without the Dirichlet flag: the elements that exist, entries
@@ -488,7 +463,7 @@ __device__ __forceinline__ void boundary_row(const AsmArgs &a, const ClassData<T
 
 // small levels (launch-bound): every row of the level in one launch, one
 // thread per row, interior rows as k_assemble_rows, boundary rows as
-// k_assemble_boundary_rows
+// k_assemble_rows
 template <int T, bool INST>
 __global__ void __launch_bounds__(128) k_assemble_rows_all(AsmArgs a, ClassData<T> cd, const double *__restrict__ flux,
                                                            double volsum, const unsigned char *__restrict__ bnd)
@@ -514,17 +489,49 @@ __global__ void __launch_bounds__(128) k_assemble_rows_all(AsmArgs a, ClassData<
     for (int s = 0; s < S::N; ++s) row[s] = acc[s];
 }
 
-// the rows of a list (the box surface), one warp per row
-template <int T>
-__global__ void __launch_bounds__(256) k_assemble_boundary_rows(AsmArgs a, ClassData<T> cd,
-                                                                const double *__restrict__ flux,
-                                                                const unsigned char *__restrict__ bnd,
-                                                                const int *__restrict__ brows, int nbrows)
+// Large levels: the first nbb blocks take the rows of a list (the box surface),
+// one warp per row, memory work that the others' FP64 work hides (a launch of
+// its own: 25 us on 129^3); the others the interior rows, one thread per row,
+// every value written once.  A warp's 32 rows go through shared memory, so that
+// consecutive threads write consecutive values (each thread writing its own row
+// of 27 touched 32 sectors, 8 bytes in each, per store).
+template <int T, bool INST>
+__global__ void __launch_bounds__(128) k_assemble_rows(AsmArgs a, ClassData<T> cd, const double *__restrict__ flux,
+                                                       double volsum, const unsigned char *__restrict__ bnd,
+                                                       const int *__restrict__ brows, int nbrows, int nbb)
 {
     PDL_ENTRY();
-    const int t = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
-    if (t >= nbrows) return;
-    boundary_row<T>(a, cd, flux, bnd, brows[t], threadIdx.x & 31);
+    using S = Stencil<T>;
+    __shared__ double rows[4][32 * S::N];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if ((int)blockIdx.x < nbb) {
+        const int t = blockIdx.x * 4 + warp;
+        if (t < nbrows) boundary_row<T>(a, cd, flux, bnd, brows[t], lane);
+        return;
+    }
+    const int nix = a.cx - 1, niy = a.cy - 1, niz = (S::DIM == 3) ? a.cz - 1 : 1;
+    const int t = (blockIdx.x - nbb) * blockDim.x + threadIdx.x;
+    int start = -1;   // of this thread's row in the values
+    if (t < nix * niy * niz) {
+        const int i = 1 + t % nix, j = 1 + (t / nix) % niy, k = (S::DIM == 3) ? 1 + t / (nix * niy) : 0;
+        const int nx = a.cx + 1, ny = a.cy + 1;
+        const int r = i + nx * (j + ny * k);
+        start = __ldg(a.rowptr + r);
+        double acc[S::N];
+#pragma unroll
+        for (int s = 0; s < S::N; ++s) acc[s] = 0.0;
+        gather_row<T>(cd, a, i, j, k, flux, [&](int s, double v) { acc[s] += v; }, [](double) {});
+        if (a.b) a.b[r] = row_rhs<T, INST>(a, acc, r, volsum);
+        if constexpr (INST) row_in_time<T>(a, acc, volsum);
+#pragma unroll
+        for (int s = 0; s < S::N; ++s) rows[warp][lane * S::N + s] = acc[s];
+    }
+    __syncwarp();
+#pragma unroll 3
+    for (int q = lane; q < 32 * S::N; q += 32) {
+        const int row = q / S::N, b = __shfl_sync(0xffffffffu, start, row);
+        if (b >= 0) a.val[(size_t)b + (q - row * S::N)] = rows[warp][q];
+    }
 }
 
 // One coefficient K for all elements and no convection: every interior row
@@ -889,9 +896,9 @@ void run_assemble_rows(Ctx &c, const Level &L, const AsmArgs &a, const ClassData
     } else if (L.nv <= kSmallLevelRows) {
         UG_LAUNCH_PDL(c, (k_assemble_rows_all<T, INST>), div_up(L.nv, 128), 128, 0, a, cd, flux, cache.volsum, L.bnd.p);
     } else {
-        UG_LAUNCH_PDL(c, (k_assemble_rows<T, INST>), div_up(nint, 128), 128, 0, a, cd, flux, cache.volsum);
-        UG_LAUNCH_PDL(c, k_assemble_boundary_rows<T>, div_up(cache.nbrows, 8), 256, 0, a, cd, flux, L.bnd.p,
-                      cache.brows.p, cache.nbrows);
+        const int nbb = (int)div_up(cache.nbrows, 4);
+        UG_LAUNCH_PDL(c, (k_assemble_rows<T, INST>), nbb + (int)div_up(nint, 128), 128, 0, a, cd, flux, cache.volsum,
+                      L.bnd.p, cache.brows.p, cache.nbrows, nbb);
     }
 }
 

@@ -552,7 +552,12 @@ __global__ void __launch_bounds__(kFillRows) k_dia_fill(const int *__restrict__ 
     const int q0 = rowptr[r0], q1 = rowptr[r1];
     const bool staged = q1 - q0 <= kFillRows * kFillMax;
     if (staged)
-        for (int q = q0 + threadIdx.x; q < q1; q += kFillRows) sv[q - q0] = ld_stream(val + q);
+        for (int q = q0 + threadIdx.x; q < q1; q += kFillRows) {
+            // asynchronous: all of a thread's copies are in flight together
+            const unsigned d = (unsigned)__cvta_generic_to_shared(sv + (q - q0));
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(d), "l"(val + q) : "memory");
+        }
+    asm volatile("cp.async.wait_all;" ::: "memory");
     __syncthreads();
     const int r = r0 + threadIdx.x;
     if (r >= nrows) return;
@@ -574,11 +579,21 @@ __global__ void __launch_bounds__(kFillRows) k_dia_fill(const int *__restrict__ 
 #pragma unroll 3
         for (int k = 0; k < len; ++k) put(k, r + m.off[k], staged ? sv[a0 - q0 + k] : val[a0 + k]);
     } else {
-        for (int a = a0; a < a0 + len; ++a) {
-            const int c = col[a];
-            int k = 0;
-            while (k < m.n && m.off[k] != c - r) ++k;
-            if (k < m.n) put(k, c, staged ? sv[a - q0] : val[a]);   // m holds every offset of A
+        // a few columns' loads in flight at a time: one after the other, these
+        // rows (two in 129 on a structured level) held up their blocks
+        constexpr int B = 9;
+        int k = 0;
+        for (int a = a0; a < a0 + len; a += B) {
+            int c[B];
+#pragma unroll
+            for (int q = 0; q < B; ++q) c[q] = a + q < a0 + len ? __ldg(col + a + q) : 0;
+#pragma unroll
+            for (int q = 0; q < B; ++q)
+                if (a + q < a0 + len) {
+                    if (!sorted) k = 0;
+                    while (k < m.n && m.off[k] != c[q] - r) ++k;
+                    if (k < m.n) put(k, c[q], staged ? sv[a + q - q0] : val[a + q]);   // m holds every offset of A
+                }
         }
     }
     if (bad) *left_out = 1;
