@@ -401,7 +401,7 @@ struct GmgT : GmgBase {
             mix(L.ilu.val.p); mix(L.ilu.col.p); mix(L.ilu.rowptr.p); mix(L.ilu.nlow.p); mix(L.ilu.uinv.p);
             h ^= (uint64_t)L.n;
             for (int k = 0; k < L.At.dia.S; ++k) mix((const void *)(intptr_t)L.At.dia.off.o[k]);
-            mix((const void *)(intptr_t)(L.gs.usable ? 1 : 0));
+            mix((const void *)(intptr_t)((L.gs.usable ? 1 : 0) + (L.level2d ? 2 : 0)));
         }
         mix(Ainv.p);
         mix(z64.p);
@@ -605,7 +605,7 @@ struct GmgT : GmgBase {
         constexpr size_t kSmemMax = 208 * 1024;
         int &coarse_ctas = c.coarse_ctas[sizeof(V) == 8 ? 0 : 1];
         if (coarse_ctas == 0) coarse_ctas = coarse_prepare<V>(c, kSmemMax);   // the most any multigrid asks for
-        constexpr double kSharedWork = 110e3, kSoloWork = 1000.0;
+        constexpr double kSharedWork = 110e3, kSharedWork2d = 400.0, kSoloWork = 1000.0;
         constexpr int kBaseRows = 32;
         constexpr int kAlign = 16 / (int)sizeof(V);   // elements per 16 bytes
         auto up = [](size_t v, size_t a) { return (v + a - 1) / a * a; };
@@ -622,8 +622,11 @@ struct GmgT : GmgBase {
                 T.gp.nx * T.gp.ny * T.gp.nz != T.n || T.gp.cnx * T.gp.cny * T.gp.cnz != lev[t - 1].n ||
                 !coarse_width_ok(T.At.dia.S) || T.At.dia.S != lev[base + 1].At.dia.S)
                 break;
-            // (a level prepared for two steps per pass keeps its own launches)
-            if (c.coarse_levels > 0 ? t - base > c.coarse_levels : work(t) > kSharedWork || T.sweep2) break;
+            // (a level prepared for two steps per pass keeps its own launches; one
+            // that takes two launches a cycle, k_level2d.cu, does so from 9^2 on:
+            // 129^2 solve 540 -> 527 us, FP32 416 -> 361 us)
+            const double limit = T.level2d && nu1 == 2 && nu2 == 2 ? kSharedWork2d : kSharedWork;
+            if (c.coarse_levels > 0 ? t - base > c.coarse_levels : work(t) > limit || T.sweep2) break;
             CoarsePlan<V> P{};
             P.m = t - base + 1;
             bool any_shared = !solo_base;
@@ -719,9 +722,14 @@ struct GmgT : GmgBase {
         }
         GLevel<V> &C = lev[l - 1];
         const V *cur = (l == T) ? top_in : L.dcur;
+        const bool pre2d = L.level2d && nu1 == 2 && first;
+        if (pre2d) {
+            level2d_pre<V>(c, L.At, L.gp, L.dinv.p, cur, L.sc.p, L.dB.p, C.dA.p, skip);
+            cur = L.dB.p;
+        }
         // ---- pre-smoothing
         if (nu1 == 0 && first) UG_LAUNCH_PDL(c, k_zero<V>, div_up(L.n, 256), 256, 0, L.n, L.sc.p, skip);
-        for (int k = 0; k < nu1; ++k) {
+        for (int k = 0; k < nu1 && !pre2d; ++k) {
             V *out = (cur == L.dA.p) ? L.dB.p : L.dA.p;
             int mode = (k == 0) ? (first ? SC_SET_FROM_BASE : SC_ADD_FROM_BASE) : SC_ADD_FROM_BASE;
             // two steps in one pass over the operator where the level allows it
@@ -742,7 +750,9 @@ struct GmgT : GmgBase {
         }
         const V *dpre = cur;
         // ---- restriction
-        if (L.grid_transfer) restrict_grid<V>(c, L.gp, dpre, C.dA.p, skip);
+        if (pre2d) {
+            // done
+        } else if (L.grid_transfer) restrict_grid<V>(c, L.gp, dpre, C.dA.p, skip);
         else restrict_apply<V>(c, L.Rs, dpre, C.dA.p, skip);
         C.dcur = C.dA.p;
         // ---- coarse correction
@@ -763,6 +773,14 @@ struct GmgT : GmgBase {
         }
         c.prof_tag = "L" + std::to_string(l);
         // ---- prolongation + post-smoothing
+        if (L.level2d && nu2 == 2 && (l == T || cycle == 1)) {
+            const bool top_level = l == T;
+            level2d_post<V>(c, L.At, L.gp, L.dinv.p, L.dfac.p, C.sc.p, dpre, L.sc.p, skip, top_level ? r_rho : nullptr,
+                            top_level ? red : nullptr, rho_kind, top_level ? z64.p : nullptr);
+            if (top_level) rho_done = (r_rho != nullptr);
+            L.dcur = const_cast<V *>(dpre);   // read by no later visit
+            return;
+        }
         if (L.grid_transfer) prolong_grid<V>(c, L.gp, C.sc.p, L.sc.p, L.dfac.p, nu2 > 0 ? L.w.p : (V *)nullptr, skip);
         else prolong_apply<V>(c, L.Ps, C.sc.p, L.sc.p, L.dfac.p, nu2 > 0 ? L.w.p : (V *)nullptr, skip);
         const V *dbase = dpre;
@@ -1000,18 +1018,21 @@ static GmgBase *build_gmg(ug4gb_gmg *m, const ug4gb_matrix *A_top, GmgT<V> *reus
             op_from_csr_cached<V>(c, L.A, L.At, m->smoother == UG4GB_SMOOTHER_JACOBI ? L.dinv64.p : nullptr,
                                   c.allow_dia, L.At_lay);
         }
-    // Gauss-Seidel sweeps by lines: structured levels whose operator has the
+    // Gauss-Seidel sweeps by lines, 2D levels in two launches: structured levels whose operator has the
     // level's element pattern (or R A P of it); a user's top operator may couple
     // vertices across the ends of grid lines
-    if (m->smoother != UG4GB_SMOOTHER_JACOBI)
-        for (int l = m->base; l < nl; ++l) {
-            GLevel<V> &L = G->lev[l];
-            const uint64_t key = (g->uid << 6) + (uint64_t)(l + 1), have = A_top->pattern_key();
-            const bool own = l < nl - 1 || have == key || have == (key | (1ULL << 63));
-            L.gs = GsLines();
-            if (own && l > m->base && L.grid_transfer && L.At.kind == 1 && L.At_lay.known)
-                L.gs = gs_lines(L.At.dia.off, L.At.dia.S, L.At_lay.all, L.gp);
-        }
+    for (int l = m->base; l < nl; ++l) {
+        GLevel<V> &L = G->lev[l];
+        const uint64_t key = (g->uid << 6) + (uint64_t)(l + 1), have = A_top->pattern_key();
+        const bool own = l < nl - 1 || have == key || have == (key | (1ULL << 63));
+        L.gs = GsLines();
+        L.level2d = false;
+        if (!own || l == m->base || !L.grid_transfer || L.At.kind != 1) continue;
+        if (m->smoother == UG4GB_SMOOTHER_JACOBI)
+            L.level2d = m->smoother2 == UG4GB_SMOOTHER_JACOBI && level2d_ok<V>(L.At, L.gp);
+        else if (L.At_lay.known)
+            L.gs = gs_lines(L.At.dia.off, L.At.dia.S, L.At_lay.all, L.gp);
+    }
     G->setup_base(c);
     G->setup_coarse(c);
     if (sizeof(V) != sizeof(double)) G->z64.alloc(g->lev[nl - 1].nv);

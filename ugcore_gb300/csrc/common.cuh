@@ -424,14 +424,15 @@ __device__ __forceinline__ void grid_reduce(const double (&v)[NV], double *parti
 {
     __shared__ double sh[NV][NT];
     __shared__ bool is_last;
+    const int block = blockIdx.x + gridDim.x * blockIdx.y, nblocks = gridDim.x * gridDim.y;
     block_sum<NT, NV>(v, sh);
     if (NV > 1) __syncthreads();
     if (threadIdx.x == 0) {
 #pragma unroll
-        for (int q = 0; q < NV; ++q) partials[q * kRedMaxBlocks + blockIdx.x] = sh[q][0];
+        for (int q = 0; q < NV; ++q) partials[q * kRedMaxBlocks + block] = sh[q][0];
         __threadfence();
         unsigned t = atomicAdd(counter, 1u);
-        is_last = (t == gridDim.x - 1);
+        is_last = (t == (unsigned)nblocks - 1u);
     }
     __syncthreads();
     if (!is_last) return;
@@ -440,7 +441,7 @@ __device__ __forceinline__ void grid_reduce(const double (&v)[NV], double *parti
 #pragma unroll
     for (int q = 0; q < NV; ++q) {
         double s = 0.0;
-        for (int b = threadIdx.x; b < (int)gridDim.x; b += NT) s += __ldcg(partials + q * kRedMaxBlocks + b);
+        for (int b = threadIdx.x; b < nblocks; b += NT) s += __ldcg(partials + q * kRedMaxBlocks + b);
         tot[q] = s;
     }
     block_sum<NT, NV>(tot, sh);

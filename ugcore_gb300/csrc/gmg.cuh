@@ -119,6 +119,7 @@ struct GLevel {
     V *dcur = nullptr;
     std::vector<DevBuf<int>> crow;   // MCGS / ILU colour row lists
     std::vector<int> ncrow;
+    bool level2d = false;            // smoothing and transfers in two launches (k_level2d.cu)
     GsLines gs;                      // colour sweeps line by line (structured levels)
     DevBuf<int> vcolor;              // unstructured levels: colours of the operator's own graph
     IluFactors<V> ilu;               // ILU smoother factors

@@ -280,6 +280,34 @@ bool coarse_width_ok(int S);
 // returns the blocks per cluster the device runs with that much (16 or 8)
 template <class V>
 int coarse_prepare(Ctx &c, size_t smem_bytes);
+// ---- a 2D level of the V-cycle in two launches (k_level2d.cu) ----
+template <class V>
+struct DiaRows {
+    const V *val;   // diagonal layout, S x ld
+    int ld;
+};
+// FP64 levels of up to this many vertices: above, the repeated vertices of the
+// tiles cost more FP64 time than the launches they save (solves in FP64: 257^2 751
+// -> 738 us, 385^2 986 either way, 513^2 1237 -> 1318 us).  FP32 levels gain at
+// more (257^2 617 -> 493 us, 513^2 862 -> 690 us; from the size of the wide steps of
+// k_smooth_dia on not: 1025^2 1279 -> 1368 us): the operator is read 1.6
+// and 1.4 times instead of four times.
+template <class V>
+constexpr int64_t kLevel2dRows = sizeof(V) == 8 ? 100000 : 900000;
+// At holds the nine-point stencil of the structured 2D level gp, quadrilaterals
+template <class V>
+bool level2d_ok(const OpMat<V> &At, const GridPair &gp);
+// two damped-Jacobi steps from sc = 0 and the defect d (sc, and the defect in
+// dout, which d is not), dc = R dout
+template <class V>
+void level2d_pre(Ctx &c, const OpMat<V> &At, const GridPair &gp, const V *dinv, const V *d, V *sc, V *dout, V *dc,
+                 const int *skip);
+// sc += P scc and two damped-Jacobi steps from the defect d; r_rho, z64 as in
+// smooth_step
+template <class V>
+void level2d_post(Ctx &c, const OpMat<V> &At, const GridPair &gp, const V *dinv, const V *dfac, const V *scc,
+                  const V *d, V *sc, const int *skip, const double *r_rho, RedArgs *red, int rho_kind, double *z64);
+
 // Multicolour Gauss-Seidel sweeps of a structured level line by line
 // (k_mcgs_lines): per colour (parity bits of the vertex), which diagonals lead
 // to vertices of lower colours, of higher ones, and which are entries at all.
