@@ -842,10 +842,15 @@ __global__ void k_transpose_symmetric(const int *rowptr, const int *col, double 
     PDL_ENTRY();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    for (int a = rowptr[i]; a < rowptr[i + 1]; ++a) {
+    const int a0 = rowptr[i], a1 = rowptr[i + 1];
+#pragma unroll 4
+    for (int a = a0; a < a1; ++a) {
         const int j = col[a];
         if (j <= i) continue;
-        const int b = row_find(rowptr, col, j, i);
+        // in a stencil's rows (i, j) stands as far from its row's end as (j, i)
+        // from the start of its own: looked at before a search is made
+        int b = rowptr[j] + (a1 - 1 - a);
+        if (b >= rowptr[j + 1] || col[b] != i) b = row_find(rowptr, col, j, i);
         if (b < 0) continue;
         const double t = val[a];
         val[a] = val[b];
