@@ -25,21 +25,25 @@ const double *disc_coefficients(ug4gb_disc *d, int level)
     }
     if (D.Kvalid[level]) return D.Klev[level].p;
     if (D.coef_kind == COEF_LOG_ELEMS) {
-        // log K on every level from the top: children's mean, then exp
-        std::vector<DevBuf<double>> logk(nl);
-        logk[nl - 1].alloc(lev[nl - 1].ne);
-        UG_CUDA(cudaMemcpyAsync(logk[nl - 1].p, D.m_top.p, D.m_top.bytes(), cudaMemcpyDeviceToDevice, c.stream));
-        for (int l = nl - 2; l >= 0; --l) {
-            logk[l].alloc(lev[l].ne);
-            if (lev[l].structured) coarsen_log(c, lev[l + 1], lev[l], logk[l + 1].p, logk[l].p);
-            else coarsen_log_children(c, lev[l + 1], lev[l], logk[l + 1].p, logk[l].p);
+        if (level == nl - 1) {
+            D.Klev[level].alloc(lev[level].ne);
+            exp_elements(c, D.m_top.p, lev[level].ne, D.Klev[level].p);
+            D.Kvalid[level] = true;
+            return D.Klev[level].p;
         }
-        for (int l = 0; l < nl; ++l) {
+        // the coarse levels together: log K as the children's mean, from the top
+        // down, in the levels' own buffers, then exp in place (no buffers of
+        // their own, allocated and freed with a wait on every new coefficient)
+        for (int l = nl - 2; l >= 0; --l) {
             D.Klev[l].alloc(lev[l].ne);
-            exp_elements(c, logk[l].p, lev[l].ne, D.Klev[l].p);
+            const double *fine = l == nl - 2 ? D.m_top.p : D.Klev[l + 1].p;
+            if (lev[l].structured) coarsen_log(c, lev[l + 1], lev[l], fine, D.Klev[l].p);
+            else coarsen_log_children(c, lev[l + 1], lev[l], fine, D.Klev[l].p);
+        }
+        for (int l = 0; l < nl - 1; ++l) {
+            exp_elements(c, D.Klev[l].p, lev[l].ne, D.Klev[l].p);
             D.Kvalid[l] = true;
         }
-        UG_CUDA(cudaStreamSynchronize(c.stream));
         return D.Klev[level].p;
     }
     D.Klev[level].alloc(lev[level].ne);
