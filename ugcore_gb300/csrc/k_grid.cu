@@ -532,16 +532,16 @@ __global__ void k_dia_used(const int *__restrict__ rowptr, const int *__restrict
 
 // CRS -> diagonals.  Bound by memory: 8 bytes read and sizeof(T) written per
 // entry.  A block takes kFillRows rows; their values, one contiguous range of
-// the CRS, are staged in shared memory by consecutive threads, then each
-// thread writes its row's entries, consecutive threads on consecutive values
+// the CRS, are staged in shared memory by consecutive threads, then four
+// threads write each row's entries, consecutive threads on consecutive values
 // of a diagonal.  A row that holds as many (increasing) columns as there are
 // offsets holds exactly those, in order, so its columns are not read; other
 // rows look theirs up.  129^3 hexes, FP64: one row per thread straight from
 // the CRS took 930 us, every entry's sector fetched by strided threads.
-constexpr int kFillRows = 128, kFillMax = 27;
+constexpr int kFillRows = 64, kFillParts = 4, kFillThreads = kFillRows * kFillParts, kFillMax = 27;
 
 template <class T>
-__global__ void __launch_bounds__(kFillRows) k_dia_fill(const int *__restrict__ rowptr, const int *__restrict__ col,
+__global__ void __launch_bounds__(kFillThreads) k_dia_fill(const int *__restrict__ rowptr, const int *__restrict__ col,
                                                         const double *__restrict__ val, int nrows, int ld, DiaMap m,
                                                         bool sorted, const double *__restrict__ col_scale,
                                                         T *__restrict__ dval, int *__restrict__ left_out)
@@ -552,14 +552,14 @@ __global__ void __launch_bounds__(kFillRows) k_dia_fill(const int *__restrict__ 
     const int q0 = rowptr[r0], q1 = rowptr[r1];
     const bool staged = q1 - q0 <= kFillRows * kFillMax;
     if (staged)
-        for (int q = q0 + threadIdx.x; q < q1; q += kFillRows) {
+        for (int q = q0 + threadIdx.x; q < q1; q += kFillThreads) {
             // asynchronous: all of a thread's copies are in flight together
             const unsigned d = (unsigned)__cvta_generic_to_shared(sv + (q - q0));
             asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(d), "l"(val + q) : "memory");
         }
     asm volatile("cp.async.wait_all;" ::: "memory");
     __syncthreads();
-    const int r = r0 + threadIdx.x;
+    const int r = r0 + (int)threadIdx.x % kFillRows, part = threadIdx.x / kFillRows;
     if (r >= nrows) return;
     const int a0 = rowptr[r], len = rowptr[r + 1] - a0;
     bool bad = false;
@@ -577,19 +577,20 @@ __global__ void __launch_bounds__(kFillRows) k_dia_fill(const int *__restrict__ 
     };
     if (sorted && len == m.n) {
 #pragma unroll 3
-        for (int k = 0; k < len; ++k) put(k, r + m.off[k], staged ? sv[a0 - q0 + k] : val[a0 + k]);
+        for (int k = part; k < len; k += kFillParts) put(k, r + m.off[k], staged ? sv[a0 - q0 + k] : val[a0 + k]);
     } else {
         // a few columns' loads in flight at a time: one after the other, these
         // rows (two in 129 on a structured level) held up their blocks
         constexpr int B = 9;
+        const int e0 = a0 + part * len / kFillParts, e1 = a0 + (part + 1) * len / kFillParts;
         int k = 0;
-        for (int a = a0; a < a0 + len; a += B) {
+        for (int a = e0; a < e1; a += B) {
             int c[B];
 #pragma unroll
-            for (int q = 0; q < B; ++q) c[q] = a + q < a0 + len ? __ldg(col + a + q) : 0;
+            for (int q = 0; q < B; ++q) c[q] = a + q < e1 ? __ldg(col + a + q) : 0;
 #pragma unroll
             for (int q = 0; q < B; ++q)
-                if (a + q < a0 + len) {
+                if (a + q < e1) {
                     if (!sorted) k = 0;
                     while (k < m.n && m.off[k] != c[q] - r) ++k;
                     if (k < m.n) put(k, c[q], staged ? sv[a + q - q0] : val[a + q]);   // m holds every offset of A
@@ -627,7 +628,7 @@ static void dia_from_csr(Ctx &c, const Csr &A, Dia<T> &D, const OpLayout &lay, c
         }
         if (values_changed) c.dia_flag_pending = true;
     }
-    UG_LAUNCH_PDL(c, k_dia_fill<T>, div_up(A.nrows, kFillRows), kFillRows, 0, A.rowptr.p, A.col.p, A.val.p, A.nrows,
+    UG_LAUNCH_PDL(c, k_dia_fill<T>, div_up(A.nrows, kFillRows), kFillThreads, 0, A.rowptr.p, A.col.p, A.val.p, A.nrows,
                   D.ld, dia_map(lay), lay.sorted, col_scale, D.vals(), c.dia_flag.p);
 }
 
