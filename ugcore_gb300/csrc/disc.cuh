@@ -35,6 +35,10 @@ struct AsmArgs {
     double k_value = 0.0;
     double sm0 = 0.0, sa0 = 1.0, sm1 = 0.0, sa1 = 0.0;
     const double *u_old = nullptr;
+    // row-wise time-discrete assembly: the class matrices hold sa0 A already, and
+    // the factor of A u_old in the right-hand side is sa1_row (sa1 or sa1 / sa0)
+    int scaled = 0;
+    double sa1_row = 0.0;
     // defect assembly (launch_defect): d += per-element defect of u
     const double *u = nullptr;
     double *d = nullptr;

@@ -415,7 +415,7 @@ __device__ __forceinline__ double row_rhs(const AsmArgs &a, const double (&acc)[
     double v = a.sa0 != 0.0 ? a.sa0 * fv : 0.0;
     v -= a.sm1 * (volsum * a.u_old[r]);
     if (a.sa1 != 0.0) {
-        v -= a.sa1 * row_product<T>(acc, a.u_old, r, a.cx + 1, a.cy + 1);
+        v -= a.sa1_row * row_product<T>(acc, a.u_old, r, a.cx + 1, a.cy + 1);
         v += a.sa1 * fv;
     }
     return v;
@@ -426,8 +426,10 @@ template <int T>
 __device__ __forceinline__ void row_in_time(const AsmArgs &a, double (&acc)[Stencil<T>::N], double volsum)
 {
     using S = Stencil<T>;
+    if (!a.scaled) {
 #pragma unroll
-    for (int s = 0; s < S::N; ++s) acc[s] *= a.sa0;
+        for (int s = 0; s < S::N; ++s) acc[s] *= a.sa0;
+    }
     acc[S::slot(0, 0, 0)] += a.sm0 * volsum;
 }
 
@@ -979,8 +981,18 @@ bool launch_assemble_rows(Ctx &c, const Level &L, const AsmArgs &a_in, RowAsmCac
         if (cache.row_check < 0 || (a.inst && !cache.all_dirichlet)) return false;
         const double *flux;
         if (!class_fluxes<T>(c, a, cache, flux)) return false;
-        if (a.inst) run_assemble_rows<T, true>(c, L, a, cd, flux, cache);
-        else run_assemble_rows<T, false>(c, L, a, cd, flux, cache);
+        if (a.inst) {
+            // sa0 into the class matrices where there are no fluxes beside them:
+            // one FP64 product less per entry
+            AsmArgs at = a;
+            at.scaled = (!flux && a.sa0 != 0.0) ? 1 : 0;
+            at.sa1_row = at.scaled ? a.sa1 / a.sa0 : a.sa1;
+            if (at.scaled)
+                for (double *p = &cd.A[0][0][0], *e = p + sizeof(cd.A) / sizeof(double); p < e; ++p) *p *= a.sa0;
+            run_assemble_rows<T, true>(c, L, at, cd, flux, cache);
+        } else {
+            run_assemble_rows<T, false>(c, L, a, cd, flux, cache);
+        }
         return true;
     });
 }

@@ -799,8 +799,10 @@ void mcgs_colour(Ctx &c, const OpMat<V> &A, const int *rows, int nrows_c, const 
 // The operator entries of the first colour are loaded before the launch wait.
 // 97^3 hexes, FP32: eight launches of one colour each, with a pass that zeroed
 // t, 54 us a sweep.
+// Three blocks per SM: a wave then holds the whole level (461 us against 515 for
+// the cycle; four blocks, 64 registers, spill: 551).
 template <class V, int S>
-__global__ void __launch_bounds__(NT) k_mcgs_lines(DiaMV<V, S> A, int nx, int ny, int b1, int b2, int nly, int nlines,
+__global__ void __launch_bounds__(NT, sizeof(V) == 4 ? 3 : 1) k_mcgs_lines(DiaMV<V, S> A, int nx, int ny, int b1, int b2, int nly, int nlines,
                                                    int nz, int per, int per_block, int first, unsigned mask_even,
                                                    unsigned mask_odd, GsLines gs, bool from_zero,
                                                    const V *__restrict__ dr,
