@@ -401,7 +401,7 @@ struct GmgT : GmgBase {
             mix(L.ilu.val.p); mix(L.ilu.col.p); mix(L.ilu.rowptr.p); mix(L.ilu.nlow.p); mix(L.ilu.uinv.p);
             h ^= (uint64_t)L.n;
             for (int k = 0; k < L.At.dia.S; ++k) mix((const void *)(intptr_t)L.At.dia.off.o[k]);
-            mix((const void *)(intptr_t)((L.gs.usable ? 1 : 0) + (L.level2d ? 2 : 0)));
+            mix((const void *)(intptr_t)((L.gs.usable ? 1 : 0) + (L.level2d ? 2 : 0) + (L.level3d ? 4 : 0)));
         }
         mix(Ainv.p);
         mix(z64.p);
@@ -727,9 +727,14 @@ struct GmgT : GmgBase {
             level2d_pre<V>(c, L.At, L.gp, L.dinv.p, cur, L.sc.p, L.dB.p, C.dA.p, skip);
             cur = L.dB.p;
         }
+        const bool pre3d = L.level3d && l < T && nu1 == 2 && first;
+        if (pre3d) {
+            level3d_pre<V>(c, L.At, L.gp, L.dinv.p, cur, L.sc.p, L.dB.p, skip);
+            cur = L.dB.p;
+        }
         // ---- pre-smoothing
         if (nu1 == 0 && first) UG_LAUNCH_PDL(c, k_zero<V>, div_up(L.n, 256), 256, 0, L.n, L.sc.p, skip);
-        for (int k = 0; k < nu1 && !pre2d; ++k) {
+        for (int k = 0; k < nu1 && !pre2d && !pre3d; ++k) {
             V *out = (cur == L.dA.p) ? L.dB.p : L.dA.p;
             int mode = (k == 0) ? (first ? SC_SET_FROM_BASE : SC_ADD_FROM_BASE) : SC_ADD_FROM_BASE;
             // two steps in one pass over the operator where the level allows it
@@ -778,6 +783,11 @@ struct GmgT : GmgBase {
             level2d_post<V>(c, L.At, L.gp, L.dinv.p, L.dfac.p, C.sc.p, dpre, L.sc.p, skip, top_level ? r_rho : nullptr,
                             top_level ? red : nullptr, rho_kind, top_level ? z64.p : nullptr);
             if (top_level) rho_done = (r_rho != nullptr);
+            L.dcur = const_cast<V *>(dpre);   // read by no later visit
+            return;
+        }
+        if (L.level3d && l < T && nu2 == 2 && cycle == 1) {
+            level3d_post<V>(c, L.At, L.gp, L.dinv.p, L.dfac.p, C.sc.p, dpre, L.sc.p, skip);
             L.dcur = const_cast<V *>(dpre);   // read by no later visit
             return;
         }
@@ -1026,10 +1036,12 @@ static GmgBase *build_gmg(ug4gb_gmg *m, const ug4gb_matrix *A_top, GmgT<V> *reus
         const uint64_t key = (g->uid << 6) + (uint64_t)(l + 1), have = A_top->pattern_key();
         const bool own = l < nl - 1 || have == key || have == (key | (1ULL << 63));
         L.gs = GsLines();
-        L.level2d = false;
+        L.level2d = L.level3d = false;
         if (!own || l == m->base || !L.grid_transfer || L.At.kind != 1) continue;
-        if (m->smoother == UG4GB_SMOOTHER_JACOBI)
+        if (m->smoother == UG4GB_SMOOTHER_JACOBI) {
             L.level2d = m->smoother2 == UG4GB_SMOOTHER_JACOBI && level2d_ok<V>(L.At, L.gp);
+            L.level3d = m->smoother2 == UG4GB_SMOOTHER_JACOBI && !L.sweep2 && level3d_ok<V>(L.At, L.gp);
+        }
         else if (L.At_lay.known)
             L.gs = gs_lines(L.At.dia.off, L.At.dia.S, L.At_lay.all, L.gp);
     }

@@ -120,6 +120,7 @@ struct GLevel {
     std::vector<DevBuf<int>> crow;   // MCGS / ILU colour row lists
     std::vector<int> ncrow;
     bool level2d = false;            // smoothing and transfers in two launches (k_level2d.cu)
+    bool level3d = false;            // smoothing in two launches, with the prolongation (k_level3d.cu)
     GsLines gs;                      // colour sweeps line by line (structured levels)
     DevBuf<int> vcolor;              // unstructured levels: colours of the operator's own graph
     IluFactors<V> ilu;               // ILU smoother factors

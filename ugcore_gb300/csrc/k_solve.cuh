@@ -308,6 +308,26 @@ template <class V>
 void level2d_post(Ctx &c, const OpMat<V> &At, const GridPair &gp, const V *dinv, const V *dfac, const V *scc,
                   const V *d, V *sc, const int *skip, const double *r_rho, RedArgs *red, int rho_kind, double *z64);
 
+// ---- a small 3D level of the V-cycle with its smoothing in two launches (k_level3d.cu) ----
+// FP32 levels of up to this many vertices: above, the repeated vertices of the
+// tiles (2.8 times the first step) cost more than the launches they save (49^3
+// beside 25^3: 97^3 time step 2262 -> 2296 us; 49 x 33 x 33 beside 25 x 17 x 17:
+// 97 x 65 x 65 gradient 15.19 -> 15.13 ms).  FP64 lost at every size (129^3 solve
+// 6805 -> 6843 us with 17^3, 7005 with 33^3), and the seven-point levels of
+// tetrahedra gained less than 1 %.
+constexpr int kLevel3dRows = 60000;
+// At holds the 27-point stencil of the structured 3D level gp
+template <class V>
+bool level3d_ok(const OpMat<V> &At, const GridPair &gp);
+// as level2d_pre without the restriction
+template <class V>
+void level3d_pre(Ctx &c, const OpMat<V> &At, const GridPair &gp, const V *dinv, const V *d, V *sc, V *dout,
+                 const int *skip);
+// as level2d_post, below the top level
+template <class V>
+void level3d_post(Ctx &c, const OpMat<V> &At, const GridPair &gp, const V *dinv, const V *dfac, const V *scc,
+                  const V *d, V *sc, const int *skip);
+
 // Multicolour Gauss-Seidel sweeps of a structured level line by line
 // (k_mcgs_lines): per colour (parity bits of the vertex), which diagonals lead
 // to vertices of lower colours, of higher ones, and which are entries at all.
