@@ -568,9 +568,12 @@ struct GmgT : GmgBase {
         if (n <= kDeviceLuMax) {
             const bool xs = n <= kLuSharedX;
             const size_t smem = (size_t)n * n * sizeof(double) * (xs ? 2 : 1);
-            if (smem > 48 * 1024)
+            // 48 KB hold the kernel's own arrays as well; beyond, the most that any
+            // base asks for, as another thread may launch with less or more
+            constexpr size_t most = sizeof(double) * std::max(2 * kLuSharedX * kLuSharedX, kDeviceLuMax * kDeviceLuMax);
+            if (smem + sizeof(unsigned) * kDeviceLuMax * kLuWords > 48 * 1024)
                 UG_CUDA(cudaFuncSetAttribute(xs ? k_base_lu<true> : k_base_lu<false>,
-                                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+                                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most));
             Ainv.alloc((size_t)n * n);
             lu_status.alloc(1);
             if (xs)

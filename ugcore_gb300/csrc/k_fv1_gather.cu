@@ -285,9 +285,11 @@ bool assemble_gather(Ctx &c, const Level &L, const AsmArgs &a, GatherCache &g)
         g.smem = sizeof(double) * (size_t)h;   // at most 64 x 256 values, 128 KB
         g.ready = true;
     }
+    // (the most that any level asks for, as another thread may launch with less or more)
     if (g.smem > 48 * 1024)
         UG_CUDA(cudaFuncSetAttribute(a.inst ? k_gather_rows<K, true> : k_gather_rows<K, false>,
-                                     cudaFuncAttributeMaxDynamicSharedMemorySize, (int)g.smem));
+                                     cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)sizeof(double) * kGatherRows * 256));
     g.ws.alloc((size_t)L.ne * S::WS);
     UG_LAUNCH(c, k_simplex_terms<K>, div_up(L.ne, 256), 256, 0, L.coords.p, L.elems.p, L.ne, a.K, g.ws.p);
     const unsigned blocks = div_up(L.nv, kGatherRows);
