@@ -1047,13 +1047,16 @@ static GmgBase *build_gmg(ug4gb_gmg *m, const ug4gb_matrix *A_top, GmgT<V> *reus
             op_from_csr_cached<V>(c, L.A, L.At, m->smoother == UG4GB_SMOOTHER_JACOBI ? L.dinv64.p : nullptr,
                                   c.allow_dia, L.At_lay);
         }
-    // Gauss-Seidel sweeps by lines, 2D levels in two launches: structured levels whose operator has the
-    // level's element pattern (or R A P of it); a user's top operator may couple
-    // vertices across the ends of grid lines
+    // Gauss-Seidel sweeps by lines, 2D and small 3D levels in two launches take a
+    // vertex outside the grid as absent: structured levels whose operator has the
+    // level's element pattern, or is R A P of one that has it.  A user's top
+    // operator may couple vertices across the grid, and then its Galerkin levels
+    // do too (a boundary vertex's rows of R and P have the weight 1 alone).
+    const uint64_t top_pattern = (g->uid << 6) + (uint64_t)nl, have = A_top->pattern_key();
+    const bool own_top = have == top_pattern || have == (top_pattern | (1ULL << 63));
     for (int l = m->base; l < nl; ++l) {
         GLevel<V> &L = G->lev[l];
-        const uint64_t key = (g->uid << 6) + (uint64_t)(l + 1), have = A_top->pattern_key();
-        const bool own = l < nl - 1 || have == key || have == (key | (1ULL << 63));
+        const bool own = own_top || (l < nl - 1 && !m->rap);
         L.gs = GsLines();
         L.level2d = L.level3d = false;
         if (!own || l == m->base || !L.grid_transfer || L.At.kind != 1) continue;
