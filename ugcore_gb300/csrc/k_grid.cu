@@ -582,7 +582,10 @@ __global__ void __launch_bounds__(kFillThreads) k_dia_fill(const int *__restrict
         // a few columns' loads in flight at a time: one after the other, these
         // rows (two in 129 on a structured level) held up their blocks
         constexpr int B = 9;
-        const int e0 = a0 + part * len / kFillParts, e1 = a0 + (part + 1) * len / kFillParts;
+        // rows in any column order: one thread each, so that of a column named
+        // twice the last value stays
+        const int e0 = sorted ? a0 + part * len / kFillParts : a0;
+        const int e1 = sorted ? a0 + (part + 1) * len / kFillParts : (part == 0 ? a0 + len : a0);
         int k = 0;
         for (int a = e0; a < e1; a += B) {
             int c[B];
