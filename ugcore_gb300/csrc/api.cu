@@ -439,7 +439,7 @@ int ug4gb_matrix_set_csr(ug4gb_matrix *m, int nrows, int ncols, int64_t nnz, con
         copy_in(c, m->A.col.p, col, sizeof(int) * (size_t)nnz);
         copy_in(c, m->A.val.p, val, sizeof(double) * (size_t)nnz);
         UG_CUDA(cudaStreamSynchronize(c.stream));
-        m->op_valid = false;
+        m->values_changed();
         m->pattern_grid = 0;
         m->derived_key = 0;
         m->pattern_level = -1;
@@ -497,7 +497,7 @@ int ug4gb_matrix_set_as_transpose_of(ug4gb_matrix *T, const ug4gb_matrix *B, int
     return guarded(T->ctx, [&] {
         csr_transpose(T->ctx->c, B->A, T->A, keep_zeros != 0);
         UG_CUDA(cudaStreamSynchronize(T->ctx->c.stream));
-        T->op_valid = false;
+        T->values_changed();
         T->pattern_grid = 0;
         T->derived_key = 0;
         T->pattern_level = -1;

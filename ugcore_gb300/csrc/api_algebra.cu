@@ -143,7 +143,7 @@ int ug4gb_matrix_resize_and_clear(ug4gb_matrix *A, int num_rows, int num_cols)
         A->A.val.alloc(1);
         UG_CUDA(cudaMemsetAsync(A->A.rowptr.p, 0, sizeof(int) * (size_t)(num_rows + 1), c.stream));
         UG_CUDA(cudaStreamSynchronize(c.stream));
-        A->op_valid = false;
+        A->values_changed();
         A->pattern_grid = 0;
         A->derived_key = 0;
         A->pattern_level = -1;
@@ -157,7 +157,7 @@ int ug4gb_matrix_clear_retain_structure(ug4gb_matrix *A)
         Ctx &c = A->ctx->c;
         if (A->A.nnz) UG_CUDA(cudaMemsetAsync(A->A.val.p, 0, sizeof(double) * (size_t)A->A.nnz, c.stream));
         UG_CUDA(cudaStreamSynchronize(c.stream));
-        A->op_valid = false;
+        A->values_changed();
     });
 }
 
@@ -182,7 +182,7 @@ int ug4gb_matrix_set_as_copy_of(ug4gb_matrix *A, const ug4gb_matrix *B, double s
             UG_LAUNCH(c, k_copy_scaled, div_up(S.nnz, 256), 256, 0, S.val.p, A->A.val.p, S.nnz, scale);
         }
         UG_CUDA(cudaStreamSynchronize(c.stream));
-        A->op_valid = false;
+        A->values_changed();
         A->pattern_grid = B->pattern_grid;
         A->pattern_level = B->pattern_level;
         A->derived_key = B->derived_key;
@@ -196,7 +196,7 @@ int ug4gb_matrix_scale(ug4gb_matrix *A, double alpha)
         Ctx &c = A->ctx->c;
         if (A->A.nnz) UG_LAUNCH(c, k_scale, div_up(A->A.nnz, 256), 256, 0, A->A.val.p, A->A.nnz, alpha);
         UG_CUDA(cudaStreamSynchronize(c.stream));
-        A->op_valid = false;
+        A->values_changed();
     });
 }
 
@@ -247,7 +247,7 @@ int ug4gb_matrix_add_entries(ug4gb_matrix *A, int n, const int *rows, const int 
         UG_LAUNCH(c, k_add_entries, div_up(n, 256), 256, 0, A->A.rowptr.p, A->A.col.p, A->A.val.p, A->A.nrows,
                   A->A.ncols, n, r.p, cc.p, v.p, err.p);
         check_err(c, err, "add_entries: an entry outside the matrix pattern");
-        A->op_valid = false;
+        A->values_changed();
     });
 }
 

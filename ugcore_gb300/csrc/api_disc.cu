@@ -72,7 +72,7 @@ void disc_assemble(ug4gb_disc *d, int level, ug4gb_matrix *A, double *b, const T
         A->pattern_grid = d->g->uid;
         A->pattern_level = level;
     }
-    A->op_valid = false;
+    A->values_changed();
     DiscImpl &D = d->d;
     bool top = (level == (int)d->g->lev.size() - 1);
     AsmArgs a;
@@ -106,7 +106,13 @@ void disc_assemble(ug4gb_disc *d, int level, ug4gb_matrix *A, double *b, const T
         a.u_old = ts->u_old;
     }
     // structured levels: row by row, every value written once
-    if (c.row_assembly && launch_assemble_rows(c, L, a, class_cache(d, level))) return;
+    if (c.row_assembly && launch_assemble_rows(c, L, a, class_cache(d, level))) {
+        // Kuhn tetrahedra: the diffusion couples along the grid axes only, every
+        // other entry of a row was written as an exact 0 (gather_row)
+        if (L.elem_type == UG4GB_TET && a.vmodes == 0 && class_cache(d, level).all_dirichlet)
+            A->axis = AxisOnly{L.nx, L.nx * L.ny};
+        return;
+    }
     // unstructured simplices: row by row from the elements around a vertex
     if (D.gather.size() < d->g->lev.size()) D.gather.resize(d->g->lev.size());
     if (c.row_assembly && launch_assemble_gather(c, L, a, D.gather[level])) return;
@@ -478,7 +484,7 @@ int ug4gb_disc_adjoint_operator(ug4gb_disc *d, int level, const ug4gb_matrix *A,
             }
             csr_transpose_symmetric_inplace(c, M->A);
             launch_dirichlet(c, d->g->lev[level], M->A, nullptr);
-            M->op_valid = false;
+            M->op_valid = false;   // (the offsets of its zeros are symmetric)
         });
     }
     return guarded(d->ctx, [&] {
@@ -494,7 +500,8 @@ int ug4gb_disc_adjoint_operator(ug4gb_disc *d, int level, const ug4gb_matrix *A,
             AT->tperm_key = src;
         }
         launch_dirichlet(c, d->g->lev[level], AT->A, nullptr);
-        AT->op_valid = false;
+        AT->values_changed();
+        AT->axis = A->axis;   // (the offsets of its zeros are symmetric)
         AT->pattern_grid = 0;
         AT->pattern_level = -1;
         AT->derived_key = key;

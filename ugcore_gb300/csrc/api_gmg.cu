@@ -429,7 +429,8 @@ struct GmgT : GmgBase {
 
     // reuse: the same structure as the previous set-up of this level (its
     // pattern, layout, colours): only values are refreshed, in place
-    void setup_level(Ctx &c, GLevel<V> &L, const Level &G, int l, double damp, bool is_base, bool reuse)
+    void setup_level(Ctx &c, GLevel<V> &L, const Level &G, int l, double damp, bool is_base, bool reuse,
+                     const AxisOnly &axis)
     {
         int n = L.A.nrows;
         L.n = n;
@@ -453,9 +454,9 @@ struct GmgT : GmgBase {
                       smoother2, L.dinv2_64.p, (double *)nullptr, L.dinv2.p, (V *)nullptr);
         }
         if (smoother == UG4GB_SMOOTHER_JACOBI) {
-            op_from_csr_cached<V>(c, L.A, L.At, L.dinv64.p, c.allow_dia, L.At_lay);
+            op_from_csr_cached<V>(c, L.A, L.At, L.dinv64.p, c.allow_dia, L.At_lay, axis);
         } else {
-            op_from_csr_cached<V>(c, L.A, L.At, nullptr, c.allow_dia, L.At_lay);
+            op_from_csr_cached<V>(c, L.A, L.At, nullptr, c.allow_dia, L.At_lay, axis);
             L.t.alloc(n);
             // colours with no coupling inside a colour: parity on structured
             // levels (valid for their stencils and for R A P of them); on
@@ -988,6 +989,7 @@ static GmgBase *build_gmg(ug4gb_gmg *m, const ug4gb_matrix *A_top, GmgT<V> *reus
             const bool same = keep_transfers && L.asm_ok &&
                               (l != nl - 1 || (A_top->pattern_key() && A_top->pattern_key() == G->top_key));
             Csr &dst = L.A;
+            AxisOnly axis = A_top->axis;
             // level operator: copy of the surface operator on the top level,
             // re-assembled on coarser levels (assemble_level_operator, :528-750)
             if (l == nl - 1) {
@@ -1009,10 +1011,12 @@ static GmgBase *build_gmg(ug4gb_gmg *m, const ug4gb_matrix *A_top, GmgT<V> *reus
                 if (m->td) ts = m->td->jacobian_scale();
                 disc_assemble(m->disc, l, &tmp, nullptr, m->td ? &ts : nullptr);
                 dst = std::move(tmp.A);
+                axis = tmp.axis;
             }
             if (m->transposed) transpose_level(l, same);
             L.asm_ok = true;
-            G->setup_level(c, L, g->lev[l], l, m->damp, l == m->base && m->base_kind == UG4GB_BASE_LU, same);
+            G->setup_level(c, L, g->lev[l], l, m->damp, l == m->base && m->base_kind == UG4GB_BASE_LU, same,
+                           axis);
             if (l > m->base) {
                 if (!keep_transfers) G->setup_transfers(c, L, g->lev[l], g->lev[l - 1], m->damp_prol, m->damp_res);
                 if (L.grid_transfer && m->smoother == UG4GB_SMOOTHER_JACOBI)
@@ -1031,7 +1035,8 @@ static GmgBase *build_gmg(ug4gb_gmg *m, const ug4gb_matrix *A_top, GmgT<V> *reus
         }
         for (int l = m->base; l < nl; ++l) {
             GLevel<V> &L = G->lev[l];
-            G->setup_level(c, L, g->lev[l], l, m->damp, l == m->base && m->base_kind == UG4GB_BASE_LU, false);
+            G->setup_level(c, L, g->lev[l], l, m->damp, l == m->base && m->base_kind == UG4GB_BASE_LU, false,
+                           AxisOnly());
             if (l > m->base && L.grid_transfer && m->smoother == UG4GB_SMOOTHER_JACOBI)
                 L.sweep2 = sweep2_prepare<V>(c, L.At, L.gp);
         }

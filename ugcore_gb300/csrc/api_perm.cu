@@ -264,7 +264,7 @@ int ug4gb_perm_matrix(ug4gb_perm *p, int to_external, const ug4gb_matrix *A, ug4
             mm.key = src;
             mm.nnz = nnz;
         }
-        B->op_valid = false;
+        B->values_changed();
         B->pattern_grid = 0;
         B->pattern_level = -1;
         B->derived_key = key;

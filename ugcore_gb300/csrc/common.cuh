@@ -512,6 +512,8 @@ bool csr_offsets(Ctx &c, const Csr &A, int max_s, std::vector<int> &offs);
 // when it was built.  A refill tests their entries again and reports a
 // nonzero one through a device flag: the caller asks dia_left_out() before
 // the operator is used and, if it is set, builds the layout with keep_all.
+// That takes a wait, so the test is left out where the assembly that wrote the
+// values vouches for the zeros (AxisOnly).
 struct OpLayout {
     bool known = false;
     int kind = 0;                 // 0 SELL-32, 1 diagonal
@@ -523,13 +525,26 @@ struct OpLayout {
     bool left_out = false;        // offs misses some of `all`
     bool keep_all = false;        // leave no offset out
 };
+// A structured level's values whose entries off the offsets 0, +-1, +-nx and
+// +-nxy (nx: vertices of a grid line, nxy: of a plane) are exact zeros; nx == 0:
+// not known
+struct AxisOnly {
+    int nx = 0, nxy = 0;
+    bool zero_at(int off) const
+    {
+        const int o = off < 0 ? -off : off;
+        return nx > 0 && o > 1 && o != nx && o != nxy;
+    }
+};
 // solve format: diagonal when A is square with <= 27 offsets and allow_dia, else SELL-32
 template <class T>
 void op_from_csr(Ctx &c, const Csr &A, OpMat<T> &M, const double *col_scale, bool allow_dia);
 template <class T>
-void op_from_csr_cached(Ctx &c, const Csr &A, OpMat<T> &M, const double *col_scale, bool allow_dia, OpLayout &lay);
+void op_from_csr_cached(Ctx &c, const Csr &A, OpMat<T> &M, const double *col_scale, bool allow_dia, OpLayout &lay,
+                        const AxisOnly &axis = AxisOnly());
 // whether a refill since the last call met a nonzero entry at an offset its
-// layout leaves out (waits for the stream only if such a layout was refilled)
+// layout leaves out (waits for the stream only if such a layout was refilled
+// with values that nothing vouches for)
 bool dia_left_out(Ctx &c);
 // T = A^T (structural zeros kept) and perm[k] = position in A of the entry
 // that lands at position k of T; transpose_values refills T's values from

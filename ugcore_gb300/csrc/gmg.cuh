@@ -42,6 +42,7 @@ struct ug4gb_matrix {
     ug4gb::Csr A;
     ug4gb::OpMat<double> op;              // solve format of A (SELL-32 or diagonal)
     bool op_valid = false;
+    ug4gb::AxisOnly axis;                 // what the assembly that wrote the values vouches for
     uint64_t pattern_grid = 0;            // uid of the grid (and the level) whose element pattern A holds
     int pattern_level = -1;
     // the transposed element pattern of a level (the adjoint operator), else 0
@@ -61,12 +62,18 @@ struct ug4gb_matrix {
         if (pattern_grid) return (pattern_grid << 6) + (uint64_t)(pattern_level + 1);
         return derived_key;
     }
+    // every call that writes values (or a pattern) says so here
+    void values_changed()
+    {
+        op_valid = false;
+        axis = ug4gb::AxisOnly();
+    }
     void ensure_op()
     {
         if (!op_valid) {
             const uint64_t key = pattern_key();
             if (!key || key != op_key) op_layout = ug4gb::OpLayout();
-            ug4gb::op_from_csr_cached<double>(ctx->c, A, op, nullptr, ctx->c.allow_dia, op_layout);
+            ug4gb::op_from_csr_cached<double>(ctx->c, A, op, nullptr, ctx->c.allow_dia, op_layout, axis);
             if (ug4gb::dia_left_out(ctx->c)) {
                 op_layout = ug4gb::OpLayout();
                 op_layout.keep_all = true;

@@ -600,16 +600,16 @@ __global__ void __launch_bounds__(kFillThreads) k_dia_fill(const int *__restrict
                 }
         }
     }
-    if (bad) *left_out = 1;
+    if (bad && left_out) *left_out = 1;
 }
 
 // refill: D already holds this pattern's layout (the same offsets, the same
 // CSR pattern): only the pattern's positions are rewritten, the zeros of the
-// absent entries, the padding rows and the guards are kept.  values_changed:
-// not the values the layout's offsets were chosen by (dia_left_out)
+// absent entries, the padding rows and the guards are kept.  test_zeros: entries
+// at the offsets that the layout leaves out may not be zero (dia_left_out)
 template <class T>
 static void dia_from_csr(Ctx &c, const Csr &A, Dia<T> &D, const OpLayout &lay, const double *col_scale, bool refill,
-                         bool values_changed)
+                         bool test_zeros)
 {
     const std::vector<int> &offs = lay.offs;
     UG_REQUIRE((int)offs.size() <= kMaxDiag && (int)lay.all.size() <= kMaxDiag, UG4GB_ERR_INVALID,
@@ -624,15 +624,15 @@ static void dia_from_csr(Ctx &c, const Csr &A, Dia<T> &D, const OpLayout &lay, c
     D.val.alloc((size_t)D.S * D.ld + 2 * Dia<T>::kGuard);
     // absent entries, the padding rows and the guards stay 0
     if (!refill) UG_CUDA(cudaMemsetAsync(D.val.p, 0, D.val.bytes(), c.stream));
-    if (lay.left_out) {
+    if (test_zeros) {
         if (!c.dia_flag.p) {
             c.dia_flag.alloc(1);
             UG_CUDA(cudaMemsetAsync(c.dia_flag.p, 0, sizeof(int), c.stream));
         }
-        if (values_changed) c.dia_flag_pending = true;
+        c.dia_flag_pending = true;
     }
     UG_LAUNCH_PDL(c, k_dia_fill<T>, div_up(A.nrows, kFillRows), kFillThreads, 0, A.rowptr.p, A.col.p, A.val.p, A.nrows,
-                  D.ld, dia_map(lay), lay.sorted, col_scale, D.vals(), c.dia_flag.p);
+                  D.ld, dia_map(lay), lay.sorted, col_scale, D.vals(), test_zeros ? c.dia_flag.p : (int *)nullptr);
 }
 
 bool dia_left_out(Ctx &c)
@@ -724,13 +724,17 @@ void op_from_csr(Ctx &c, const Csr &A, OpMat<T> &M, const double *col_scale, boo
 }
 
 template <class T>
-void op_from_csr_cached(Ctx &c, const Csr &A, OpMat<T> &M, const double *col_scale, bool allow_dia, OpLayout &lay)
+void op_from_csr_cached(Ctx &c, const Csr &A, OpMat<T> &M, const double *col_scale, bool allow_dia, OpLayout &lay,
+                        const AxisOnly &axis)
 {
     // the fused sweeps, switched on since, take the whole stencil (choose_offsets)
     const bool widen = lay.left_out && sizeof(T) == 4 && (c.sweep_fusion & 1);
     if (lay.known && lay.nrows == A.nrows && lay.nnz == A.nnz && (lay.kind == 0 || allow_dia) && !widen) {
         if (lay.kind == 1) {
-            dia_from_csr<T>(c, A, M.dia, lay, col_scale, M.kind == 1, true);
+            bool test = false;   // some offset that is left out may hold an entry now
+            for (int off : lay.all)
+                test = test || (!std::binary_search(lay.offs.begin(), lay.offs.end(), off) && !axis.zero_at(off));
+            dia_from_csr<T>(c, A, M.dia, lay, col_scale, M.kind == 1, test);
         } else {
             UG_LAUNCH(c, k_sell_fill<T>, div_up((size_t)M.sell.nslices * kSliceH, 256), 256, 0, A.rowptr.p, A.col.p,
                       A.val.p, A.nrows, M.sell.sptr.p, M.sell.swidth.p, col_scale, M.sell.col.p, M.sell.val.p);
@@ -740,8 +744,10 @@ void op_from_csr_cached(Ctx &c, const Csr &A, OpMat<T> &M, const double *col_sca
     op_build<T>(c, A, M, col_scale, allow_dia, lay);
 }
 
-template void op_from_csr_cached<double>(Ctx &, const Csr &, OpMat<double> &, const double *, bool, OpLayout &);
-template void op_from_csr_cached<float>(Ctx &, const Csr &, OpMat<float> &, const double *, bool, OpLayout &);
+template void op_from_csr_cached<double>(Ctx &, const Csr &, OpMat<double> &, const double *, bool, OpLayout &,
+                                         const AxisOnly &);
+template void op_from_csr_cached<float>(Ctx &, const Csr &, OpMat<float> &, const double *, bool, OpLayout &,
+                                        const AxisOnly &);
 
 __global__ void k_iota_val(double *v, int64_t n)
 {
