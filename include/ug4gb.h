@@ -140,6 +140,11 @@ UG4GB_API int ug4gb_set_operator_format(ug4gb_ctx *ctx, int format);
    launches.  Corrections are bit-identical either way.  Applies to
    multigrids set up after the call. */
 #define UG4GB_TUNE_COARSE_LEVELS 6
+/* UG4GB_TUNE_SCRATCH_TEST (0 or 1; default 0): failure test only.  The row-wise
+   assembly of unstructured simplex levels asks for more device memory than
+   there is for its lists and workspace, so that its allocations fail; the
+   levels are then assembled element by element, which needs neither. */
+#define UG4GB_TUNE_SCRATCH_TEST 7
 UG4GB_API int ug4gb_set_tuning(ug4gb_ctx *ctx, int knob, int value);
 /* per-launch CUDA-event timing of every kernel until profile_end, which
    writes "tag|kernel<TAB>launches<TAB>total_ms" lines into buf.  While it is

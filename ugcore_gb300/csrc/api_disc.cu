@@ -115,7 +115,7 @@ void disc_assemble(ug4gb_disc *d, int level, ug4gb_matrix *A, double *b, const T
     }
     // unstructured simplices: row by row from the elements around a vertex
     if (D.gather.size() < d->g->lev.size()) D.gather.resize(d->g->lev.size());
-    if (c.row_assembly && launch_assemble_gather(c, L, a, D.gather[level])) return;
+    if (c.row_assembly && launch_assemble_gather(c, L, a, D.gather[level], D.gather_ws)) return;
     if (!fresh) UG_CUDA(cudaMemsetAsync(A->A.val.p, 0, sizeof(double) * (size_t)A->A.nnz, c.stream));
     if (b) UG_CUDA(cudaMemsetAsync(b, 0, sizeof(double) * (size_t)L.nv, c.stream));
     launch_assemble(c, L, a);

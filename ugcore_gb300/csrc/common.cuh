@@ -132,6 +132,7 @@ struct Ctx {
     DevBuf<int> dia_flag;       // see dia_left_out
     bool dia_flag_pending = false;
     int sweep_wait_test = 0;    // failure test only: bytes no copy delivers (fused sweeps' bounded waits run out)
+    int scratch_test = 0;       // failure test only: the unstructured assembly asks for more memory than there is
     // levels above the base cycled by the one-block coarse kernel (-1: as
     // many as its cost model finds faster than separate launches, 0: none)
     int coarse_levels = -1;

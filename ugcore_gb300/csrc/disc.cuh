@@ -75,15 +75,19 @@ bool launch_grad_logk_rows(Ctx &c, const Level &L, const double *K, const double
 bool launch_grad_source_rows(Ctx &c, const Level &L, const double *lam, double *g, RowAsmCache &cache);
 // Unstructured simplex levels without convection (k_fv1_gather.cu): every
 // value of A and b written once, Dirichlet rows included; false, launching
-// nothing, where it does not apply.  The lists depend on the mesh only.
+// nothing, where it does not apply or the device has no memory left for its
+// lists and workspace.  The lists depend on the mesh only: 32 bytes per
+// tetrahedron (24 per triangle) and 4 per vertex, kept with the discretisation.
+// ws, for the levels in turn: 64 bytes per tetrahedron (32 per triangle) of the
+// largest level that was assembled (element entries, SCV volumes; nothing in it
+// outlives the call).
 struct GatherCache {
     bool ready = false;
     DevBuf<int> vptr;                   // per vertex: its range in adj
     DevBuf<unsigned> adj, slots;        // per vertex and element: 4 * element + corner; corner positions in the row
     size_t smem = 0;                    // shared memory of a block's rows
-    DevBuf<double> ws;                  // per element: off-diagonal entries, SCV volume
 };
-bool launch_assemble_gather(Ctx &c, const Level &L, const AsmArgs &a, GatherCache &g);
+bool launch_assemble_gather(Ctx &c, const Level &L, const AsmArgs &a, GatherCache &g, DevBuf<double> &ws);
 void launch_dirichlet(Ctx &c, const Level &L, Csr &A, double *b);
 // d = defect of a.u on level L (a.d must be zero on entry; Dirichlet rows 0);
 // stationary, or instationary with a.inst and the scalings of AsmArgs

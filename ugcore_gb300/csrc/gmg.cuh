@@ -108,6 +108,7 @@ struct DiscImpl {
     uint64_t f_seed = 0;
     std::vector<RowAsmCache> rows;         // per level: class geometry of the row-wise assembly
     std::vector<GatherCache> gather;       // per level: lists of the unstructured row-wise assembly
+    DevBuf<double> gather_ws;              // and its workspace, one for all levels
 };
 
 template <class V>

@@ -259,18 +259,35 @@ __global__ void __launch_bounds__(256) k_gather_rows(AsmArgs a, int nv, const in
     for (int i = threadIdx.x; i < nq; i += blockDim.x) a.val[q0 + i] = acc[i];
 }
 
+// b with room for n values; false where the device has no memory for them
+template <class T>
+bool reserve(const Ctx &c, DevBuf<T> &b, size_t n)
+{
+    if (b.n >= n && !c.scratch_test) return true;
+    try {
+        b.alloc(c.scratch_test ? (size_t)1 << 48 : n);
+    } catch (const Error &e) {
+        if (e.code != UG4GB_ERR_NOMEM) throw;
+        (void)cudaGetLastError();
+        return false;
+    }
+    return true;
+}
+
 template <int K>
-bool assemble_gather(Ctx &c, const Level &L, const AsmArgs &a, GatherCache &g)
+bool assemble_gather(Ctx &c, const Level &L, const AsmArgs &a, GatherCache &g, DevBuf<double> &ws)
 {
     using S = Simplex<K>;
+    // (the element kernel needs none of this)
+    if (!reserve(c, ws, (size_t)L.ne * S::WS)) return false;
     if (!g.ready) {
         const int nek = L.ne * K;
         DevBuf<int> deg, most;
-        deg.alloc(L.nv + 1);
-        most.alloc(1);
-        g.vptr.alloc(L.nv + 1);
-        g.adj.alloc(nek);
-        g.slots.alloc(nek);
+        if (!reserve(c, deg, L.nv + 1) || !reserve(c, most, 1) || !reserve(c, g.vptr, L.nv + 1) ||
+            !reserve(c, g.adj, nek) || !reserve(c, g.slots, nek)) {
+            g = GatherCache();
+            return false;
+        }
         UG_CUDA(cudaMemsetAsync(deg.p, 0, deg.bytes(), c.stream));
         UG_CUDA(cudaMemsetAsync(most.p, 0, sizeof(int), c.stream));
         UG_LAUNCH(c, k_count_corner, div_up(nek, 256), 256, 0, L.elems.p, nek, deg.p);
@@ -290,25 +307,24 @@ bool assemble_gather(Ctx &c, const Level &L, const AsmArgs &a, GatherCache &g)
         UG_CUDA(cudaFuncSetAttribute(a.inst ? k_gather_rows<K, true> : k_gather_rows<K, false>,
                                      cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)sizeof(double) * kGatherRows * 256));
-    g.ws.alloc((size_t)L.ne * S::WS);
-    UG_LAUNCH(c, k_simplex_terms<K>, div_up(L.ne, 256), 256, 0, L.coords.p, L.elems.p, L.ne, a.K, g.ws.p);
+    UG_LAUNCH(c, k_simplex_terms<K>, div_up(L.ne, 256), 256, 0, L.coords.p, L.elems.p, L.ne, a.K, ws.p);
     const unsigned blocks = div_up(L.nv, kGatherRows);
     if (a.inst)
-        UG_LAUNCH(c, (k_gather_rows<K, true>), blocks, 256, g.smem, a, L.nv, g.vptr.p, g.adj.p, g.slots.p, g.ws.p,
+        UG_LAUNCH(c, (k_gather_rows<K, true>), blocks, 256, g.smem, a, L.nv, g.vptr.p, g.adj.p, g.slots.p, ws.p,
                   L.bnd.p);
     else
-        UG_LAUNCH(c, (k_gather_rows<K, false>), blocks, 256, g.smem, a, L.nv, g.vptr.p, g.adj.p, g.slots.p, g.ws.p,
+        UG_LAUNCH(c, (k_gather_rows<K, false>), blocks, 256, g.smem, a, L.nv, g.vptr.p, g.adj.p, g.slots.p, ws.p,
                   L.bnd.p);
     return true;
 }
 
 }  // namespace
 
-bool launch_assemble_gather(Ctx &c, const Level &L, const AsmArgs &a, GatherCache &g)
+bool launch_assemble_gather(Ctx &c, const Level &L, const AsmArgs &a, GatherCache &g, DevBuf<double> &ws)
 {
     if (L.structured || a.vmodes > 0 || L.ne == 0) return false;
-    if (L.elem_type == UG4GB_TET) return assemble_gather<4>(c, L, a, g);
-    if (L.elem_type == UG4GB_TRI) return assemble_gather<3>(c, L, a, g);
+    if (L.elem_type == UG4GB_TET) return assemble_gather<4>(c, L, a, g, ws);
+    if (L.elem_type == UG4GB_TRI) return assemble_gather<3>(c, L, a, g, ws);
     return false;
 }
 
