@@ -145,6 +145,12 @@ UG4GB_API int ug4gb_set_operator_format(ug4gb_ctx *ctx, int format);
    there is for its lists and workspace, so that its allocations fail; the
    levels are then assembled element by element, which needs neither. */
 #define UG4GB_TUNE_SCRATCH_TEST 7
+/* UG4GB_TUNE_COARSE_BLOCKS (0..16; default 16): the most blocks of the cluster
+   that cycles the coarse end of a V-cycle.  The device is asked for 16, 8, 4, 2
+   and 1 blocks in turn; where it runs none of them (or with 0) every level takes
+   separate launches.  Corrections are bit-identical either way.  Applies to
+   multigrids set up after the call. */
+#define UG4GB_TUNE_COARSE_BLOCKS 8
 UG4GB_API int ug4gb_set_tuning(ug4gb_ctx *ctx, int knob, int value);
 /* per-launch CUDA-event timing of every kernel until profile_end, which
    writes "tag|kernel<TAB>launches<TAB>total_ms" lines into buf.  While it is

@@ -26,6 +26,7 @@ TUNE_ROW_ASSEMBLY = 4
 TUNE_SWEEP_WAIT_TEST = 5
 TUNE_COARSE_LEVELS = 6
 TUNE_SCRATCH_TEST = 7
+TUNE_COARSE_BLOCKS = 8
 
 _ERRNAMES = {ERR_INVALID: "invalid argument", ERR_CUDA: "CUDA error", ERR_NOMEM: "out of device memory",
              ERR_SINGULAR: "singular base matrix", ERR_NOT_CONVERGED: "not converged",

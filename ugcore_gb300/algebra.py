@@ -79,7 +79,7 @@ class Context:
         check(lib().ug4gb_set_operator_format(self.h, {"auto": 0, "sell": 1}[fmt]), self.h)
 
     def set_tuning(self, pdl=None, sweep_fusion=None, sweep_planes=None, row_assembly=None, sweep_wait_test=None,
-                   coarse_levels=None, scratch_test=None):
+                   coarse_levels=None, scratch_test=None, coarse_blocks=None):
         """performance switches:
         pdl: programmatic dependent launch of the solve kernels;
         sweep_fusion: bit mask (1 on, 2 every level size) of the
@@ -93,13 +93,17 @@ class Context:
         0); the same values to rounding;
         coarse_levels: levels above the base that one launch cycles at the
         coarse end of a V-cycle (-1 as many as pay, the default; 0 none;
-        bit-identical corrections; multigrids set up afterwards)."""
+        bit-identical corrections; multigrids set up afterwards);
+        coarse_blocks: the most blocks of the cluster that this launch takes
+        (0 to 16, the default; 0 as coarse_levels 0)."""
         if sweep_wait_test is not None:
             # failure test of the fused sweeps' bounded waits only
             check(lib().ug4gb_set_tuning(self.h, _lib.TUNE_SWEEP_WAIT_TEST, int(sweep_wait_test)), self.h)
         if scratch_test is not None:
             # failure test of the unstructured assembly's allocations only
             check(lib().ug4gb_set_tuning(self.h, _lib.TUNE_SCRATCH_TEST, int(scratch_test)), self.h)
+        if coarse_blocks is not None:
+            check(lib().ug4gb_set_tuning(self.h, _lib.TUNE_COARSE_BLOCKS, int(coarse_blocks)), self.h)
         if row_assembly is not None:
             check(lib().ug4gb_set_tuning(self.h, _lib.TUNE_ROW_ASSEMBLY, int(row_assembly)), self.h)
         if pdl is not None:

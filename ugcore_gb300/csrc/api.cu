@@ -174,6 +174,12 @@ int ug4gb_set_tuning(ug4gb_ctx *ctx, int knob, int value)
         if (value < 0 || value > 4096 || value % 16) return UG4GB_ERR_INVALID;
         ctx->c.sweep_wait_test = value;
         return UG4GB_OK;
+    case UG4GB_TUNE_COARSE_BLOCKS:
+        if (value < 0 || value > 16) return UG4GB_ERR_INVALID;
+        ctx->c.coarse_blocks = value;
+        for (auto &q : ctx->c.coarse_ctas)
+            for (int &n : q) n = 0;
+        return UG4GB_OK;
     case UG4GB_TUNE_SCRATCH_TEST:
         if (value != 0 && value != 1) return UG4GB_ERR_INVALID;
         ctx->c.scratch_test = value;

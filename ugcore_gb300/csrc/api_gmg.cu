@@ -623,8 +623,15 @@ struct GmgT : GmgBase {
             smoother2 != UG4GB_SMOOTHER_JACOBI || base_kind != UG4GB_BASE_LU)
             return;
         constexpr size_t kSmemMax = 208 * 1024;
-        int &coarse_ctas = c.coarse_ctas[sizeof(V) == 8 ? 0 : 1];
-        if (coarse_ctas == 0) coarse_ctas = coarse_prepare<V>(c, kSmemMax);   // the most any multigrid asks for
+        if (base >= top()) return;
+        const int S = lev[base + 1].At.kind == 1 ? lev[base + 1].At.dia.S : 0;
+        if (!coarse_width_ok(S)) return;
+        int &coarse_ctas = c.coarse_ctas[sizeof(V) == 8 ? 0 : 1][S];
+        if (coarse_ctas == 0) {
+            coarse_ctas = coarse_prepare<V>(c, S, c.coarse_blocks, kSmemMax);   // the most any multigrid asks for
+            if (coarse_ctas == 0) coarse_ctas = -1;
+        }
+        if (coarse_ctas < 0) return;   // separate launches
         constexpr double kSharedWork = 110e3, kSharedWork2d = 400.0, kSoloWork = 1000.0;
         constexpr int kBaseRows = 32;
         constexpr int kAlign = 16 / (int)sizeof(V);   // elements per 16 bytes
@@ -640,7 +647,7 @@ struct GmgT : GmgBase {
             const GLevel<V> &T = lev[t];
             if (!T.grid_transfer || T.At.kind != 1 || T.At.nrows != T.n || T.At.ncols != T.n ||
                 T.gp.nx * T.gp.ny * T.gp.nz != T.n || T.gp.cnx * T.gp.cny * T.gp.cnz != lev[t - 1].n ||
-                !coarse_width_ok(T.At.dia.S) || T.At.dia.S != lev[base + 1].At.dia.S)
+                T.At.dia.S != S)
                 break;
             // (a level prepared for two steps per pass keeps its own launches; one
             // that takes two launches a cycle, k_level2d.cu, does so from 9^2 on:

@@ -112,6 +112,8 @@ struct ProfRec {
     cudaEvent_t a, b;
 };
 
+constexpr int kMaxDiag = 32;   // diagonals of a constant-offset layout (Dia)
+
 struct Ctx {
     int device = 0;
     int num_sms = 152;
@@ -133,10 +135,11 @@ struct Ctx {
     bool dia_flag_pending = false;
     int sweep_wait_test = 0;    // failure test only: bytes no copy delivers (fused sweeps' bounded waits run out)
     int scratch_test = 0;       // failure test only: the unstructured assembly asks for more memory than there is
-    // levels above the base cycled by the one-block coarse kernel (-1: as
-    // many as its cost model finds faster than separate launches, 0: none)
+    // levels above the base cycled by the coarse kernel's cluster of blocks (-1:
+    // as many as were measured faster than separate launches, 0: none)
     int coarse_levels = -1;
-    int coarse_ctas[2] = {0, 0};   // blocks per cluster it runs with, FP64 and FP32 levels (0: not asked yet)
+    int coarse_blocks = 16;        // the most blocks of that cluster
+    int coarse_ctas[2][kMaxDiag] = {};   // blocks it runs with, FP64 and FP32 levels, by stencil width (-1: none fit, 0: not asked yet)
     std::string prof_tag;       // set by the orchestration (level / phase)
     std::vector<ProfRec> prof;
     std::vector<cudaEvent_t> ev_pool;
@@ -253,7 +256,6 @@ inline SellView<T> view(const Sell<T> &s)
 // distinct column offsets (every level operator of a structured hierarchy:
 // 9, 15 or 27 of them); it carries no column indices at all and its loads do
 // not depend on each other.
-constexpr int kMaxDiag = 32;
 struct Offs {
     int o[kMaxDiag];
 };

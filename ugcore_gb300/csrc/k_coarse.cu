@@ -377,26 +377,27 @@ void coarse_cycle(Ctx &c, const CoarsePlan<V> *plan_dev, int ctas, int S, size_t
 bool coarse_width_ok(int S) { return S == 7 || S == 9 || S == 15 || S == 27; }
 
 template <class V>
-int coarse_prepare(Ctx &c, size_t smem_bytes)
+int coarse_prepare(Ctx &c, int S, int most_blocks, size_t smem_bytes)
 {
-    for (int S : {7, 9, 15, 27}) {
-        UG_CUDA(cudaFuncSetAttribute(coarse_kernel<V>(S), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes));
-        UG_CUDA(cudaFuncSetAttribute(coarse_kernel<V>(S), cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-    }
-    // 16 blocks need a processing cluster of the GPU with that many free SMs
-    cudaLaunchAttribute at[2];
-    const cudaLaunchConfig_t cfg = coarse_config<V>(c, 16, smem_bytes, at, false);
-    int most = 0;
-    if (cudaOccupancyMaxActiveClusters(&most, coarse_kernel<V>(27), &cfg) != cudaSuccess) {
+    const CoarseKernel<V> kernel = coarse_kernel<V>(S);
+    UG_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes));
+    UG_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    // a cluster needs a processing cluster of the GPU (or of the partition of it
+    // that is visible) with that many free SMs
+    for (int ctas = 16; ctas >= 1; ctas /= 2) {
+        if (ctas > most_blocks) continue;
+        cudaLaunchAttribute at[2];
+        const cudaLaunchConfig_t cfg = coarse_config<V>(c, ctas, smem_bytes, at, false);
+        int clusters = 0;
+        if (cudaOccupancyMaxActiveClusters(&clusters, kernel, &cfg) == cudaSuccess && clusters > 0) return ctas;
         (void)cudaGetLastError();
-        most = 0;
     }
-    return most > 0 ? 16 : 8;
+    return 0;
 }
 
 template void coarse_cycle<double>(Ctx &, const CoarsePlan<double> *, int, int, size_t, const int *);
 template void coarse_cycle<float>(Ctx &, const CoarsePlan<float> *, int, int, size_t, const int *);
-template int coarse_prepare<double>(Ctx &, size_t);
-template int coarse_prepare<float>(Ctx &, size_t);
+template int coarse_prepare<double>(Ctx &, int, int, size_t);
+template int coarse_prepare<float>(Ctx &, int, int, size_t);
 
 }  // namespace ug4gb

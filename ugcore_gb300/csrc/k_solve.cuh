@@ -276,10 +276,12 @@ struct alignas(16) CoarsePlan {
 template <class V>
 void coarse_cycle(Ctx &c, const CoarsePlan<V> *plan_dev, int ctas, int S, size_t smem_bytes, const int *skip);
 bool coarse_width_ok(int S);
-// set-up: allows launches with up to smem_bytes of dynamic shared memory;
-// returns the blocks per cluster the device runs with that much (16 or 8)
+// set-up: allows launches for width S with up to smem_bytes of dynamic shared
+// memory; returns the blocks per cluster that the device runs with that much: 16,
+// 8, 4, 2 or 1, at most most_blocks; 0 where it runs none
 template <class V>
-int coarse_prepare(Ctx &c, size_t smem_bytes);
+int coarse_prepare(Ctx &c, int S, int most_blocks, size_t smem_bytes);
+
 // ---- a 2D level of the V-cycle in two launches (k_level2d.cu) ----
 template <class V>
 struct DiaRows {
