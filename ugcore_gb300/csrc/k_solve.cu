@@ -899,10 +899,34 @@ __global__ void __launch_bounds__(NT, sizeof(V) == 4 ? 3 : 1) k_mcgs_lines(DiaMV
         }
 }
 
-GsLines gs_lines(const Offs &offs, int S, const std::vector<int> &entries, const GridPair &gp)
+// vertices of one x parity in a line, lines per block
+static int line_half(const GridPair &gp) { return (gp.nx + 1) / 2; }
+static int lines_per_block(const GridPair &gp) { return line_half(gp) < NT ? NT / line_half(gp) : 1; }
+
+// A block takes a line of more than 2 NT vertices in several rounds, one after the
+// other; with few such lines most of the GPU is idle, where a launch per colour
+// fills it.  Up to three rounds, or with blocks on half of the SMs, the lines are
+// faster.  Cycles with lines only within these limits / on all levels / on none:
+// 32769 x 65 quads FP32 618 / 1876 / 633 us, FP64 1089 / 3259 / 1101; 4097 x 65
+// FP32 276 / 332 / 340, FP64 411 / 563 / 499; 4097 x 9 x 9 hexes FP32 553 / 756 /
+// 585; 2049 x 1025 quads FP32 561 / 565 / 792 (limits of one and two rounds, or
+// blocks on all SMs, were slower: 4097 x 65 304 / 287, 4097 x 513 FP32 424).
+// FP64 rounds of 15 and 27 diagonals take 2 us of an SM's FP64 pipe: with fewer
+// than four blocks one round is the limit (1025 x 3 x 3 hexes below 4097 x 9 x 9: a
+// cycle 895 us with three rounds, 833 with one, 816 by colours).
+static bool lines_fill(const Ctx &c, const GridPair &gp, bool fp64_bound)
+{
+    const int rounds = (int)div_up(line_half(gp), NT);
+    const int lines = (gp.ny / 2) * (gp.dim == 3 ? gp.nz / 2 : 1);   // of the smallest set
+    const int blocks = (int)div_up(lines, lines_per_block(gp));
+    if (rounds <= 1 || blocks >= c.num_sms / 2) return true;
+    return rounds <= 3 && (!fp64_bound || blocks >= 4);
+}
+
+GsLines gs_lines(const Ctx &c, bool fp64, const Offs &offs, int S, const std::vector<int> &entries, const GridPair &gp)
 {
     GsLines g;
-    if (gp.nx < 3 || gp.ny < 3 || S > 32) return g;
+    if (gp.nx < 3 || gp.ny < 3 || S > 32 || !lines_fill(c, gp, fp64 && S >= 15)) return g;
     for (int k = 0; k < S; ++k) {
         const int o = offs.o[k];
         if (!std::binary_search(entries.begin(), entries.end(), o)) continue;
@@ -934,7 +958,7 @@ void mcgs_sweep_lines(Ctx &c, const OpMat<V> &A, const GsLines &gs, const GridPa
     with_mv(A, [&](auto mv) {
         using MV = decltype(mv);
         if constexpr (is_dia<MV>::value) {
-            const int np = gp.dim == 3 ? 4 : 2, per = (gp.nx + 1) / 2, per_block = per < NT ? NT / per : 1;
+            const int np = gp.dim == 3 ? 4 : 2, per = line_half(gp), per_block = lines_per_block(gp);
             for (int s = 0; s < np; ++s) {
                 const int p = backward ? np - 1 - s : s, b1 = p & 1, b2 = p >> 1;
                 const int nly = (gp.ny - b1 + 1) / 2, nlz = gp.dim == 3 ? (gp.nz - b2 + 1) / 2 : 1;
