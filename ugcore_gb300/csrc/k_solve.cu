@@ -65,7 +65,10 @@ struct SellMV {
             }
         }
     }
-    // dot with a prefetched row; same order of operations as dot
+    // dot with a prefetched row; same order of operations as dot.  FP64 leaves at the
+    // row's end: a product that a predicate turns off still takes its turn on the
+    // FP64 pipe (triangles, 7 of 8 slots, 2400 rows: a V(2,2) cycle 53.3 us, 50.0
+    // with the branches; FP32 the other way round, 41.1 and 41.7).
     template <class ACC, class XT>
     __device__ __forceinline__ ACC dot_cached(const XT *__restrict__ x, int, const Cache &c) const
     {
@@ -75,8 +78,14 @@ struct SellMV {
             if (k < c.w) xv[k] = (ACC)x[c.col[k]];
         ACC acc = (ACC)0;
 #pragma unroll
-        for (int k = 0; k < kCache; ++k)
-            if (k < c.w) acc = fma_rn((ACC)c.val[k], xv[k], acc);
+        for (int k = 0; k < kCache; ++k) {
+            if constexpr (sizeof(ACC) == 8) {
+                if (k >= c.w) return acc;
+                acc = fma_rn((ACC)c.val[k], xv[k], acc);
+            } else {
+                if (k < c.w) acc = fma_rn((ACC)c.val[k], xv[k], acc);
+            }
+        }
         // the rest: the loads of kCache entries issued before their sum (one
         // entry after the other cost a level of 15000 rows 2 us per product)
 #pragma unroll 1
@@ -93,8 +102,14 @@ struct SellMV {
             for (int q = 0; q < kCache; ++q)
                 if (k + q < c.w) xv[q] = (ACC)x[col[q]];
 #pragma unroll
-            for (int q = 0; q < kCache; ++q)
-                if (k + q < c.w) acc = fma_rn((ACC)val[q], xv[q], acc);
+            for (int q = 0; q < kCache; ++q) {
+                if constexpr (sizeof(ACC) == 8) {
+                    if (k + q >= c.w) return acc;
+                    acc = fma_rn((ACC)val[q], xv[q], acc);
+                } else {
+                    if (k + q < c.w) acc = fma_rn((ACC)val[q], xv[q], acc);
+                }
+            }
         }
         return acc;
     }
@@ -114,17 +129,26 @@ struct SellMV {
     }
 };
 
-// The view of a SELL matrix for products of few rows (up to a block per SM):
-// whole rows are loaded ahead of the launch wait, as the 15 to 24 entries of a
-// tetrahedral vertex otherwise take another round of dependent loads.  Solves on
-// unstructured tetrahedra with 8 / 16 / 24 / 32 entries: 0.9M rows FP32 10.51 /
-// 10.08 / 9.74 / 9.79 ms, FP64 15.8 / 15.5 / 14.7 / 15.0; 0.12M rows FP32 4.25 /
-// 3.83 / 3.46 / 3.52, FP64 6.59 / 6.37 / 5.50 / 5.83.  With more rows the registers
-// cost more than the loads: a step of 117000 rows FP32 11.1 -> 13.6 us with 24.
-template <class V>
-SellMV<V, 24> few_rows(const SellMV<V> &m)
+// Products of few rows (up to a block per SM) of a SELL matrix load whole rows
+// ahead of the launch wait, as an entry beyond takes another round of dependent
+// loads; slots that a row does not fill cost instructions and registers.  So the
+// slots follow the slices' mean width.  V(2,2) cycles with 8 / 12 / 16 / 24 slots
+// (us; FP64, then FP32):
+//   triangles, 7 entries, 37000 rows         73.3 / 71.9 / 72.4 / 74.0    57.5 / 58.0 / 59.0 / 59.6
+//   the same, 148000 rows                   107.7 /101.6 /104.1 /107.3    73.7 / 74.0 / 74.7 / 75.4
+//   quadrilaterals, 9 entries, 37000 rows    91.5 / 78.3 / 79.0 / 81.2    71.5 / 61.6 / 62.0 / 61.6
+//   tetrahedra, 15 to 24, 36000 rows         88.5 / 78.5 / 79.9 / 71.4    63.1 / 66.0 / 56.5 / 46.7
+//   hexahedra, 27, 36000 rows               113.9 /110.2 / 98.1 / 96.6    86.7 /121.9 / 66.5 / 78.0
+// With more rows the registers cost more than the loads: a step of 117000 rows of
+// tetrahedra FP32 11.1 -> 13.6 us with 24.
+template <class V, class F>
+void with_few_rows(const Sell<V> &m, const SellMV<V> &mv, F &&f)
 {
-    return SellMV<V, 24>{m.s};
+    const int64_t slots = (int64_t)m.nslices * kSliceH;
+    if (sizeof(V) == 4 && m.stored <= 8 * slots) f(mv);
+    else if (m.stored <= 12 * slots) f(SellMV<V, 12>{mv.s});
+    else if (m.stored <= 24 * slots) f(SellMV<V, 24>{mv.s});
+    else f(SellMV<V, 16>{mv.s});
 }
 
 template <class V, int S>
@@ -464,9 +488,10 @@ void smooth_step(Ctx &c, const OpMat<V> &At, const XT *x, const DT *dbase, const
         RedArgs none{nullptr, nullptr, nullptr};
         if constexpr (!is_dia<MV>::value) {
             if (pf && !r_rho && At.nrows <= c.num_sms * NT) {
-                const auto few = few_rows(mv);
-                UG_LAUNCH_PDL(c, (k_smooth<decltype(few_rows(mv)), V, XT, DT, false, true>), g, NT, 0, few, x, dbase,
-                              dinv, sc, dout, sc_mode, skip, (const double *)nullptr, none, 0, z64);
+                with_few_rows(At.sell, mv, [&](auto few) {
+                    UG_LAUNCH_PDL(c, (k_smooth<decltype(few), V, XT, DT, false, true>), g, NT, 0, few, x, dbase, dinv,
+                                  sc, dout, sc_mode, skip, (const double *)nullptr, none, 0, z64);
+                });
                 return;
             }
         }
@@ -516,9 +541,10 @@ void restrict_apply(Ctx &c, const OpMat<V> &R, const V *d, V *dc, const int *ski
     with_mv(R, [&](auto mv) {
         if constexpr (!is_dia<decltype(mv)>::value) {
             if (R.nrows <= c.num_sms * NT) {
-                const auto few = few_rows(mv);
-                UG_LAUNCH_PDL(c, (k_restrict<decltype(few_rows(mv)), V, true>), row_grid(c, R.nrows), NT, 0, few, d,
-                              dc, skip);
+                with_few_rows(R.sell, mv, [&](auto few) {
+                    UG_LAUNCH_PDL(c, (k_restrict<decltype(few), V, true>), row_grid(c, R.nrows), NT, 0, few, d, dc,
+                                  skip);
+                });
                 return;
             }
         }
@@ -559,6 +585,15 @@ template <class V>
 void prolong_apply(Ctx &c, const OpMat<V> &P, const V *scc, V *sc, const V *dfac, V *w, const int *skip)
 {
     with_mv(P, [&](auto mv) {
+        if constexpr (!is_dia<decltype(mv)>::value) {
+            // rows of one or two parents (triangles, tetrahedra: a V(2,2) cycle of
+            // 148000 FP64 rows of triangles 108.0 -> 105.2 us)
+            if (P.nrows <= c.num_sms * NT && P.sell.stored <= 2 * (int64_t)P.sell.nslices * kSliceH) {
+                UG_LAUNCH_PDL(c, (k_prolong<SellMV<V, 2>, V, true>), row_grid(c, P.nrows), NT, 0, (SellMV<V, 2>{mv.s}),
+                              scc, sc, dfac, w, skip);
+                return;
+            }
+        }
         if (P.nrows <= c.num_sms * NT * (sizeof(V) == 4 ? 8 : 1))
             UG_LAUNCH_PDL(c, (k_prolong<decltype(mv), V, true>), row_grid(c, P.nrows), NT, 0, mv, scc, sc, dfac, w,
                           skip);
