@@ -503,8 +503,6 @@ constexpr int kRapCap = 64;
 void csr_rap(Ctx &c, const Csr &R, const Csr &A, const Csr &P, Csr &M);
 template <class T>
 void sell_from_csr(Ctx &c, const Csr &A, Sell<T> &S, const double *col_scale /* nullable */);
-// distinct column offsets (col - row) of A, sorted; false if more than max_s
-bool csr_offsets(Ctx &c, const Csr &A, int max_s, std::vector<int> &offs);
 // The layout an operator's solve format was built with (diagonal offsets or
 // SELL-32 slices).  While the caller knows the CRS pattern is unchanged (the
 // same level, re-assembled), op_from_csr_cached refills the values of the

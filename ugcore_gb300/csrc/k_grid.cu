@@ -446,16 +446,34 @@ __global__ void k_offset_range(const int *rowptr, const int *col, int nrows, int
     }
 }
 
-__global__ void k_offset_mark(const int *rowptr, const int *col, int nrows, int lo, int *mark)
+// which offsets (from lo, n of them) occur with a zero entry (mark[0 .. n - 1]) and
+// with a nonzero one (mark[n ..]); mark[2 n]: some row's columns are not strictly
+// increasing
+__global__ void k_offset_mark(const int *__restrict__ rowptr, const int *__restrict__ col,
+                              const double *__restrict__ val, int nrows, int lo, size_t n, unsigned char *mark)
 {
-    int r = blockIdx.x * blockDim.x + threadIdx.x;
+    const int r = blockIdx.x * blockDim.x + threadIdx.x;
     if (r >= nrows) return;
-    for (int a = rowptr[r]; a < rowptr[r + 1]; ++a) mark[col[a] - r - lo] = 1;
+    int last = -1;
+    bool bad = false;
+    for (int a = rowptr[r]; a < rowptr[r + 1]; ++a) {
+        const int cc = col[a], o = cc - r - lo;
+        mark[val[a] != 0.0 ? n + o : (size_t)o] = 1;
+        bad = bad || cc <= last;
+        last = cc;
+    }
+    if (bad) mark[2 * n] = 1;
 }
 
-bool csr_offsets(Ctx &c, const Csr &A, int max_s, std::vector<int> &offs)
+// The distinct column offsets (col - row) of A, increasing, and for each whether
+// a nonzero entry has it; sorted: every row's columns are strictly increasing.
+// False if there are more than max_s.  (One pass and one wait for all three: a
+// pass of its own over the values made the set-up of Galerkin levels up to 9%
+// longer.)
+static bool csr_offsets(Ctx &c, const Csr &A, int max_s, std::vector<int> &offs, std::vector<bool> &used, bool &sorted)
 {
     offs.clear();
+    used.clear();
     if (A.nrows == 0 || A.nnz == 0) return false;
     DevBuf<int> mm;
     mm.alloc(2);
@@ -465,20 +483,23 @@ bool csr_offsets(Ctx &c, const Csr &A, int max_s, std::vector<int> &offs)
     int h[2];
     UG_CUDA(cudaMemcpyAsync(h, mm.p, sizeof(h), cudaMemcpyDeviceToHost, c.stream));
     UG_CUDA(cudaStreamSynchronize(c.stream));
-    int64_t span = (int64_t)h[1] - h[0] + 1;
+    const int64_t span = (int64_t)h[1] - h[0] + 1;
     if (span <= 0 || span > (int64_t)64 << 20) return false;
-    DevBuf<int> mark;
-    mark.alloc(span);
+    DevBuf<unsigned char> mark;
+    mark.alloc(2 * (size_t)span + 1);
     UG_CUDA(cudaMemsetAsync(mark.p, 0, mark.bytes(), c.stream));
-    UG_LAUNCH(c, k_offset_mark, div_up(A.nrows, 256), 256, 0, A.rowptr.p, A.col.p, A.nrows, h[0], mark.p);
-    std::vector<int> hm(span);
+    UG_LAUNCH(c, k_offset_mark, div_up(A.nrows, 256), 256, 0, A.rowptr.p, A.col.p, A.val.p, A.nrows, h[0],
+              (size_t)span, mark.p);
+    std::vector<unsigned char> hm(mark.n);
     UG_CUDA(cudaMemcpyAsync(hm.data(), mark.p, mark.bytes(), cudaMemcpyDeviceToHost, c.stream));
     UG_CUDA(cudaStreamSynchronize(c.stream));
     for (int64_t i = 0; i < span; ++i)
-        if (hm[i]) {
+        if (hm[i] || hm[span + i]) {
             offs.push_back((int)(i + h[0]));
+            used.push_back(hm[span + i] != 0);
             if ((int)offs.size() > max_s) return false;
         }
+    sorted = hm[2 * span] == 0;
     return true;
 }
 
@@ -500,34 +521,6 @@ static DiaMap dia_map(const OpLayout &lay)
         m.slot[k] = (it != lay.offs.end() && *it == lay.all[k]) ? (int)(it - lay.offs.begin()) : -1;
     }
     return m;
-}
-
-// which offsets hold a nonzero entry (bit k of used: offset m.off[k]), and
-// whether any row's columns are not strictly increasing
-__global__ void k_dia_used(const int *__restrict__ rowptr, const int *__restrict__ col,
-                           const double *__restrict__ val, int nrows, DiaMap m, unsigned *used, int *unsorted)
-{
-    __shared__ unsigned block_bits;
-    if (threadIdx.x == 0) block_bits = 0u;
-    __syncthreads();
-    unsigned bits = 0u;
-    bool bad = false;
-    const int stride = gridDim.x * blockDim.x;
-    for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < nrows; r += stride) {
-        int last = -1, k = 0;
-        for (int a = rowptr[r]; a < rowptr[r + 1]; ++a) {
-            const int cc = col[a];
-            bad = bad || cc <= last;
-            if (cc <= last) k = 0;
-            last = cc;
-            while (k < m.n && m.off[k] != cc - r) ++k;
-            if (k < m.n && val[a] != 0.0) bits |= 1u << k;
-        }
-    }
-    if (bits) atomicOr(&block_bits, bits);
-    if (bad) atomicExch(unsorted, 1);
-    __syncthreads();
-    if (threadIdx.x == 0 && block_bits) atomicOr(used, block_bits);
 }
 
 // CRS -> diagonals.  Bound by memory: 8 bytes read and sizeof(T) written per
@@ -659,28 +652,17 @@ static int dia_width(int s)
     return 0;
 }
 
-// the offsets of lay.all a layout of A stores: those with a nonzero entry
-// (all of them if none has one, or with keep_all), padded
+// the offsets of lay.all a layout stores: those with a nonzero entry (all of
+// them if none has one, or with keep_all), padded
 template <class T>
-static void choose_offsets(Ctx &c, const Csr &A, OpLayout &lay)
+static void choose_offsets(const Ctx &c, const std::vector<bool> &used, OpLayout &lay)
 {
-    OpLayout every;
-    every.offs = every.all = lay.all;
-    DevBuf<int> st;
-    st.alloc(2);
-    UG_CUDA(cudaMemsetAsync(st.p, 0, 2 * sizeof(int), c.stream));
-    UG_LAUNCH(c, k_dia_used, std::min<int>((int)div_up(A.nrows, 256), c.num_sms * 8), 256, 0, A.rowptr.p, A.col.p,
-              A.val.p, A.nrows, dia_map(every), (unsigned *)st.p, st.p + 1);
-    int h[2];
-    UG_CUDA(cudaMemcpyAsync(h, st.p, sizeof(h), cudaMemcpyDeviceToHost, c.stream));
-    UG_CUDA(cudaStreamSynchronize(c.stream));
-    const unsigned used = (unsigned)h[0];
-    lay.sorted = h[1] == 0;
     // the fused sweeps (k_sweep2.cu) take the element types' whole stencils
-    const bool whole = lay.keep_all || used == 0 || (sizeof(T) == 4 && (c.sweep_fusion & 1));
+    const bool any = std::find(used.begin(), used.end(), true) != used.end();
+    const bool whole = lay.keep_all || !any || (sizeof(T) == 4 && (c.sweep_fusion & 1));
     lay.offs.clear();
     for (size_t k = 0; k < lay.all.size(); ++k)
-        if (whole || ((used >> k) & 1u)) lay.offs.push_back(lay.all[k]);
+        if (whole || used[k]) lay.offs.push_back(lay.all[k]);
     // fewer offsets that still fill the same kernel's width save nothing
     if (dia_width((int)lay.offs.size()) == dia_width((int)lay.all.size())) lay.offs = lay.all;
     lay.left_out = lay.offs.size() < lay.all.size();
@@ -699,8 +681,9 @@ static void op_build(Ctx &c, const Csr &A, OpMat<T> &M, const double *col_scale,
     lay.all.clear();
     lay.offs.clear();
     lay.left_out = false;
-    if (allow_dia && A.nrows == A.ncols && csr_offsets(c, A, 27, lay.all)) {
-        choose_offsets<T>(c, A, lay);
+    std::vector<bool> used;
+    if (allow_dia && A.nrows == A.ncols && csr_offsets(c, A, 27, lay.all, used, lay.sorted)) {
+        choose_offsets<T>(c, used, lay);
         M.kind = 1;
         // the offsets were just chosen by these values: no entry to report
         dia_from_csr<T>(c, A, M.dia, lay, col_scale, false, false);
