@@ -632,7 +632,7 @@ struct GmgT : GmgBase {
             if (coarse_ctas == 0) coarse_ctas = -1;
         }
         if (coarse_ctas < 0) return;   // separate launches
-        constexpr double kSharedWork = 110e3, kSharedWork2d = 400.0, kSoloWork = 1000.0;
+        constexpr double kSharedWork = 110e3, kSharedWork2d = 400.0, kSharedWorkSweep2 = 16e3, kSoloWork = 1000.0;
         constexpr int kBaseRows = 32;
         constexpr int kAlign = 16 / (int)sizeof(V);   // elements per 16 bytes
         auto up = [](size_t v, size_t a) { return (v + a - 1) / a * a; };
@@ -649,11 +649,15 @@ struct GmgT : GmgBase {
                 T.gp.nx * T.gp.ny * T.gp.nz != T.n || T.gp.cnx * T.gp.cny * T.gp.cnz != lev[t - 1].n ||
                 T.At.dia.S != S)
                 break;
-            // (a level prepared for two steps per pass keeps its own launches; one
-            // that takes two launches a cycle, k_level2d.cu, does so from 9^2 on:
-            // 129^2 solve 540 -> 527 us, FP32 416 -> 361 us)
-            const double limit = T.level2d && nu1 == 2 && nu2 == 2 ? kSharedWork2d : kSharedWork;
-            if (c.coarse_levels > 0 ? t - base > c.coarse_levels : work(t) > limit || T.sweep2) break;
+            // (a level that takes two launches a cycle, k_level2d.cu, does so from 9^2
+            // on: 129^2 solve 540 -> 527 us, FP32 416 -> 361 us; one prepared for two
+            // steps per pass, k_sweep2.cu, keeps its launches from some 500 rows of 27
+            // diagonals or 900 of 15 on: V(4,4) on 65 x 257 x 65 tetrahedra with every
+            // level prepared 385 us with none of them here, 351 with those of 81 and
+            // 425 rows)
+            const double limit = T.sweep2 ? kSharedWorkSweep2
+                                          : (T.level2d && nu1 == 2 && nu2 == 2 ? kSharedWork2d : kSharedWork);
+            if (c.coarse_levels > 0 ? t - base > c.coarse_levels : work(t) > limit) break;
             CoarsePlan<V> P{};
             P.m = t - base + 1;
             bool any_shared = !solo_base;
