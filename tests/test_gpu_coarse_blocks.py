@@ -38,3 +38,15 @@ def test_bit_identical(name, over, prec):
             assert np.array_equal(got, want), (blocks, levels)
             # (a few blocks' shared memory may not hold a base of 216 unknowns)
             assert launches == (1 if blocks else 0) or (levels == -1 or 0 < blocks < 8)
+
+
+@pytest.mark.parametrize("prec", ["fp64", "mixed"])
+@pytest.mark.parametrize("over,launches", [
+    (dict(mx=15, my=15, nref=2), 1), (dict(mx=16, my=15, nref=2), 0),       # bases of 256 and 272 rows
+    (dict(mx=1, my=9, nref=3, nu1=4, nu2=4), 1), (dict(mx=3, my=3, nref=3, nu1=4, nu2=4), 1),   # one block
+    (dict(mx=3, my=4, nref=4, nu1=4, nu2=4), 1)])                            # a cluster
+def test_automatic_plans(over, launches, prec):
+    over = dict(over, nu1=over.get("nu1", 1), nu2=over.get("nu2", 1))
+    want, _ = _correction("c3", over, prec, coarse_levels=0)
+    got, n = _correction("c3", over, prec)
+    assert np.array_equal(got, want) and n == launches

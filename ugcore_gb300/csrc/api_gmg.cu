@@ -614,7 +614,12 @@ struct GmgT : GmgBase {
     // about 1000.  Against separate launches above one block's levels: 129^2
     // solve 690 -> 651 us, 257^2 gradient 4.13 -> 3.98 ms, Newton on 49^3 tets
     // 4.45 -> 4.07 ms.  A base of more than 32 rows is shared too: one warp per
-    // row is FP64 bound on one SM.
+    // row is FP64 bound on one SM.  Of more than 256 rows its inverse takes so long
+    // to stage that separate launches are faster (FP32 levels on a base of 473 rows,
+    // a CG step with V(2,2), V(1,1), V(1,0): 30.7, 34.6, 32.6 us by separate launches,
+    // 30.4, 39.1, 38.6 by a cluster).  Where no level passes 4000 row-operations in
+    // FP64 or 8000 in FP32, one block does all of it without a cluster (V(4,4) on 9 x
+    // 73 quads, FP32, a CG step 50.1 -> 47.3 us).
     void setup_coarse(Ctx &c)
     {
         coarse_top = -1;
@@ -633,7 +638,9 @@ struct GmgT : GmgBase {
         }
         if (coarse_ctas < 0) return;   // separate launches
         constexpr double kSharedWork = 110e3, kSharedWork2d = 400.0, kSharedWorkSweep2 = 16e3, kSoloWork = 1000.0;
-        constexpr int kBaseRows = 32;
+        constexpr double kOneBlockWork = sizeof(V) == 8 ? 4000.0 : 8000.0;
+        constexpr int kBaseRows = 32, kBaseRowsMax = 256;
+        if (c.coarse_levels < 0 && nbase > kBaseRowsMax) return;
         constexpr int kAlign = 16 / (int)sizeof(V);   // elements per 16 bytes
         auto up = [](size_t v, size_t a) { return (v + a - 1) / a * a; };
         auto work = [&](int l) { return (double)lev[l].n * (lev[l].At.dia.S + 3); };
@@ -661,7 +668,7 @@ struct GmgT : GmgBase {
             CoarsePlan<V> P{};
             P.m = t - base + 1;
             bool any_shared = !solo_base;
-            for (int l = base + 1; l <= t; ++l) any_shared |= work(l) > kSoloWork;
+            for (int l = base + 1; l <= t; ++l) any_shared |= work(l) > kOneBlockWork;
             P.ctas = any_shared ? coarse_ctas : 1;
             size_t e = 0;   // level-precision elements so far
             bool solo = any_shared ? solo_base : true, ok = true;
