@@ -766,10 +766,11 @@ struct GmgT : GmgBase {
             cur = L.dB.p;
         }
         const bool pre3d = L.level3d && l < T && nu1 == 2 && first;
-        if (pre3d) {
-            level3d_pre<V>(c, L.At, L.gp, L.dinv.p, cur, L.sc.p, L.dB.p, skip);
-            cur = L.dB.p;
-        }
+        if constexpr (sizeof(V) == 4)
+            if (pre3d) {
+                level3d_pre(c, L.At, L.gp, L.dinv.p, cur, L.sc.p, L.dB.p, skip);
+                cur = L.dB.p;
+            }
         // ---- pre-smoothing
         if (nu1 == 0 && first) UG_LAUNCH_PDL(c, k_zero<V>, div_up(L.n, 256), 256, 0, L.n, L.sc.p, skip);
         for (int k = 0; k < nu1 && !pre2d && !pre3d; ++k) {
@@ -792,11 +793,11 @@ struct GmgT : GmgBase {
             cur = out;
         }
         const V *dpre = cur;
-        // ---- restriction
-        if (pre2d) {
-            // done
-        } else if (L.grid_transfer) restrict_grid<V>(c, L.gp, dpre, C.dA.p, skip);
-        else restrict_apply<V>(c, L.Rs, dpre, C.dA.p, skip);
+        // ---- restriction (level2d_pre has done it)
+        if (!pre2d) {
+            if (L.grid_transfer) restrict_grid<V>(c, L.gp, dpre, C.dA.p, skip);
+            else restrict_apply<V>(c, L.Rs, dpre, C.dA.p, skip);
+        }
         C.dcur = C.dA.p;
         // ---- coarse correction
         if (l - 1 == base) {
@@ -824,11 +825,12 @@ struct GmgT : GmgBase {
             L.dcur = const_cast<V *>(dpre);   // read by no later visit
             return;
         }
-        if (L.level3d && l < T && nu2 == 2 && cycle == 1) {
-            level3d_post<V>(c, L.At, L.gp, L.dinv.p, L.dfac.p, C.sc.p, dpre, L.sc.p, skip);
-            L.dcur = const_cast<V *>(dpre);   // read by no later visit
-            return;
-        }
+        if constexpr (sizeof(V) == 4)
+            if (L.level3d && l < T && nu2 == 2 && cycle == 1) {
+                level3d_post(c, L.At, L.gp, L.dinv.p, L.dfac.p, C.sc.p, dpre, L.sc.p, skip);
+                L.dcur = const_cast<V *>(dpre);   // read by no later visit
+                return;
+            }
         if (L.grid_transfer) prolong_grid<V>(c, L.gp, C.sc.p, L.sc.p, L.dfac.p, nu2 > 0 ? L.w.p : (V *)nullptr, skip);
         else prolong_apply<V>(c, L.Ps, C.sc.p, L.sc.p, L.dfac.p, nu2 > 0 ? L.w.p : (V *)nullptr, skip);
         const V *dbase = dpre;
@@ -1085,9 +1087,9 @@ static GmgBase *build_gmg(ug4gb_gmg *m, const ug4gb_matrix *A_top, GmgT<V> *reus
         if (!own || l == m->base || !L.grid_transfer || L.At.kind != 1) continue;
         if (m->smoother == UG4GB_SMOOTHER_JACOBI) {
             L.level2d = m->smoother2 == UG4GB_SMOOTHER_JACOBI && level2d_ok<V>(L.At, L.gp);
-            L.level3d = m->smoother2 == UG4GB_SMOOTHER_JACOBI && !L.sweep2 && level3d_ok<V>(L.At, L.gp);
-        }
-        else if (L.At_lay.known)
+            if constexpr (sizeof(V) == 4)
+                L.level3d = m->smoother2 == UG4GB_SMOOTHER_JACOBI && !L.sweep2 && level3d_ok(L.At, L.gp);
+        } else if (L.At_lay.known)
             L.gs = gs_lines(c, sizeof(V) == 8, L.At.dia.off, L.At.dia.S, L.At_lay.all, L.gp);
     }
     G->setup_base(c);

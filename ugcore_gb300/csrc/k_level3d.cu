@@ -28,13 +28,12 @@ constexpr int kA = kAX * kAY * kAZ, kW = kWX * kWY * kWZ;
 constexpr int kT = (kA + 31) / 32 * 32;                          // threads: one per vertex of the first step
 
 // (At x) of the vertex at *t of a region of lines of sx and planes of sxy values
-template <class V>
-__device__ __forceinline__ V tile_row(const V (&a)[27], const V *t, int sx, int sxy)
+__device__ __forceinline__ float tile_row(const float (&a)[27], const float *t, int sx, int sxy)
 {
-    V v[27];
+    float v[27];
 #pragma unroll
     for (int k = 0; k < 27; ++k) v[k] = t[k % 3 - 1 + sx * (k / 3 % 3 - 1) + sxy * (k / 9 - 1)];
-    return row_sum<V, 27>(a, v);
+    return row_sum<float, 27>(a, v);
 }
 
 // this thread's vertex of the first step
@@ -59,52 +58,50 @@ struct Place {
 };
 
 // the operator row and Jacobi factor; 0 outside the level
-template <class V>
-__device__ __forceinline__ void load_row(const DiaRows<V> &A, const V *__restrict__ dinv, const Place &p, V (&a)[27],
-                                         V &di)
+__device__ __forceinline__ void load_row(const DiaRows<float> &A, const float *__restrict__ dinv, const Place &p,
+                                         float (&a)[27], float &di)
 {
 #pragma unroll
-    for (int k = 0; k < 27; ++k) a[k] = p.in ? ld_stream(A.val + (size_t)k * A.ld + p.row) : (V)0;
-    di = p.in ? __ldg(dinv + p.row) : (V)0;
+    for (int k = 0; k < 27; ++k) a[k] = p.in ? ld_stream(A.val + (size_t)k * A.ld + p.row) : 0.0f;
+    di = p.in ? __ldg(dinv + p.row) : 0.0f;
 }
 
 // f(vertex, its place in the region read by the first step) for all of it; the
 // value outside the level is 0
-template <class V, class F>
-__device__ __forceinline__ void fill_region(const GridPair &g, V *s, F &&f)
+template <class F>
+__device__ __forceinline__ void fill_region(const GridPair &g, float *s, F &&f)
 {
     for (int q = threadIdx.x; q < kW; q += kT) {
         const int x = q % kWX, y = q / kWX % kWY, z = q / (kWX * kWY);
         const int i = (int)blockIdx.x * kOX - 2 + x, j = (int)blockIdx.y * kOY - 2 + y,
                   k = (int)blockIdx.z * kOZ - 2 + z;
         const bool in = i >= 0 && i < g.nx && j >= 0 && j < g.ny && k >= 0 && k < g.nz;
-        s[q] = in ? f(i, j, k, q) : (V)0;
+        s[q] = in ? f(i, j, k, q) : 0.0f;
     }
 }
 
 // d1 = d - At d, sc = dinv d; d2 = d1 - At d1, sc += dinv d1
-template <class V>
 __global__ void __launch_bounds__(kT, 2)
-    k_pre3d(DiaRows<V> A, GridPair g, const V *__restrict__ dinv, const V *__restrict__ d, V *__restrict__ sc,
-            V *__restrict__ dout, const int *skip)
+    k_pre3d(DiaRows<float> A, GridPair g, const float *__restrict__ dinv, const float *__restrict__ d,
+            float *__restrict__ sc, float *__restrict__ dout, const int *skip)
 {
-    __shared__ V s0[kW], s1[kA];
+    __shared__ float s0[kW], s1[kA];
     const Place p(g);
-    V a[27], di;
+    float a[27], di;
     pdl_trigger();
-    load_row<V>(A, dinv, p, a, di);
+    load_row(A, dinv, p, a, di);
     pdl_wait();
     if (skip && *skip) return;
-    fill_region<V>(g, s0, [&](int i, int j, int k, int) { return d[i + g.nx * (j + g.ny * k)]; });
+    fill_region(g, s0, [&](int i, int j, int k, int) { return d[i + g.nx * (j + g.ny * k)]; });
     __syncthreads();
-    V d1 = (V)0, s = (V)0;
-    if (p.in) d1 = jacobi_row<V>(tile_row<V>(a, s0 + p.in_w(), kWX, kWX * kWY), s0[p.in_w()], di,
-                                 SC_SET_FROM_BASE, (V)0, s);
+    float d1 = 0.0f, s = 0.0f;
+    if (p.in) d1 = jacobi_row<float>(tile_row(a, s0 + p.in_w(), kWX, kWX * kWY), s0[p.in_w()], di, SC_SET_FROM_BASE,
+                                     0.0f, s);
     if (threadIdx.x < kA) s1[p.in_a()] = d1;
     __syncthreads();
     if (p.own) {
-        V sn;
-        const V d2 = jacobi_row<V>(tile_row<V>(a, s1 + p.in_a(), kAX, kAX * kAY), d1, di, SC_ADD_FROM_BASE, s, sn);
+        float sn;
+        const float d2 = jacobi_row<float>(tile_row(a, s1 + p.in_a(), kAX, kAX * kAY), d1, di, SC_ADD_FROM_BASE, s, sn);
         sc[p.row] = sn;
         dout[p.row] = d2;
     }
@@ -112,86 +109,68 @@ __global__ void __launch_bounds__(kT, 2)
 
 // t = P scc, sc += t, w = t dfac; d3 = d - At w, sc += dinv d3; d4 = d3 - At d3,
 // sc += dinv d4
-template <class V>
 __global__ void __launch_bounds__(kT, 2)
-    k_post3d(DiaRows<V> A, GridPair g, const V *__restrict__ dinv, const V *__restrict__ dfac,
-             const V *__restrict__ scc, const V *__restrict__ d, V *__restrict__ sc, const int *skip)
+    k_post3d(DiaRows<float> A, GridPair g, const float *__restrict__ dinv, const float *__restrict__ dfac,
+             const float *__restrict__ scc, const float *__restrict__ d, float *__restrict__ sc, const int *skip)
 {
-    __shared__ V sw[kW], st[kW], s3[kA];
+    __shared__ float sw[kW], st[kW], s3[kA];
     const Place p(g);
-    V a[27], di;
+    float a[27], di;
     pdl_trigger();
-    load_row<V>(A, dinv, p, a, di);
+    load_row(A, dinv, p, a, di);
     pdl_wait();
     if (skip && *skip) return;
-    const V db = p.in ? d[p.row] : (V)0;
-    V s = p.own ? sc[p.row] : (V)0;
-    fill_region<V>(g, sw, [&](int i, int j, int k, int q) {
-        const V df = __ldg(dfac + (i + g.nx * (j + g.ny * k)));
-        V t = prolong_value<V>(g, [&](int c) { return scc[c]; }, i, j, k);
-        if (g.dprol != 1.0) t = mul_rn(t, (V)g.dprol);
+    const float db = p.in ? d[p.row] : 0.0f;
+    float s = p.own ? sc[p.row] : 0.0f;
+    fill_region(g, sw, [&](int i, int j, int k, int q) {
+        const float df = __ldg(dfac + (i + g.nx * (j + g.ny * k)));
+        float t = prolong_value<float>(g, [&](int c) { return scc[c]; }, i, j, k);
+        if (g.dprol != 1.0) t = mul_rn(t, (float)g.dprol);
         st[q] = t;
         return mul_rn(t, df);
     });
     __syncthreads();
-    V d3 = (V)0;
+    float d3 = 0.0f;
     if (p.in) {
-        V sn;
+        float sn;
         s = add_rn(s, st[p.in_w()]);
-        d3 = jacobi_row<V>(tile_row<V>(a, sw + p.in_w(), kWX, kWX * kWY), db, di, SC_ADD_FROM_NEW, s, sn);
+        d3 = jacobi_row<float>(tile_row(a, sw + p.in_w(), kWX, kWX * kWY), db, di, SC_ADD_FROM_NEW, s, sn);
         s = sn;
     }
     if (threadIdx.x < kA) s3[p.in_a()] = d3;
     __syncthreads();
     if (p.own) {
-        V sn;
-        jacobi_row<V>(tile_row<V>(a, s3 + p.in_a(), kAX, kAX * kAY), d3, di, SC_ADD_FROM_NEW, s, sn);
+        float sn;
+        jacobi_row<float>(tile_row(a, s3 + p.in_a(), kAX, kAX * kAY), d3, di, SC_ADD_FROM_NEW, s, sn);
         sc[p.row] = sn;
     }
 }
 
-template <class V>
-DiaRows<V> rows_of(const OpMat<V> &At)
-{
-    return DiaRows<V>{At.dia.vals(), At.dia.ld};
-}
+DiaRows<float> rows_of(const OpMat<float> &At) { return DiaRows<float>{At.dia.vals(), At.dia.ld}; }
 dim3 tiles(const GridPair &g) { return dim3(div_up(g.nx, kOX), div_up(g.ny, kOY), div_up(g.nz, kOZ)); }
 
 }  // namespace
 
-template <class V>
-bool level3d_ok(const OpMat<V> &At, const GridPair &g)
+bool level3d_ok(const OpMat<float> &At, const GridPair &g)
 {
     if (At.kind != 1 || g.dim != 3 || g.nx < 3 || g.ny < 3 || g.nz < 3) return false;
     if (At.nrows != g.nx * g.ny * g.nz || At.ncols != At.nrows) return false;
-    if (sizeof(V) != 4 || At.dia.S != 27 || At.nrows > kLevel3dRows) return false;
+    if (At.dia.S != 27 || At.nrows > kLevel3dRows) return false;
     for (int k = 0; k < 27; ++k)
         if (At.dia.off.o[k] != k % 3 - 1 + g.nx * (k / 3 % 3 - 1) + g.nx * g.ny * (k / 9 - 1)) return false;
     return true;
 }
 
-template <class V>
-void level3d_pre(Ctx &c, const OpMat<V> &At, const GridPair &g, const V *dinv, const V *d, V *sc, V *dout,
-                 const int *skip)
+void level3d_pre(Ctx &c, const OpMat<float> &At, const GridPair &g, const float *dinv, const float *d, float *sc,
+                 float *dout, const int *skip)
 {
-    if constexpr (sizeof(V) == 4) UG_LAUNCH_PDL(c, k_pre3d<V>, tiles(g), kT, 0, rows_of(At), g, dinv, d, sc, dout, skip);
+    UG_LAUNCH_PDL(c, k_pre3d, tiles(g), kT, 0, rows_of(At), g, dinv, d, sc, dout, skip);
 }
 
-template <class V>
-void level3d_post(Ctx &c, const OpMat<V> &At, const GridPair &g, const V *dinv, const V *dfac, const V *scc, const V *d,
-                  V *sc, const int *skip)
+void level3d_post(Ctx &c, const OpMat<float> &At, const GridPair &g, const float *dinv, const float *dfac,
+                  const float *scc, const float *d, float *sc, const int *skip)
 {
-    if constexpr (sizeof(V) == 4)
-        UG_LAUNCH_PDL(c, k_post3d<V>, tiles(g), kT, 0, rows_of(At), g, dinv, dfac, scc, d, sc, skip);
+    UG_LAUNCH_PDL(c, k_post3d, tiles(g), kT, 0, rows_of(At), g, dinv, dfac, scc, d, sc, skip);
 }
-
-#define INST_LEVEL3D(V)                                                                                            \
-    template bool level3d_ok<V>(const OpMat<V> &, const GridPair &);                                               \
-    template void level3d_pre<V>(Ctx &, const OpMat<V> &, const GridPair &, const V *, const V *, V *, V *,        \
-                                 const int *);                                                                     \
-    template void level3d_post<V>(Ctx &, const OpMat<V> &, const GridPair &, const V *, const V *, const V *,      \
-                                  const V *, V *, const int *);
-INST_LEVEL3D(double)
-INST_LEVEL3D(float)
 
 }  // namespace ug4gb

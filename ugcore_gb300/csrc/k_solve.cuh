@@ -319,16 +319,13 @@ void level2d_post(Ctx &c, const OpMat<V> &At, const GridPair &gp, const V *dinv,
 // tetrahedra gained less than 1 %.
 constexpr int kLevel3dRows = 60000;
 // At holds the 27-point stencil of the structured 3D level gp
-template <class V>
-bool level3d_ok(const OpMat<V> &At, const GridPair &gp);
+bool level3d_ok(const OpMat<float> &At, const GridPair &gp);
 // as level2d_pre without the restriction
-template <class V>
-void level3d_pre(Ctx &c, const OpMat<V> &At, const GridPair &gp, const V *dinv, const V *d, V *sc, V *dout,
-                 const int *skip);
+void level3d_pre(Ctx &c, const OpMat<float> &At, const GridPair &gp, const float *dinv, const float *d, float *sc,
+                 float *dout, const int *skip);
 // as level2d_post, below the top level
-template <class V>
-void level3d_post(Ctx &c, const OpMat<V> &At, const GridPair &gp, const V *dinv, const V *dfac, const V *scc,
-                  const V *d, V *sc, const int *skip);
+void level3d_post(Ctx &c, const OpMat<float> &At, const GridPair &gp, const float *dinv, const float *dfac,
+                  const float *scc, const float *d, float *sc, const int *skip);
 
 // Multicolour Gauss-Seidel sweeps of a structured level line by line
 // (k_mcgs_lines): per colour (parity bits of the vertex), which diagonals lead
