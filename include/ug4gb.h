@@ -133,12 +133,15 @@ UG4GB_API int ug4gb_set_operator_format(ug4gb_ctx *ctx, int format);
    (Jacobi smoothers on both sides, dense LU base solver, structured levels
    with grid transfers) run by one cluster of up to 16 blocks in one launch:
    the base level and up to this many levels above it (never the top level),
-   their operators, Jacobi factors and vectors in the blocks' shared memory.
-   -1: the levels where this was measured faster on GB300 (a Jacobi sweep of
-   at most about 110000 row-operations, rows x (stencil width + 3)); 0: every
-   level by separate
-   launches.  Corrections are bit-identical either way.  Applies to
-   multigrids set up after the call. */
+   their operators, Jacobi factors and vectors in the blocks' shared memory
+   (208 KB each).  -1: the levels where this was measured faster on GB300.
+   These are levels whose Jacobi sweep takes at most 110000 row-operations, rows x
+   (stencil width + 3): some 11000 rows of 7 diagonals, 9000 of 9, 6000 of 15, 3600
+   of 27; with V(2,2) on quadrilaterals, whose levels then take two launches each,
+   at most 400 (33 rows); of levels prepared for two steps per pass
+   (UG4GB_TUNE_SWEEP_FUSION) at most 16000; and none above a base of more than
+   256 rows.  0: every level by separate launches.  Corrections are bit-identical
+   either way.  Applies to multigrids set up after the call. */
 #define UG4GB_TUNE_COARSE_LEVELS 6
 /* UG4GB_TUNE_SCRATCH_TEST (0 or 1; default 0): failure test only.  The row-wise
    assembly of unstructured simplex levels asks for more device memory than

@@ -139,7 +139,8 @@ struct Ctx {
     // as many as were measured faster than separate launches, 0: none)
     int coarse_levels = -1;
     int coarse_blocks = 16;        // the most blocks of that cluster
-    int coarse_ctas[2][kMaxDiag] = {};   // blocks it runs with, FP64 and FP32 levels, by stencil width (-1: none fit, 0: not asked yet)
+    // blocks it runs with, FP64 and FP32 levels, by stencil width (-1: none fit, 0: not asked yet)
+    int coarse_ctas[2][kMaxDiag] = {};
     std::string prof_tag;       // set by the orchestration (level / phase)
     std::vector<ProfRec> prof;
     std::vector<cudaEvent_t> ev_pool;

@@ -213,7 +213,8 @@ __global__ void __launch_bounds__(256) k_gather_rows(AsmArgs a, int nv, const in
             for (int t = s0; t < s1; ++t) {
                 const unsigned ea = __ldg(adj + t), packed = __ldg(slots + t);
                 const int li = (int)(ea & 3u);
-                if (j < K) acc[slot(packed, j)] += __ldg(ws + (size_t)(ea >> 2) * S::WS + (j == li ? S::NOFF : S::pos(li, j)));
+                if (j < K)
+                    acc[slot(packed, j)] += __ldg(ws + (size_t)(ea >> 2) * S::WS + (j == li ? S::NOFF : S::pos(li, j)));
                 __syncwarp(group);   // another lane may add to this slot next
             }
             const int diag = slot(__ldg(slots + s0), (int)(__ldg(adj + s0) & 3u));

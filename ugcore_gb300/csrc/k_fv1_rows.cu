@@ -13,10 +13,11 @@
 //
 // One thread per interior row gathers the contributions of the elements
 // around its vertex (8 cells in 3D, 4 in 2D; for Kuhn cells the tets that
-// contain the vertex) in increasing cell order, the order in which the
-// element-wise reference adds them, and writes every value of the row and
-// its right-hand side once: no read-modify-write of the matrix, no colour
-// passes, no atomics.  The right-hand side of an interior row is
+// contain the vertex) and writes every value of the row and its right-hand
+// side once: no read-modify-write of the matrix, no colour passes, no atomics.
+// Quadrilaterals and tetrahedra are added in increasing cell order, the order in
+// which the element-wise reference adds them; hexahedra sum their coefficients
+// first (gather_row).  The right-hand side of an interior row is
 // f_i * sum_e |SCV_i^e|, the volumes summed once per level in the gather
 // order (the element-wise reference adds the products f_i |SCV_i^e|; the two
 // agree to rounding).  Convection (full upwind, ConvectionShapesFullUpwind,
@@ -33,11 +34,12 @@
 // assembly of 97^3 hexahedra took 7.3 ms and the defect of 49^3 Kuhn cells
 // 2.7 ms.
 //
-// The element kernels of k_fv1.cu stay the path of unstructured levels and of
-// boundary vertices without the Dirichlet flag outside the stationary
-// assembly.  Values agree with it (and with the oracle,
-// which computes every element's geometry from its own corner coordinates)
-// to rounding: the cells of a structured level are congruent up to the
+// The element kernels of k_fv1.cu stay the path of boundary vertices without
+// the Dirichlet flag outside the stationary assembly, and of what the row-wise
+// assembly of unstructured simplices (k_fv1_gather.cu) does not take: unstructured
+// quadrilaterals and hexahedra, convection, defects and gradients.  Values agree
+// with it (and with the oracle, which computes every element's geometry from its
+// own corner coordinates) to rounding: the cells of a structured level are congruent up to the
 // rounding of their corner coordinates i / (n - 1).
 #include <algorithm>
 #include <cmath>
@@ -433,8 +435,6 @@ __device__ __forceinline__ void row_in_time(const AsmArgs &a, double (&acc)[Sten
     acc[S::slot(0, 0, 0)] += a.sm0 * volsum;
 }
 
-// rows on the box boundary: the identity row and b = 0 at Dirichlet
-// vertices; otherwise the elements that exist, entries found by search
 // a boundary row without the Dirichlet flag: the elements that exist, entries
 // found by binary search in the row (rare; kept out of line)
 template <int T>

@@ -3,8 +3,10 @@
 // On 2D levels of up to some 10^5 vertices a Jacobi step or a transfer is a
 // launch of about 3 us, most of it the launch and chains of dependent loads and
 // FP64 operations, and a level takes six.  Two kernels replace them for
-// nu1 = nu2 = 2 (the levels' row arithmetic is that of the separate kernels, in
-// their order, so the corrections are the same bits):
+// nu1 = nu2 = 2, with the row arithmetic of the separate kernels in their order.
+// (FP32 corrections are the same bits.  FP64 rows are summed in two chains,
+// row_sum, which the separate kernels do on levels of up to a block of rows per SM
+// only, 38912 rows: above them the rounding differs.)
 //   k_pre2d    two pre-smoothing steps and the restriction
 //   k_post2d   the prolongation and two post-smoothing steps (on the top level
 //              with the fused (z, r) and the FP64 copy of the correction)
@@ -13,7 +15,7 @@
 // 19 x 11 vertices, the second on 17 x 9 (after the prolongation 20 x 12 and 18 x
 // 10), one vertex per thread, the vectors in shared memory, each thread's
 // operator row in registers for both steps, loaded before the launch wait.
-// 129^2 solve, FP64: 632 -> 526 us; 257^2 adjoint gradient 3.86 -> 3.54 ms.
+// 129^2 solve, FP64: 632 -> 526 us; 257^2 adjoint gradient 3.86 -> 3.59 ms.
 #include "k_solve.cuh"
 
 namespace ug4gb {

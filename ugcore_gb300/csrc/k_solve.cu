@@ -365,10 +365,10 @@ __global__ void __launch_bounds__(NT) k_smooth(MV A, const XT *__restrict__ x, c
 constexpr int smooth_dia_blocks(int S, bool rho) { return S == 7 && rho ? 6 : 8; }   // resident per SM
 
 template <class V, int S, bool RHO>
-__global__ void __launch_bounds__(NT, smooth_dia_blocks(S, RHO)) k_smooth_dia(DiaMV<V, S> A, const V *__restrict__ x, const V *__restrict__ dbase,
-                                                   const V *__restrict__ dinv, V *__restrict__ sc, V *__restrict__ dout,
-                                                   int sc_mode, const int *skip, const double *__restrict__ r_rho,
-                                                   RedArgs red, int rho_kind, double *__restrict__ z64)
+__global__ void __launch_bounds__(NT, smooth_dia_blocks(S, RHO))
+    k_smooth_dia(DiaMV<V, S> A, const V *__restrict__ x, const V *__restrict__ dbase, const V *__restrict__ dinv,
+                 V *__restrict__ sc, V *__restrict__ dout, int sc_mode, const int *skip,
+                 const double *__restrict__ r_rho, RedArgs red, int rho_kind, double *__restrict__ z64)
 {
     constexpr int W = 16 / sizeof(V);
     PDL_ENTRY();
@@ -866,11 +866,10 @@ void mcgs_colour(Ctx &c, const OpMat<V> &A, const int *rows, int nrows_c, const 
 // Three blocks per SM: a wave then holds the whole level (461 us against 515 for
 // the cycle; four blocks, 64 registers, spill: 551).
 template <class V, int S>
-__global__ void __launch_bounds__(NT, sizeof(V) == 4 ? 3 : 1) k_mcgs_lines(DiaMV<V, S> A, int nx, int ny, int b1, int b2, int nly, int nlines,
-                                                   int nz, int per, int per_block, int first, unsigned mask_even,
-                                                   unsigned mask_odd, GsLines gs, bool from_zero,
-                                                   const V *__restrict__ dr,
-                                                   const V *__restrict__ d, V *t, const int *skip)
+__global__ void __launch_bounds__(NT, sizeof(V) == 4 ? 3 : 1)
+    k_mcgs_lines(DiaMV<V, S> A, int nx, int ny, int b1, int b2, int nly, int nlines, int nz, int per, int per_block,
+                 int first, unsigned mask_even, unsigned mask_odd, GsLines gs, bool from_zero,
+                 const V *__restrict__ dr, const V *__restrict__ d, V *t, const int *skip)
 {
     const int step = per < NT ? per : NT;   // vertices of a line (one x parity) that are in work at a time
     const int ln = threadIdx.x / step, q0 = threadIdx.x - ln * step;
@@ -1134,7 +1133,8 @@ __global__ void __launch_bounds__(NT) k_krylov_start(MV A, const double *__restr
 void krylov_start(Ctx &c, const OpMat<double> &A, const double *x, double *r, RedArgs red, float *r32, bool bicg)
 {
     with_mv(A, [&](auto mv) {
-        UG_LAUNCH_PDL(c, k_krylov_start<decltype(mv)>, (spmv_grid<decltype(mv), double>(c, A.nrows, true)), NT, 0, mv, x, r, r32, bicg, red);
+        const int g = spmv_grid<decltype(mv), double>(c, A.nrows, true);
+        UG_LAUNCH_PDL(c, k_krylov_start<decltype(mv)>, g, NT, 0, mv, x, r, r32, bicg, red);
     });
 }
 
@@ -1172,7 +1172,8 @@ template <class ZT>
 void cg_spmv_dot_t(Ctx &c, const OpMat<double> &A, const ZT *z, double *p, double *q, int first, RedArgs red)
 {
     with_mv(A, [&](auto mv) {
-        UG_LAUNCH_PDL(c, (k_cg_spmv_dot<decltype(mv), ZT>), (spmv_grid<decltype(mv), double>(c, A.nrows, true)), NT, 0, mv, z, p, q, first, red);
+        const int g = spmv_grid<decltype(mv), double>(c, A.nrows, true);
+        UG_LAUNCH_PDL(c, (k_cg_spmv_dot<decltype(mv), ZT>), g, NT, 0, mv, z, p, q, first, red);
     });
 }
 template void cg_spmv_dot_t<double>(Ctx &, const OpMat<double> &, const double *, double *, double *, int, RedArgs);
@@ -1354,7 +1355,8 @@ template <class ZT>
 void bicg_spmv_dot_t(Ctx &c, const OpMat<double> &A, const ZT *q, double *v, const double *r0, RedArgs red)
 {
     with_mv(A, [&](auto mv) {
-        UG_LAUNCH_PDL(c, (k_bicg_spmv_dot<decltype(mv), ZT>), (spmv_grid<decltype(mv), double>(c, A.nrows, true)), NT, 0, mv, q, v, r0, red);
+        const int g = spmv_grid<decltype(mv), double>(c, A.nrows, true);
+        UG_LAUNCH_PDL(c, (k_bicg_spmv_dot<decltype(mv), ZT>), g, NT, 0, mv, q, v, r0, red);
     });
 }
 template void bicg_spmv_dot_t<double>(Ctx &, const OpMat<double> &, const double *, double *, const double *, RedArgs);
@@ -1437,7 +1439,8 @@ template <class ZT>
 void bicg_spmv_2dot_t(Ctx &c, const OpMat<double> &A, const ZT *q, double *t, const double *s, RedArgs red)
 {
     with_mv(A, [&](auto mv) {
-        UG_LAUNCH_PDL(c, (k_bicg_spmv_2dot<decltype(mv), ZT>), (spmv_grid<decltype(mv), double>(c, A.nrows, true)), NT, 0, mv, q, t, s, red);
+        const int g = spmv_grid<decltype(mv), double>(c, A.nrows, true);
+        UG_LAUNCH_PDL(c, (k_bicg_spmv_2dot<decltype(mv), ZT>), g, NT, 0, mv, q, t, s, red);
     });
 }
 template void bicg_spmv_2dot_t<double>(Ctx &, const OpMat<double> &, const double *, double *, const double *,
@@ -1533,7 +1536,8 @@ void op_axpy(Ctx &c, const OpMat<double> &A, double *dest, double alpha, const d
              const double *w1)
 {
     with_mv(A, [&](auto mv) {
-        UG_LAUNCH_PDL(c, k_op_axpy<decltype(mv)>, (spmv_grid<decltype(mv), double>(c, A.nrows, false)), NT, 0, mv, dest, alpha, v1, beta, w1);
+        const int g = spmv_grid<decltype(mv), double>(c, A.nrows, false);
+        UG_LAUNCH_PDL(c, k_op_axpy<decltype(mv)>, g, NT, 0, mv, dest, alpha, v1, beta, w1);
     });
 }
 
