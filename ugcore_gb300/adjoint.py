@@ -51,10 +51,13 @@ class DifferentiableProblem(problems.Problem):
         (on an unchanged hierarchy the multigrid and the solvers refresh their
         values in place and keep their captured graphs)."""
         _library_waits_for_torch(self.ctx)
-        # kept alive until the library has read them (the uploads synchronise)
         self._inputs = (m.detach().contiguous(), f.detach().contiguous())
         self.disc.set_log_diffusion(self._inputs[0])
         self.disc.set_source(self._inputs[1])
+        # the library copies them in its stream's order, some time after this
+        # call: torch may change them, or give their memory to other tensors,
+        # only behind those copies
+        _torch_waits_for_library(self.ctx)
         self.disc.assemble_linear(self.A, self.b)
         self.gmg.set_transposed(False)
         self.gmg.init(self.A)
