@@ -1,6 +1,7 @@
-"""Gauss-Seidel on long, narrow grids: a level whose few lines of more than three
-rounds of a block would leave the GPU idle is swept colour by colour, any other
-line by line; the same corrections as the SELL format's, to rounding of the
+"""Gauss-Seidel on long, narrow grids and on large FP64 levels: a level whose few
+lines of more than three rounds of a block would leave the GPU idle is swept colour
+by colour, so is an FP64 level of 27 diagonals above 700000 rows, any other line by
+line; the same corrections as the SELL format's, to rounding of the
 transfers (1e-13 of the largest entry in FP64, 1e-6 in FP32)."""
 import numpy as np
 import pytest
@@ -34,9 +35,10 @@ def _correction(fmt, elem, m, nref, precision):
 
 
 # vertices per line 1505, 1537 (three and four rounds of 256 threads per colour),
-# few lines of them; 1537 with 76 and more lines per set; 3D
+# few lines of them; 1537 with 80 and with 144 lines per set; 3D
 @pytest.mark.parametrize("elem,m,nref,lines", [("quad", (47, 1, 1), 5, True), ("quad", (48, 1, 1), 5, False),
-                                               ("quad", (48, 5, 1), 5, True), ("hex", (192, 1, 1), 3, False),
+                                               ("quad", (48, 5, 1), 5, False),
+                                               ("quad", (48, 9, 1), 5, True), ("hex", (192, 1, 1), 3, False),
                                                ("tet", (256, 2, 1), 3, False)])
 @pytest.mark.parametrize("precision,tol", [("fp64", 1e-13), ("mixed", 1e-6)])
 def test_route_and_result(elem, m, nref, lines, precision, tol):
@@ -52,4 +54,14 @@ def test_one_block_of_two_rounds(precision, tol, lines):
     got, used = _correction("auto", "hex", (256, 1, 1), 1, precision)
     assert used == lines
     want, _ = _correction("sell", "hex", (256, 1, 1), 1, precision)
+    assert np.abs(got - want).max() <= tol * np.abs(want).max()
+
+
+@pytest.mark.parametrize("m,precision,tol,lines", [((5, 5, 5), "fp64", 1e-13, True), ((6, 5, 6), "fp64", 1e-13, False),
+                                                   ((6, 5, 6), "mixed", 1e-6, True)])
+def test_large_fp64_levels(m, precision, tol, lines):
+    """81^3 and 97 x 81 x 97 hexahedra: 531441 and 762129 rows"""
+    got, used = _correction("auto", "hex", m, 4, precision)
+    assert used == lines
+    want, _ = _correction("sell", "hex", m, 4, precision)
     assert np.abs(got - want).max() <= tol * np.abs(want).max()

@@ -1090,7 +1090,7 @@ static GmgBase *build_gmg(ug4gb_gmg *m, const ug4gb_matrix *A_top, GmgT<V> *reus
             if constexpr (sizeof(V) == 4)
                 L.level3d = m->smoother2 == UG4GB_SMOOTHER_JACOBI && !L.sweep2 && level3d_ok(L.At, L.gp);
         } else if (L.At_lay.known)
-            L.gs = gs_lines(c, sizeof(V) == 8, L.At.dia.off, L.At.dia.S, L.At_lay.all, L.gp);
+            L.gs = gs_lines(sizeof(V) == 8, L.At.dia.off, L.At.dia.S, L.At_lay.all, L.gp);
     }
     G->setup_base(c);
     G->setup_coarse(c);

@@ -939,28 +939,34 @@ static int lines_per_block(const GridPair &gp) { return line_half(gp) < NT ? NT 
 
 // A block takes a line of more than 2 NT vertices in several rounds, one after the
 // other; with few such lines most of the GPU is idle, where a launch per colour
-// fills it.  Up to three rounds, or with blocks on half of the SMs, the lines are
-// faster.  Cycles with lines only within these limits / on all levels / on none:
-// 32769 x 65 quads FP32 618 / 1876 / 633 us, FP64 1089 / 3259 / 1101; 4097 x 65
-// FP32 276 / 332 / 340, FP64 411 / 563 / 499; 4097 x 9 x 9 hexes FP32 553 / 756 /
-// 585; 2049 x 1025 quads FP32 561 / 565 / 792 (limits of one and two rounds, or
-// blocks on all SMs, were slower: 4097 x 65 304 / 287, 4097 x 513 FP32 424).
-// FP64 rounds of 15 and 27 diagonals take 2 us of an SM's FP64 pipe: with fewer
-// than four blocks one round is the limit (1025 x 3 x 3 hexes below 4097 x 9 x 9: a
-// cycle 895 us with three rounds, 833 with one, 816 by colours).
-static bool lines_fill(const Ctx &c, const GridPair &gp, bool fp64_bound)
+// fills it.  Up to three rounds, or with 32 blocks per round, the lines are faster.
+// Cycles with the top level by lines, against by colours (forward / symmetric sweeps):
+// FP32 1025 x 257 quads, 3 rounds, 128 blocks 0.95 / 0.93; 2049 x 257, 5 rounds 0.99 /
+// 1.01; 4097 x 257, 9 rounds - / 1.08; 12545 x 257, 25 rounds - / 1.26; 2049 x 33 x 33
+// hexes, 5 rounds, 256 blocks 0.87 / 0.91; 2049 x 17 x 17, 64 blocks - / 1.07; 4097^2
+// quads, 9 rounds, 2048 blocks 0.78 / 0.82 (FP64 0.87 / 0.93).
+// FP64 rounds of 15 and 27 diagonals take 2 us of an SM's FP64 pipe and hold a row's
+// entries in registers, at one or two blocks per SM.  With fewer than four blocks one
+// round is the limit (1025 x 3 x 3 hexes below 4097 x 9 x 9: a cycle 895 us with three
+// rounds, 833 with one, 816 by colours), and on large levels the colours' full
+// occupancy is faster: 65^3 hexes 0.84 / 0.81, 513 x 33 x 33 0.97 / 0.97, 769 x 33 x 33
+// 1.03 / 1.03, 97^3 1.00 / 1.02, 129^3 1.07 / 1.14.
+static bool lines_fill(const GridPair &gp, bool fp64_bound)
 {
+    constexpr int64_t kFp64Rows = 700000;
+    if (fp64_bound && (int64_t)gp.nx * gp.ny * gp.nz > kFp64Rows) return false;
     const int rounds = (int)div_up(line_half(gp), NT);
     const int lines = (gp.ny / 2) * (gp.dim == 3 ? gp.nz / 2 : 1);   // of the smallest set
     const int blocks = (int)div_up(lines, lines_per_block(gp));
-    if (rounds <= 1 || blocks >= c.num_sms / 2) return true;
-    return rounds <= 3 && (!fp64_bound || blocks >= 4);
+    if (rounds <= 1) return true;
+    if (rounds <= 3) return !fp64_bound || blocks >= 4;
+    return blocks >= 32 * rounds;
 }
 
-GsLines gs_lines(const Ctx &c, bool fp64, const Offs &offs, int S, const std::vector<int> &entries, const GridPair &gp)
+GsLines gs_lines(bool fp64, const Offs &offs, int S, const std::vector<int> &entries, const GridPair &gp)
 {
     GsLines g;
-    if (gp.nx < 3 || gp.ny < 3 || S > 32 || !lines_fill(c, gp, fp64 && S >= 15)) return g;
+    if (gp.nx < 3 || gp.ny < 3 || S > 32 || !lines_fill(gp, fp64 && S >= 15)) return g;
     for (int k = 0; k < S; ++k) {
         const int o = offs.o[k];
         if (!std::binary_search(entries.begin(), entries.end(), o)) continue;

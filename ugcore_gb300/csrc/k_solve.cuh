@@ -341,7 +341,7 @@ struct GsLines {
 // offs: the layout's offsets, entries: those of them that the CRS holds (the
 // rest is padding); unusable where an entry is no neighbour in the grid or
 // couples vertices of one colour, and where few long lines would leave the GPU idle
-GsLines gs_lines(const Ctx &c, bool fp64, const Offs &offs, int S, const std::vector<int> &entries, const GridPair &gp);
+GsLines gs_lines(bool fp64, const Offs &offs, int S, const std::vector<int> &entries, const GridPair &gp);
 // one sweep over all colours: t_i = t_i + dinv_relax_i (d_i - (A t)_i), colours
 // increasing or (backward) decreasing; from_zero: t is 0 before the sweep and
 // need not be written
