@@ -617,9 +617,12 @@ struct GmgT : GmgBase {
     // row is FP64 bound on one SM.  Of more than 256 rows its inverse takes so long
     // to stage that separate launches are faster (FP32 levels on a base of 473 rows,
     // a CG step with V(2,2), V(1,1), V(1,0): 30.7, 34.6, 32.6 us by separate launches,
-    // 30.4, 39.1, 38.6 by a cluster).  Where no level passes 4000 row-operations in
-    // FP64 or 8000 in FP32, one block does all of it without a cluster (V(4,4) on 9 x
-    // 73 quads, FP32, a CG step 50.1 -> 47.3 us).
+    // 30.4, 39.1, 38.6 by a cluster).  Where no level passes 3300 row-operations in
+    // FP64 or 8000 in FP32, one block does all of it without a cluster (a CG step with
+    // V(4,4), cluster -> one block: FP32 9 x 73 quads 50.5 -> 49.9 us, 33^2 56.8 ->
+    // 54.6; FP64 13^2 below 25^2 quads, 2028 row-operations, 63.2 -> 61.3, 3 x 5 x 7
+    // below 5 x 9 x 13 hexes, 3150, 71.2 -> 67.8, 17^2 below 33^2 quads, 3468, 75.1 ->
+    // 76.8).
     void setup_coarse(Ctx &c)
     {
         coarse_top = -1;
@@ -638,7 +641,7 @@ struct GmgT : GmgBase {
         }
         if (coarse_ctas < 0) return;   // separate launches
         constexpr double kSharedWork = 110e3, kSharedWork2d = 400.0, kSharedWorkSweep2 = 16e3, kSoloWork = 1000.0;
-        constexpr double kOneBlockWork = sizeof(V) == 8 ? 4000.0 : 8000.0;
+        constexpr double kOneBlockWork = sizeof(V) == 8 ? 3300.0 : 8000.0;
         constexpr int kBaseRows = 32, kBaseRowsMax = 256;
         if (c.coarse_levels < 0 && nbase > kBaseRowsMax) return;
         constexpr int kAlign = 16 / (int)sizeof(V);   // elements per 16 bytes

@@ -147,14 +147,11 @@ template <class V>
 __device__ __noinline__ void coarse_restrict(const CoarseLevel<V> &L, const V *d, V *dc, int c0, int nc)
 {
     const GridPair &g = L.gp;
-    auto rows = [&](const auto &at) {
-        for (int q = threadIdx.x; q < nc; q += blockDim.x) {
-            const int c = c0 + q;
-            dc[q] = restrict_value<V>(g, at, c % g.cnx, (c / g.cnx) % g.cny, c / (g.cnx * g.cny));
-        }
-    };
-    if (L.solo) rows(LocalVec<V>{d});
-    else rows(ClusterVec<V>(L, d));
+    const ClusterVec<V> at(L, d);
+    for (int q = threadIdx.x; q < nc; q += blockDim.x) {
+        const int c = c0 + q;
+        dc[q] = restrict_value<V>(g, at, c % g.cnx, (c / g.cnx) % g.cny, c / (g.cnx * g.cny));
+    }
 }
 
 // sc += P scc, w = t * dfac (w nullable); C: the level below
@@ -163,17 +160,14 @@ __device__ __noinline__ void coarse_prolong(const CoarseLevel<V> &L, const Coars
                                             const V *dfac, V *w, int r0, int nr)
 {
     const GridPair &g = L.gp;
-    auto rows = [&](const auto &at) {
-        for (int q = threadIdx.x; q < nr; q += blockDim.x) {
-            const int f = r0 + q;
-            V t = prolong_value<V>(g, at, f % g.nx, (f / g.nx) % g.ny, f / (g.nx * g.ny));
-            if (g.dprol != 1.0) t = mul_rn(t, (V)g.dprol);
-            sc[q] = add_rn(sc[q], t);
-            if (w) w[q] = mul_rn(t, dfac[q]);
-        }
-    };
-    if (L.solo) rows(LocalVec<V>{scc});   // (then the level below is block 0's too)
-    else rows(ClusterVec<V>(C, scc));
+    const ClusterVec<V> at(C, scc);
+    for (int q = threadIdx.x; q < nr; q += blockDim.x) {
+        const int f = r0 + q;
+        V t = prolong_value<V>(g, at, f % g.nx, (f / g.nx) % g.ny, f / (g.nx * g.ny));
+        if (g.dprol != 1.0) t = mul_rn(t, (V)g.dprol);
+        sc[q] = add_rn(sc[q], t);
+        if (w) w[q] = mul_rn(t, dfac[q]);
+    }
 }
 
 template <class V, int S>
