@@ -21,14 +21,21 @@ from . import problems
 from .algebra import GPUVector
 
 
+def _stream(ctx):
+    """the library's stream as torch sees it (one object per context)"""
+    if getattr(ctx, "_torch_stream", None) is None:
+        ctx._torch_stream = torch.cuda.ExternalStream(ctx.stream)
+    return ctx._torch_stream
+
+
 def _library_waits_for_torch(ctx):
     """the library's stream waits (on the device, through an event) for the
     work queued so far on torch's current stream"""
-    torch.cuda.ExternalStream(ctx.stream).wait_stream(torch.cuda.current_stream())
+    _stream(ctx).wait_stream(torch.cuda.current_stream())
 
 
 def _torch_waits_for_library(ctx):
-    torch.cuda.current_stream().wait_stream(torch.cuda.ExternalStream(ctx.stream))
+    torch.cuda.current_stream().wait_stream(_stream(ctx))
 
 
 class DifferentiableProblem(problems.Problem):
