@@ -539,28 +539,30 @@ __global__ void __launch_bounds__(128) k_assemble_rows_all(AsmArgs a, ClassData<
     for (int s = 0; s < S::N; ++s) row[s] = acc[s];
 }
 
-// Large levels: the first nbb blocks take the rows of a list (the box surface),
-// one warp per row, memory work that the others' FP64 work hides (a launch of
-// its own: 25 us on 129^3); the others the interior rows, one thread per row,
-// every value written once.  A warp's 32 rows go through shared memory, so that
-// consecutive threads write consecutive values (each thread writing its own row
-// of 27 touched 32 sectors, 8 bytes in each, per store).
+// Large levels: the first nib blocks take the interior rows, one thread per row,
+// every value written once; the others the rows of a list (the box surface), one
+// warp per row, memory work that fills in beside and behind the FP64 work (a launch
+// of its own: 25 us on 129^3; in front it kept the interior rows waiting: 17 x 17 x
+// 241 tetrahedra with convection 65 -> 41 us, 129^3 229 -> 225).  A warp's 32
+// interior rows go through shared memory, so that consecutive threads write
+// consecutive values (each thread writing its own row of 27 touched 32 sectors, 8
+// bytes in each, per store).
 template <int T, bool INST>
 __global__ void __launch_bounds__(128) k_assemble_rows(AsmArgs a, ClassData<T> cd, const double *__restrict__ flux,
                                                        double volsum, const unsigned char *__restrict__ bnd,
-                                                       const int *__restrict__ brows, int nbrows, int nbb)
+                                                       const int *__restrict__ brows, int nbrows, int nib)
 {
     PDL_ENTRY();
     using S = Stencil<T>;
     __shared__ double rows[4][32 * S::N];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    if ((int)blockIdx.x < nbb) {
-        const int t = blockIdx.x * 4 + warp;
+    if ((int)blockIdx.x >= nib) {
+        const int t = (blockIdx.x - nib) * 4 + warp;
         if (t < nbrows) boundary_row<T>(a, cd, flux, bnd, brows[t], lane);
         return;
     }
     const int nix = a.cx - 1, niy = a.cy - 1, niz = (S::DIM == 3) ? a.cz - 1 : 1;
-    const int t = (blockIdx.x - nbb) * blockDim.x + threadIdx.x;
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
     int start = -1;   // of this thread's row in the values
     if (t < nix * niy * niz) {
         const int i = 1 + t % nix, j = 1 + (t / nix) % niy, k = (S::DIM == 3) ? 1 + t / (nix * niy) : 0;
@@ -960,9 +962,9 @@ void run_assemble_rows(Ctx &c, const Level &L, const AsmArgs &a, const ClassData
     } else if (L.nv <= kSmallLevelRows) {
         UG_LAUNCH_PDL(c, (k_assemble_rows_all<T, INST>), div_up(L.nv, 128), 128, 0, a, cd, flux, cache.volsum, L.bnd.p);
     } else {
-        const int nbb = (int)div_up(cache.nbrows, 4);
-        UG_LAUNCH_PDL(c, (k_assemble_rows<T, INST>), nbb + (int)div_up(nint, 128), 128, 0, a, cd, flux, cache.volsum,
-                      L.bnd.p, cache.brows.p, cache.nbrows, nbb);
+        const int nib = (int)div_up(nint, 128);
+        UG_LAUNCH_PDL(c, (k_assemble_rows<T, INST>), nib + (int)div_up(cache.nbrows, 4), 128, 0, a, cd, flux,
+                      cache.volsum, L.bnd.p, cache.brows.p, cache.nbrows, nib);
     }
 }
 
